@@ -1,8 +1,10 @@
-"""ctypes binding of the C ABI declared in ``include/flash_colsum_b200.h``."""
+"""ctypes binding of the C ABI declared in ``include/flash_colsum_b200.h``, and the native
+binding (``csrc/torch_binding.cpp``) that PyTorch calls of the operator go through."""
 
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import warnings
 from typing import Optional
@@ -30,6 +32,7 @@ FCS_DTYPE_FP16 = 0
 FCS_DTYPE_BF16 = 1
 
 _lib: Optional[ctypes.CDLL] = None
+_native = None
 
 _i, _i64, _f, _p, _sz = ctypes.c_int, ctypes.c_int64, ctypes.c_float, ctypes.c_void_p, ctypes.c_size_t
 
@@ -142,6 +145,21 @@ def load() -> ctypes.CDLL:
     lib.fcs_plan_info.argtypes = [_i] * 5 + [_p] * 4
     _lib = lib
     return lib
+
+
+def native():
+    """The extension module of ``csrc/torch_binding.cpp``, bound to the loaded library."""
+    global _native
+    if _native is None:
+        lib = load()
+        if not os.path.exists(_build.BINDING_PATH):
+            raise LibraryMissing(f"{_build.BINDING_PATH} is missing; run `python -m flash_colsum_b200.build`")
+        spec = importlib.util.spec_from_file_location(_build.BINDING_NAME, _build.BINDING_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind(lib._handle)
+        _native = module
+    return _native
 
 
 def last_error() -> str:

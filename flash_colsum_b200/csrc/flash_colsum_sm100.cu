@@ -41,6 +41,7 @@
 #include <string.h>
 
 #include "../../include/flash_colsum_b200.h"
+#include "host_api.h"
 
 #include "colsum_single_pass.cuh"
 #include "select_topk.cuh"
@@ -1344,10 +1345,12 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
                        void* workspace, size_t workspace_bytes, int* status, void* stream_v,
                        bool clear_out = true, int passes = PASSES_BOTH, float* shared_lse = nullptr,
                        long long norm_rows = 0, float* clear_extra = nullptr, long long clear_extra_n = 0,
-                       const FcsPeerSignals* sig = nullptr) {
+                       const FcsPeerSignals* sig = nullptr, void* (*alloc)(void*, size_t) = nullptr,
+                       void* alloc_ctx = nullptr) {
     // passes: both, or one of the two for work split over devices (non-causal only) --
     // PASSES_STATS writes -(log-sum-exp + log2(h_norm * norm_rows)) of the given query rows to
     // `shared_lse`; PASSES_COLUMNS takes that vector for ALL query rows and the given keys.
+    // Scratch is `workspace`, or without one what `alloc` returns for the bytes the call needs.
     g_err[0] = 0;
     if (B <= 0 || H <= 0 || Sq_full <= 0 || Sk <= 0)
         return fail(FCS_ERR_INVALID_ARGUMENT, "sizes must be positive (B=%d H=%d Sq=%d Sk=%d)", B, H, Sq_full, Sk);
@@ -1468,6 +1471,10 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
     // the two streaming passes are the only kernels that use scratch memory
     size_t part_off = 0, ext_off = 0;
     const size_t need = workspace_layout(p, &part_off, &ext_off);
+    if (!workspace && alloc) {
+        workspace = alloc(alloc_ctx, need);
+        workspace_bytes = workspace ? need : 0;
+    }
     if (!workspace || workspace_bytes < need)
         return fail(FCS_ERR_WORKSPACE, "workspace too small: need %zu bytes, got %zu", need, workspace_bytes);
     if (reinterpret_cast<uintptr_t>(workspace) % 256)
@@ -1741,6 +1748,13 @@ int fcs_colsum_causal_batched(const void* q, const void* k, float* out, int64_t 
     return fcs::colsum_impl(q, k, out, out_ld, B, H, q_len, k_len, D, dtype, q_stride_b, q_stride_h, q_stride_s,
                             k_stride_b, k_stride_h, k_stride_s, scale, 1, k_past, -1, h_norm, workspace,
                             workspace_bytes, status, stream);
+}
+
+int fcs_run_call(const FcsCall* c) {
+    return fcs::colsum_impl(c->q, c->k, c->out, c->out_ld, c->B, c->H, c->Sq, c->Sk, c->D, c->dtype, c->q_stride[0],
+                            c->q_stride[1], c->q_stride[2], c->k_stride[0], c->k_stride[1], c->k_stride[2], c->scale,
+                            c->causal, c->k_past, c->cls_n, c->h_norm, nullptr, 0, c->status, c->stream, true,
+                            fcs::PASSES_BOTH, nullptr, 0, nullptr, 0, nullptr, c->alloc, c->alloc_ctx);
 }
 
 size_t fcs_statistics_rows(int q_rows) {

@@ -1,0 +1,34 @@
+// What the PyTorch binding (torch_binding.cpp) calls in the CUDA library: one call of the
+// operator with the scratch taken from the caller's allocator as part of the call, so that the
+// sizes are planned once.  Internal to this package; the C ABI for other hosts is
+// include/flash_colsum_b200.h.
+#pragma once
+
+#include <stddef.h>
+#include <stdint.h>
+
+extern "C" {
+
+typedef struct FcsCall {
+    const void* q;
+    const void* k;
+    float* out;
+    int64_t out_ld;
+    int B, H, Sq, Sk, D;          // Sq: query rows of the tensor
+    int dtype;                    // FCS_DTYPE_*
+    int64_t q_stride[3], k_stride[3];   // batch, head, row; in elements
+    float scale;
+    int causal, k_past, cls_n, h_norm;  // as in fcs_colsum_causal_batched / fcs_colsum_batched
+    int* status;
+    void* stream;
+    void* (*alloc)(void* ctx, size_t bytes);   // 256-byte aligned device memory, valid for the stream's work queued so far; NULL on failure
+    void* alloc_ctx;
+} FcsCall;
+
+typedef int (*FcsRunCallFn)(const FcsCall*);
+typedef int (*FcsSelectTopkFn)(const float*, int64_t, int, int, int, int*, float*, void*);
+typedef int (*FcsSelectThresholdFn)(const float*, int64_t, int, int, float, int, int*, int*, void*);
+typedef const char* (*FcsLastErrorFn)(void);
+
+int fcs_run_call(const FcsCall* call);
+}

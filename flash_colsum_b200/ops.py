@@ -1,10 +1,11 @@
 """The operator: column means of softmax attention without forming the matrix.
 
 Same call as the reference's ``flash_colsum`` (flash_colsum/ops.py:13-105): same
-arguments, same validation order and messages, same three-way dispatch (causal /
-single-sample / batched) -- each branch calls one C-ABI entry point of the CUDA
-library instead of a Triton launcher.  There is no CPU path and no fallback: if
-the library is missing the call raises.
+arguments, same validation order and messages.  A valid call goes straight to the native host
+path (``csrc/torch_binding.cpp``), which makes the output, takes scratch from torch's allocator
+and launches the kernels of the CUDA library; the Python below it is what finds out why a call
+is refused, and the entry points whose callers hold their own buffers.  There is no CPU path and
+no fallback: if the library is missing the call raises.
 """
 
 from __future__ import annotations
@@ -22,6 +23,11 @@ _DTYPE_CODE = {torch.float16: _cabi.FCS_DTYPE_FP16, torch.bfloat16: _cabi.FCS_DT
 # one sticky device-status word per device, zeroed once
 _status: Dict[int, torch.Tensor] = {}
 
+# The native host path (csrc/torch_binding.cpp), once the first call has loaded it.  It takes a
+# call from the Python arguments to the launches and answers None for arguments it does not take:
+# those go through the checks below, which raise or make the call takeable.
+_native = None
+
 
 def _status_word(device: torch.device) -> torch.Tensor:
     idx = device.index if device.index is not None else torch.cuda.current_device()
@@ -30,6 +36,16 @@ def _status_word(device: torch.device) -> torch.Tensor:
         t = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
         _status[idx] = t
     return t
+
+
+def _load_native(device: torch.device):
+    """The native host path, with this device's status word made known to it."""
+    global _native
+    module = _cabi.native()
+    word = _status_word(device)
+    module.set_status(word.device.index, word.data_ptr())
+    _native = module
+    return module
 
 
 def device_status(device=None) -> int:
@@ -46,9 +62,8 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     return t.contiguous()
 
 
-# The wrappers below run for every call, and calls of a dozen microseconds of GPU work are
-# bound by them: the device guard is skipped when the tensors' device is the current one, and
-# the stream handle comes from the raw getter instead of a Stream object.
+# (the entry points below that hold caller's buffers go through ctypes: the device guard is skipped
+# when the tensors' device is the current one, the stream handle comes from the raw getter)
 _NO_GUARD = contextlib.nullcontext()
 _raw_stream_getter = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
@@ -68,10 +83,6 @@ def _raw_stream(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-def _rows(cls_n: int, S: int) -> int:
-    return S if cls_n == -1 else min(cls_n, S)
-
-
 def _check(rc: int) -> None:
     if rc != _cabi.FCS_OK:
         raise RuntimeError(f"flash_colsum_b200: {_cabi.last_error()} (code {rc})")
@@ -88,7 +99,8 @@ def _round_fp32(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, t
     return query.to(dt), key.to(dt)
 
 
-def _prepare(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, int]:
+def _prepare_types(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """The operands in a type the kernels take; raises for what they do not."""
     if key.dtype != query.dtype:
         raise ValueError(f"query and key must have the same dtype, got {query.dtype} and {key.dtype}")
     if key.device != query.device:
@@ -99,6 +111,11 @@ def _prepare(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, torc
         raise ValueError(f"flash_colsum supports float16, bfloat16 and float32 inputs, got {query.dtype}")
     if query.shape[3] % 8 or not 8 <= query.shape[3] <= 128:
         raise ValueError(f"head_dim must be a multiple of 8 from 8 to 128, got {query.shape[3]}")
+    return query, key
+
+
+def _prepare(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, int]:
+    query, key = _prepare_types(query, key)
     return _tma_ready(query), _tma_ready(key), _DTYPE_CODE[query.dtype]
 
 
@@ -134,38 +151,27 @@ def _workspace_two_pass(lib, device, B, H, rows, Sk, D) -> torch.Tensor:
     return torch.empty(n, dtype=torch.uint8, device=device)
 
 
+def _launch(Q: torch.Tensor, K: torch.Tensor, scale: float, is_causal: bool, k_past: int, cls_n: int,
+            h_norm: int) -> torch.Tensor:
+    """One call on operands of valid shape: (B, S_k) fp32.  ``k_past`` / ``cls_n`` -1 and ``h_norm`` 0
+    stand for the defaults."""
+    Q, K = _prepare_types(Q, K)
+    out = _load_native(Q.device).launch(Q, K, float(scale), is_causal, k_past, cls_n, h_norm)
+    if out is None:
+        raise ValueError(f"unsupported operands: query {tuple(Q.shape)}, key {tuple(K.shape)}")
+    return out
+
+
 def _flash_colsum_batched(Q: torch.Tensor, K: torch.Tensor, scale: float, CLS_N: int = -1,
                           h_norm: int = 0) -> torch.Tensor:
     """(B, S) fp32.  Counterpart of kernel_noncausal_batched.py:102."""
-    lib = _cabi.load()
-    Q, K, code = _prepare(Q, K)
-    B, H, S, D = Q.shape
-    with _on_device(Q.device):
-        out = torch.empty((B, S), device=Q.device, dtype=torch.float32)
-        ws = _workspace(lib, Q.device, B, H, _rows(CLS_N, S), S, D, False)
-        _check(lib.fcs_colsum_batched(
-            Q.data_ptr(), K.data_ptr(), out.data_ptr(), S, B, H, S, D, code,
-            Q.stride(0), Q.stride(1), Q.stride(2), K.stride(0), K.stride(1), K.stride(2),
-            float(scale), int(CLS_N), int(h_norm), ws.data_ptr(), ws.numel(),
-            _status_word(Q.device).data_ptr(), _raw_stream(Q.device)))
-    return out
+    return _launch(Q, K, scale, False, -1, int(CLS_N), int(h_norm))
 
 
 def _flash_colsum_non_batched(Q: torch.Tensor, K: torch.Tensor, scale: float, CLS_N: int = -1,
                               h_norm: int = 0) -> torch.Tensor:
     """(1, S) fp32.  Counterpart of kernel_noncausal.py:95."""
-    lib = _cabi.load()
-    Q, K, code = _prepare(Q, K)
-    _, H, S, D = Q.shape
-    with _on_device(Q.device):
-        out = torch.empty((1, S), device=Q.device, dtype=torch.float32)
-        ws = _workspace(lib, Q.device, 1, H, _rows(CLS_N, S), S, D, False)
-        _check(lib.fcs_colsum_non_batched(
-            Q.data_ptr(), K.data_ptr(), out.data_ptr(), H, S, D, code,
-            Q.stride(1), Q.stride(2), K.stride(1), K.stride(2),
-            float(scale), int(CLS_N), int(h_norm), ws.data_ptr(), ws.numel(),
-            _status_word(Q.device).data_ptr(), _raw_stream(Q.device)))
-    return out
+    return _launch(Q[:1], K[:1], scale, False, -1, int(CLS_N), int(h_norm))
 
 
 def _flash_colsum_causal(Q: torch.Tensor, K: torch.Tensor, scale: float, K_past: Optional[int] = None,
@@ -181,33 +187,31 @@ def _flash_colsum_causal(Q: torch.Tensor, K: torch.Tensor, scale: float, K_past:
     other GPUs -- the call then returns None, having launched nothing, when its shape takes
     a kernel that cannot do so (at most four query rows).
     """
+    k_past = -1 if K_past is None else int(K_past)
+    if accumulate_into is None:
+        return _launch(Q, K, scale, True, k_past, -1, int(h_norm))
     lib = _cabi.load()
     Q, K, code = _prepare(Q, K)
     _, H, Q_len, D = Q.shape
     K_len = K.shape[2]
+    out = accumulate_into
+    for t in (out,) if clear_next is None else (out, clear_next):
+        if t.dtype != torch.float32 or t.numel() != K_len or not t.is_contiguous():
+            raise ValueError("accumulate_into / clear_next must be contiguous fp32 tensors with K_len elements")
+    entry, head, tail = lib.fcs_colsum_causal_accumulate, (), ()
+    if signals is not None:
+        entry = lib.fcs_colsum_causal_accumulate_signalled
+        head = (0 if clear_next is None else clear_next.data_ptr(),)
+        tail = (ctypes.byref(signals),)
+    elif clear_next is not None:
+        entry = lib.fcs_colsum_causal_accumulate_and_clear
+        head = (clear_next.data_ptr(),)
     with _on_device(Q.device):
-        head, tail = (), ()
-        if accumulate_into is None:
-            out = torch.empty((1, K_len), device=Q.device, dtype=torch.float32)
-            entry = lib.fcs_colsum_causal
-        else:
-            out = accumulate_into
-            for t in (out,) if clear_next is None else (out, clear_next):
-                if t.dtype != torch.float32 or t.numel() != K_len or not t.is_contiguous():
-                    raise ValueError("accumulate_into / clear_next must be contiguous fp32 tensors with K_len elements")
-            entry = lib.fcs_colsum_causal_accumulate
-            if signals is not None:
-                entry = lib.fcs_colsum_causal_accumulate_signalled
-                head = (0 if clear_next is None else clear_next.data_ptr(),)
-                tail = (ctypes.byref(signals),)
-            elif clear_next is not None:
-                entry = lib.fcs_colsum_causal_accumulate_and_clear
-                head = (clear_next.data_ptr(),)
-        ws = _workspace(lib, Q.device, 1, H, Q_len, K_len, D, True, -1 if K_past is None else int(K_past))
+        ws = _workspace(lib, Q.device, 1, H, Q_len, K_len, D, True, k_past)
         rc = entry(
             Q.data_ptr(), K.data_ptr(), out.data_ptr(), *head, H, Q_len, K_len, D, code,
             Q.stride(1), Q.stride(2), K.stride(1), K.stride(2),
-            float(scale), -1 if K_past is None else int(K_past), int(h_norm),
+            float(scale), k_past, int(h_norm),
             ws.data_ptr(), ws.numel(),
             _status_word(Q.device).data_ptr(), _raw_stream(Q.device), *tail)
         if signals is not None and rc == _cabi.FCS_ERR_UNSUPPORTED:
@@ -261,6 +265,10 @@ def flash_colsum(
         ValueError: invalid shapes/arguments, with the reference's messages
         (flash_colsum/ops.py:59-97).
     """
+    if _native is not None:
+        out = _native.colsum(query, key, scale, is_causal, cls_len)
+        if out is not None:
+            return out if out_dtype is None or out_dtype == torch.float32 else out.to(out_dtype)
     if query.ndim != 4 or key.ndim != 4:
         raise ValueError(f"Expected 4D tensors, got query.ndim={query.ndim}, key.ndim={key.ndim}")
 
@@ -286,22 +294,16 @@ def flash_colsum(
             raise ValueError(
                 f"Query and key must have same heads and head_dim, got "
                 f"H_q={H_q}, H_k={H_k}, D_q={D_q}, D_k={D_k}")
-        out = _without_work(query, key)
-        if out is None:
-            out = _flash_colsum_causal(query, key, scale)
+        cls_n = -1
     else:
         if B_q != B_k or H_q != H_k or S_q != S_k or D_q != D_k:
             raise ValueError(
                 f"For non-causal attention, query and key must have same shape, got "
                 f"query: {query.shape}, key: {key.shape}")
         cls_n = -1 if cls_len is None else int(cls_len)
-        out = _without_work(query, key)
-        if out is not None:
-            pass
-        elif B_q == 1:
-            out = _flash_colsum_non_batched(query, key, scale, CLS_N=cls_n)
-        else:
-            out = _flash_colsum_batched(query, key, scale, CLS_N=cls_n)
+    out = _without_work(query, key)
+    if out is None:
+        out = _launch(query, key, scale, bool(is_causal), -1, cls_n, 0)
 
     if out_dtype is not None and out_dtype != out.dtype:
         out = out.to(out_dtype)
@@ -331,6 +333,10 @@ def flash_colsum_causal(
     Returns:
         (B, K_len), fp32 unless ``out_dtype`` says otherwise.
     """
+    if _native is not None and (k_past is None or k_past >= 0):
+        out = _native.launch(query, key, scale, True, -1 if k_past is None else k_past, -1, 0)
+        if out is not None:
+            return out if out_dtype is None or out_dtype == torch.float32 else out.to(out_dtype)
     if query.ndim != 4 or key.ndim != 4:
         raise ValueError(f"Expected 4D tensors, got query.ndim={query.ndim}, key.ndim={key.ndim}")
     if query.device.type != 'cuda':
@@ -346,17 +352,7 @@ def flash_colsum_causal(
     out = _without_work(query, key)
     if out is not None:
         return out if out_dtype is None else out.to(out_dtype)
-    lib = _cabi.load()
-    Q, K, code = _prepare(query, key)
-    K_len = K.shape[2]
-    with _on_device(Q.device):
-        out = torch.empty((B, K_len), device=Q.device, dtype=torch.float32)
-        ws = _workspace(lib, Q.device, B, H, Q_len, K_len, D, True, -1 if k_past is None else int(k_past))
-        _check(lib.fcs_colsum_causal_batched(
-            Q.data_ptr(), K.data_ptr(), out.data_ptr(), K_len, B, H, Q_len, K_len, D, code,
-            Q.stride(0), Q.stride(1), Q.stride(2), K.stride(0), K.stride(1), K.stride(2),
-            float(scale), -1 if k_past is None else int(k_past), 0, ws.data_ptr(), ws.numel(),
-            _status_word(Q.device).data_ptr(), _raw_stream(Q.device)))
+    out = _launch(query, key, scale, True, -1 if k_past is None else int(k_past), -1, 0)
     if out_dtype is not None and out_dtype != out.dtype:
         out = out.to(out_dtype)
     return out
@@ -425,20 +421,16 @@ def topk_columns(colsum: torch.Tensor, k: int) -> Tuple[torch.Tensor, torch.Tens
     stream without synchronising -- the pruning step of the reference's use case,
     which the reference leaves to the caller.
     """
+    if _native is not None:
+        out = _native.topk(colsum, k)
+        if out is not None:
+            return out
     if colsum.ndim != 2 or colsum.dtype != torch.float32 or colsum.device.type != "cuda":
         raise ValueError("topk_columns takes a 2-D fp32 CUDA tensor")
     B, S = colsum.shape
     if not 1 <= k <= S:
         raise ValueError(f"k must be in 1..{S}, got {k}")
-    if colsum.stride(1) != 1:
-        colsum = colsum.contiguous()
-    lib = _cabi.load()
-    with _on_device(colsum.device):
-        idx = torch.empty((B, k), dtype=torch.int32, device=colsum.device)
-        val = torch.empty((B, k), dtype=torch.float32, device=colsum.device)
-        _check(lib.fcs_select_topk(colsum.data_ptr(), colsum.stride(0), B, S, int(k), idx.data_ptr(),
-                                   val.data_ptr(), _raw_stream(colsum.device)))
-    return val, idx
+    return _load_native(colsum.device).topk(colsum, int(k))
 
 
 def threshold_columns(colsum: torch.Tensor, threshold: float, relative: bool = False
@@ -452,20 +444,15 @@ def threshold_columns(colsum: torch.Tensor, threshold: float, relative: bool = F
     ``counts[b]`` entries and -1 after them; ``counts`` is (B,) int32.  Runs on the current
     stream without synchronising (the number kept stays on the device).
     """
+    if _native is not None:
+        out = _native.threshold(colsum, threshold, relative)
+        if out is not None:
+            return out
     if colsum.ndim != 2 or colsum.dtype != torch.float32 or colsum.device.type != "cuda":
         raise ValueError("threshold_columns takes a 2-D fp32 CUDA tensor")
     if threshold != threshold:
         raise ValueError("threshold is not a number")
-    B, S = colsum.shape
-    if colsum.stride(1) != 1:
-        colsum = colsum.contiguous()
-    lib = _cabi.load()
-    with _on_device(colsum.device):
-        idx = torch.empty((B, S), dtype=torch.int32, device=colsum.device)
-        cnt = torch.empty((B,), dtype=torch.int32, device=colsum.device)
-        _check(lib.fcs_select_threshold(colsum.data_ptr(), colsum.stride(0), B, S, float(threshold), int(relative),
-                                        idx.data_ptr(), cnt.data_ptr(), _raw_stream(colsum.device)))
-    return idx, cnt
+    return _load_native(colsum.device).threshold(colsum, float(threshold), bool(relative))
 
 
 _copy_streams: Dict[int, torch.cuda.Stream] = {}
