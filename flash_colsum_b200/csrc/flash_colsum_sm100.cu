@@ -1569,6 +1569,86 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
 }
 
 // ---------------------------------------------------------------------------
+// Pruning step (select_topk.cuh): rows of at most 1024 elements take CTAs of 256 threads with
+// four elements each and 8-bit digits, longer ones 1024 threads with as few of 4, 8 or 16 elements
+// as hold a CTA's slice (a thread's elements are consecutive: with more, whole warps would have none).
+// ---------------------------------------------------------------------------
+template <typename... Params, typename... Args>
+static cudaError_t launch_row_clusters(void (*kern)(Params...), int smem, bool (&configured)[64], int B, int cl,
+                                       int threads, cudaStream_t stream, Args... args) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)((long long)B * cl));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = (unsigned)cl;
+    attrs[0].val.clusterDim.y = 1;
+    attrs[0].val.clusterDim.z = 1;
+    // the set-up may overlap the end of the kernel that produced the means; it is waited for inside
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kern, Params(args)...);
+}
+
+template <int NT, int E, int BITS, int CL>
+static cudaError_t launch_topk_t(const float* colsum, long long ld, int B, int S, int k, int* indices, float* values,
+                                 cudaStream_t stream) {
+    static bool configured[64] = {false};
+    return launch_row_clusters(sel::topk_kernel<NT, E, BITS, CL>, sel::topk_smem<NT, E, BITS>(), configured, B, CL, NT,
+                               stream, colsum, ld, S, k, indices, values);
+}
+static cudaError_t launch_topk(const float* colsum, long long ld, int B, int S, int k, int* indices, float* values,
+                               cudaStream_t stream) {
+    const int cl = sel::cluster_size(S);
+#define FCS_TOPK(NT, E, BITS, CL) return launch_topk_t<NT, E, BITS, CL>(colsum, ld, B, S, k, indices, values, stream)
+    if (S <= 1024) FCS_TOPK(256, 4, 8, 1);
+    if (cl == 1) FCS_TOPK(1024, 4, 11, 1);
+    if (cl == 2) FCS_TOPK(1024, 4, 11, 2);
+    if (cl == 4) FCS_TOPK(1024, 4, 11, 4);
+    if (cl == 8 && S <= 8 * 4096) FCS_TOPK(1024, 4, 11, 8);
+    if (cl == 8 && S <= 8 * 8192) FCS_TOPK(1024, 8, 11, 8);
+    if (cl == 8) FCS_TOPK(1024, 16, 11, 8);
+    FCS_TOPK(1024, 16, 11, 16);
+#undef FCS_TOPK
+}
+
+template <int NT, int E, int CL>
+static cudaError_t launch_threshold_t(const float* colsum, long long ld, int B, int S, float threshold, int relative,
+                                      int* indices, int* counts, cudaStream_t stream) {
+    static bool configured[64] = {false};
+    return launch_row_clusters(sel::threshold_kernel<NT, E, CL>, sel::stage_bytes<NT, E>(), configured, B, CL, NT, stream,
+                               colsum, ld, S, threshold, relative, indices, counts);
+}
+static cudaError_t launch_threshold(const float* colsum, long long ld, int B, int S, float threshold, int relative,
+                                    int* indices, int* counts, cudaStream_t stream) {
+    const int cl = sel::cluster_size(S);
+#define FCS_THRESHOLD(NT, E, CL) \
+    return launch_threshold_t<NT, E, CL>(colsum, ld, B, S, threshold, relative, indices, counts, stream)
+    if (S <= 1024) FCS_THRESHOLD(256, 4, 1);
+    if (cl == 1) FCS_THRESHOLD(1024, 4, 1);
+    if (cl == 2) FCS_THRESHOLD(1024, 4, 2);
+    if (cl == 4) FCS_THRESHOLD(1024, 4, 4);
+    if (cl == 8 && S <= 8 * 4096) FCS_THRESHOLD(1024, 4, 8);
+    if (cl == 8 && S <= 8 * 8192) FCS_THRESHOLD(1024, 8, 8);
+    if (cl == 8) FCS_THRESHOLD(1024, 16, 8);
+    FCS_THRESHOLD(1024, 16, 16);
+#undef FCS_THRESHOLD
+}
+
+// ---------------------------------------------------------------------------
 // Built-in scratch for callers that have no device allocator to draw from.
 // One copy lives in every device that loads this library, for the life of the
 // process.  The name below is a host-side handle in host code, not a device
@@ -1792,9 +1872,7 @@ int fcs_select_topk(const float* colsum, int64_t ld, int B, int S, int k, int* i
     if (B <= 0 || S <= 0 || ld < S)
         return fcs::fail(FCS_ERR_INVALID_ARGUMENT, "bad sizes (B=%d S=%d ld=%lld)", B, S, (long long)ld);
     if (k <= 0 || k > S) return fcs::fail(FCS_ERR_INVALID_ARGUMENT, "k must be in 1..S, got %d (S=%d)", k, S);
-    fcs::select_topk_kernel<<<B, fcs::TOPK_THREADS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        colsum, (long long)ld, S, k, indices, values);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = fcs::launch_topk(colsum, (long long)ld, B, S, k, indices, values, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fcs::fail(FCS_ERR_CUDA, "top-k selection launch failed: %s", cudaGetErrorString(e));
     return FCS_OK;
 }
@@ -1918,9 +1996,8 @@ int fcs_select_threshold(const float* colsum, int64_t ld, int B, int S, float th
     if (B <= 0 || S <= 0 || ld < S)
         return fcs::fail(FCS_ERR_INVALID_ARGUMENT, "bad sizes (B=%d S=%d ld=%lld)", B, S, (long long)ld);
     if (!(threshold == threshold)) return fcs::fail(FCS_ERR_INVALID_ARGUMENT, "threshold is not a number");
-    fcs::select_threshold_kernel<<<B, fcs::TOPK_THREADS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        colsum, (long long)ld, S, threshold, relative ? 1 : 0, indices, counts);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = fcs::launch_threshold(colsum, (long long)ld, B, S, threshold, relative ? 1 : 0, indices, counts,
+                                                reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fcs::fail(FCS_ERR_CUDA, "threshold selection launch failed: %s", cudaGetErrorString(e));
     return FCS_OK;
 }

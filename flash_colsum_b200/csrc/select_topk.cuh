@@ -1,158 +1,390 @@
-// Token pruning on top of the column means: per batch row, the k key positions with
-// the largest mean, in ascending position order (ties go to the lower position), on
-// the stream that produced the means.  One CTA per row.
+// Token pruning on top of the column means, on the stream that produced the means: per batch
+// row the k key positions with the largest mean, or those that reach a threshold, in ascending
+// position order (top-k ties go to the lower position).
 //
-// Exact selection by radix: four passes over the row, most significant byte first,
-// each counting the byte values of the elements that still match the prefix chosen so
-// far; after the fourth pass the k-th largest value is known exactly, together with
-// how many elements equal to it are still needed.  A last ordered pass writes the
-// positions of everything above that value plus the first of the equal ones.  The row
-// (at most a few hundred KiB) stays in L2 between passes.
+// A row belongs to one thread-block cluster of 1, 2, 4, 8 or 16 CTAs, each of which holds a
+// contiguous slice of it: the row is read once, through shared memory into registers (a thread
+// holds `E` consecutive elements), and everything after that is on chip.  Only slices of more
+// than 16384 elements (rows past 262144) are read again, from L2, by every pass.
+//
+//   top-k      exact radix selection, 11 bits at a time from the top (8 for rows of at most
+//              1024, where scanning 2048 bins costs more than a fourth pass): every CTA
+//              counts its elements that still match the prefix chosen so far, sums its bins in
+//              groups of 32, and one warp of every CTA reads the group sums of all CTAs
+//              through distributed shared memory, finds the group and then the bin the k-th
+//              largest falls into -- every CTA for itself, so that a pass has one
+//              cluster barrier.  A bin that is wanted whole ends the selection early.
+//   threshold  (with `relative`: against a share of the row's average) a comparison per element.
+//   both       one scan over the block of the kept elements per thread, the counts of the CTAs
+//              exchanged once, and every kept element knows its place in the output.
+//
+// What bounds it: a dozen dependent steps of half a microsecond to one (launch of the cluster,
+// load, cluster barriers, scans), not bytes.  Back to back on a B200, one CTA per row going over
+// it from L2 with an element per thread and step (the form before) against this one: the 16384
+// largest of 131072 216 -> 14.6 us, 2048 of 16384 32 -> 7.5, 32 rows of 65536 118 -> 31; values
+// above the mean, 131072 122 -> 11.6 us, 32 rows of 65536 64 -> 13.6.  Rows of a few thousand are
+// bound by the host (4.4 us a call).  Four copies of the first pass's bins, against lanes meeting
+// on one bin, were no faster (14.9 us): the hardware adds equal addresses of a warp in one go.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "colsum_small_q.cuh"
+#include "sm100_ptx.cuh"
+
 namespace fcs {
+namespace sel {
 
-constexpr int TOPK_THREADS = 1024;
+constexpr int MAX_CL = 16;         // (above eight: an opt-in of the launch)
 
-// Order-preserving map from float to unsigned (larger float -> larger key).
-__device__ __forceinline__ uint32_t topk_key(float v) {
-    const uint32_t u = __float_as_uint(v);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+// Order-reversing map from float to unsigned (larger float -> smaller key), and its inverse.
+__device__ __forceinline__ uint32_t key_of(uint32_t bits) {
+    return (bits & 0x80000000u) ? bits : ~(bits | 0x80000000u);
+}
+__device__ __forceinline__ uint32_t bits_of(uint32_t key) {
+    return (key & 0x80000000u) ? key : ~key & 0x7fffffffu;
+}
+__device__ __forceinline__ uint32_t ld_peer_u32(uint32_t local_addr, uint32_t rank) {
+    uint32_t addr, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+// The sum over the first `n` of the cluster's CL CTAs of the word at `local_addr` in each, all loads in
+// flight at once (a loop over a runtime count waits for each: half a microsecond more per pass).
+template <int CL>
+__device__ __forceinline__ uint32_t sum_over_cluster(uint32_t local_addr, uint32_t n = CL) {
+    uint32_t v[CL], sum = 0;
+#pragma unroll
+    for (int r = 0; r < CL; ++r) v[r] = (uint32_t)r < n ? ld_peer_u32(local_addr, (uint32_t)r) : 0u;
+#pragma unroll
+    for (int r = 0; r < CL; ++r) sum += v[r];
+    return sum;
+}
+__device__ __forceinline__ void cluster_sync() {
+    smallq_cluster_arrive();
+    smallq_cluster_wait();
+}
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v, int lane) {   // inclusive
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    return v;
 }
 
-__global__ void __launch_bounds__(TOPK_THREADS)
-select_topk_kernel(const float* __restrict__ colsum, long long ld, int S, int k, int* __restrict__ indices,
-                   float* __restrict__ values) {
-    __shared__ unsigned hist[256];
-    __shared__ unsigned sh_prefix, sh_need;
-    __shared__ unsigned warp_gt[TOPK_THREADS / 32], warp_eq[TOPK_THREADS / 32];
-    __shared__ unsigned run_out, run_eq;
-    const float* row = colsum + (long long)blockIdx.x * ld;
-    int* out_idx = indices + (long long)blockIdx.x * k;
-    float* out_val = values ? values + (long long)blockIdx.x * k : nullptr;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+// One CTA's part of a row: elements [lo, hi), in tiles of NT * E.
+template <int NT, int E>
+struct Slice {
+    static constexpr int TILE_ELEMS = NT * E;
+    static constexpr int PITCH = E + 1;             // a thread's run in shared memory, conflict-free
+    const uint32_t* row;
+    uint32_t* stage;                                // [NT * PITCH]
+    uint32_t lo, hi;
+    int tiles;
 
-    // ---- the k-th largest key, byte by byte
-    unsigned prefix = 0, need = (unsigned)k;   // still to take among the elements matching `prefix`
-    for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 24 - 8 * pass;
-        const unsigned mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-        if (tid < 256) hist[tid] = 0;
-        __syncthreads();
-        for (int i = tid; i < S; i += TOPK_THREADS) {
-            const uint32_t key = topk_key(row[i]);
-            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        if (tid == 0) {
-            unsigned above = 0;
-            int d = 255;
-            for (; d > 0; --d) {
-                if (above + hist[d] >= need) break;
-                above += hist[d];
-            }
-            sh_prefix = prefix | ((unsigned)d << shift);
-            sh_need = need - above;
-        }
-        __syncthreads();
-        prefix = sh_prefix;
-        need = sh_need;
-        __syncthreads();
+    __device__ void init(const float* row_, uint32_t* stage_, int S, int cl, uint32_t rank) {
+        row = reinterpret_cast<const uint32_t*>(row_);
+        stage = stage_;
+        const uint32_t n = (uint32_t)S, per = (n + cl - 1) / cl;
+        lo = rank * per < n ? rank * per : n;
+        hi = n - lo < per ? n : lo + per;
+        tiles = (int)((per + TILE_ELEMS - 1) / TILE_ELEMS);
     }
-    const uint32_t kth = prefix;   // exact key of the k-th largest element; `need` equal ones are wanted
+    __device__ uint32_t first(int tile) const { return lo + (uint32_t)tile * TILE_ELEMS + threadIdx.x * E; }
+    // This thread's E consecutive elements of a tile, as bits.  (Elements at hi and past it are undefined.)
+    __device__ void load(int tile, uint32_t (&v)[E]) const {
+        const uint32_t base = lo + (uint32_t)tile * TILE_ELEMS;
+        uint32_t t[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const uint32_t i = base + j * NT + threadIdx.x;
+            t[j] = i < hi ? row[i] : 0u;
+        }
+        if (tile > 0) __syncthreads();              // (the tile before has been taken out of the stage)
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const int at = j * NT + (int)threadIdx.x;
+            stage[at + at / E] = t[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = stage[(int)threadIdx.x * PITCH + j];
+    }
+};
 
-    // ---- positions in ascending order: everything above kth, and the first `need` equal to it
-    if (tid == 0) { run_out = 0; run_eq = 0; }
+// Exclusive scan over the block of one packed count per thread; `total` is the block's sum.
+template <int NT>
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* warp_sums, uint32_t& total) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t inc = warp_scan(v, lane);
+    __syncthreads();                                // (warp_sums of the scan before have been read)
+    if (lane == 31) warp_sums[wid] = inc;
     __syncthreads();
-    for (int base = 0; base < S; base += TOPK_THREADS) {
-        const int i = base + tid;
-        uint32_t key = 0;
-        float v = 0.f;
-        bool gt = false, eq = false;
-        if (i < S) {
-            v = row[i];
-            key = topk_key(v);
-            gt = key > kth;
-            eq = key == kth;
-        }
-        const unsigned m_gt = __ballot_sync(0xffffffffu, gt), m_eq = __ballot_sync(0xffffffffu, eq);
-        if (lane == 0) { warp_gt[wid] = __popc(m_gt); warp_eq[wid] = __popc(m_eq); }
-        __syncthreads();
-        unsigned gt_before = 0, eq_before = 0;   // in earlier warps of this chunk
-        for (int w = 0; w < wid; ++w) { gt_before += warp_gt[w]; eq_before += warp_eq[w]; }
-        const unsigned lower = (1u << lane) - 1u;
-        gt_before += __popc(m_gt & lower);
-        eq_before += __popc(m_eq & lower);
-        const unsigned eq_seen = run_eq + eq_before;            // equal elements before this one in the row
-        const unsigned eq_taken_before = eq_seen < need ? eq_seen : need;
-        const bool take = gt || (eq && eq_seen < need);
-        if (take) {
-            // taken elements before this one: all greater ones, and the equal ones still within `need`
-            const unsigned chunk_eq_taken = eq_taken_before - (run_eq < need ? run_eq : need);
-            const unsigned pos = run_out + gt_before + chunk_eq_taken;
-            out_idx[pos] = i;
-            if (out_val) out_val[pos] = v;
-        }
-        __syncthreads();
-        if (tid == TOPK_THREADS - 1) {
-            const unsigned chunk_gt = gt_before + (gt ? 1u : 0u);
-            const unsigned chunk_eq = eq_before + (eq ? 1u : 0u);
-            const unsigned eq_old = run_eq < need ? run_eq : need;
-            const unsigned eq_new_total = run_eq + chunk_eq;
-            const unsigned eq_new = eq_new_total < need ? eq_new_total : need;
-            run_out += chunk_gt + (eq_new - eq_old);
-            run_eq = eq_new_total;
-        }
-        __syncthreads();
-    }
+    const uint32_t w = lane < NT / 32 ? warp_sums[lane] : 0u;
+    const uint32_t ws = warp_scan(w, lane);
+    total = __shfl_sync(0xffffffffu, ws, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, ws, wid == 0 ? 0 : wid - 1);
+    return inc - v + (wid == 0 ? 0u : before);
 }
 
-// The threshold form of the pruning step: per batch row, the positions whose column mean is at
-// least `threshold` (relative = 0) or at least `threshold` times the row's mean value
-// (relative = 1; the means of a row sum to one, so that is threshold / S), ascending, written to
-// indices[row][0 .. counts[row]); the rest of the row of `indices` is filled with -1.
-__global__ void __launch_bounds__(TOPK_THREADS)
-select_threshold_kernel(const float* __restrict__ colsum, long long ld, int S, float threshold, int relative,
-                        int* __restrict__ indices, int* __restrict__ counts) {
-    __shared__ unsigned warp_n[TOPK_THREADS / 32];
-    __shared__ unsigned run_out;
-    __shared__ float warp_sum[TOPK_THREADS / 32];
-    const float* row = colsum + (long long)blockIdx.x * ld;
-    int* out_idx = indices + (long long)blockIdx.x * S;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+template <int NT, int E>
+constexpr int stage_bytes() { return NT * (E + 1) * 4; }
+template <int BITS>
+struct Digits {
+    static constexpr int BINS = 1 << BITS, GROUPS = BINS / 32, PASSES = (32 + BITS - 1) / BITS;
+};
+template <int NT, int E, int BITS>
+constexpr int topk_smem() {
+    return stage_bytes<NT, E>() + Digits<BITS>::PASSES * (Digits<BITS>::BINS + Digits<BITS>::GROUPS) * 4;
+}
+
+template <int NT, int E, int BITS, int CL>
+__global__ void __launch_bounds__(NT)
+topk_kernel(const float* __restrict__ colsum, long long ld, int S, int k, int* __restrict__ indices,
+            float* __restrict__ values) {
+    constexpr int BINS = Digits<BITS>::BINS, GROUPS = Digits<BITS>::GROUPS, PASSES = Digits<BITS>::PASSES;
+    constexpr int GPL = (GROUPS + 31) / 32;         // groups per lane of the choosing warp
+    extern __shared__ __align__(16) uint32_t sel_smem[];
+    uint32_t* stage = sel_smem;
+    uint32_t* hist = sel_smem + NT * (E + 1);       // [PASSES][BINS]: a fresh one per pass, cleared once
+    uint32_t* gsum = hist + PASSES * BINS;          // [PASSES][GROUPS]
+    __shared__ uint32_t warp_sums[32];
+    __shared__ uint32_t totals[2];                  // this CTA's elements before the k-th's bin / in it
+    __shared__ uint32_t choice[3];                  // digit, elements before its bin, elements in it
+    const uint32_t rank = smallq_cluster_rank();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long b = blockIdx.x / CL;
+
+    for (int i = threadIdx.x; i < PASSES * BINS; i += NT) hist[i] = 0u;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    Slice<NT, E> sl;
+    sl.init(colsum + b * ld, stage, S, CL, rank);
+    uint32_t key[E];
+    auto fetch = [&](int tile) {
+        sl.load(tile, key);
+#pragma unroll
+        for (int j = 0; j < E; ++j) key[j] = key_of(key[j]);
+    };
+    const bool resident = sl.tiles == 1;
+    if (resident) fetch(0);
+    else __syncthreads();                           // (the bins are clear)
+
+    // ---- the k-th smallest key, BITS bits at a time
+    uint32_t prefix = 0, mask = 0, need = (uint32_t)k;   // `need`: still to take among the elements matching `prefix`
+    for (int pass = 0; pass < PASSES; ++pass) {
+        const int shift = 32 - BITS * (pass + 1) > 0 ? 32 - BITS * (pass + 1) : 0;
+        const uint32_t digits = pass == PASSES - 1 ? (1u << (32 - BITS * pass)) - 1u : (uint32_t)(BINS - 1);
+        uint32_t* h = hist + pass * BINS;
+        uint32_t* gs = gsum + pass * GROUPS;
+        for (int tile = 0; tile < sl.tiles; ++tile) {
+            if (!resident) fetch(tile);
+            const uint32_t i0 = sl.first(tile);
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+                if (i0 + j < sl.hi && (key[j] & mask) == prefix) atomicAdd(&h[(key[j] >> shift) & digits], 1u);
+        }
+        __syncthreads();
+        for (int g = wid; g < GROUPS; g += NT / 32) {
+            uint32_t v = h[g * 32 + lane];
+            v = __reduce_add_sync(0xffffffffu, v);
+            if (lane == 0) gs[g] = v;
+        }
+        if constexpr (CL > 1) cluster_sync(); else __syncthreads();
+        if (wid == 0) {
+            uint32_t gv[GPL], sum = 0;
+#pragma unroll
+            for (int i = 0; i < GPL; ++i) {
+                const int g = lane * GPL + i;
+                gv[i] = g < GROUPS ? sum_over_cluster<CL>(smem_u32(gs + g)) : 0u;
+                sum += gv[i];
+            }
+            const uint32_t inc = warp_scan(sum, lane);
+            const int f = __ffs(__ballot_sync(0xffffffffu, inc >= need)) - 1;
+            uint32_t before = inc - sum;            // (of lane f, below)
+            int g = lane * GPL;
+#pragma unroll
+            for (int i = 0; i + 1 < GPL; ++i)
+                if (before + gv[i] < need && g == lane * GPL + i) { before += gv[i]; ++g; }
+            g = __shfl_sync(0xffffffffu, g, f);
+            before = __shfl_sync(0xffffffffu, before, f);
+            const uint32_t v = sum_over_cluster<CL>(smem_u32(h + g * 32 + lane));
+            const uint32_t vi = before + warp_scan(v, lane);
+            const int d = __ffs(__ballot_sync(0xffffffffu, vi >= need)) - 1;
+            if (lane == d) { choice[0] = (uint32_t)(g * 32 + d); choice[1] = vi - v; choice[2] = v; }
+        }
+        __syncthreads();
+        prefix |= choice[0] << shift;
+        mask |= digits << shift;
+        need -= choice[1];
+        const bool whole = choice[2] == need;       // every element of the bin is wanted
+        if (whole) break;
+    }
+
+    // ---- how many elements of the row precede this CTA's: below the prefix, and matching it
+    auto counts = [&](int tile) {
+        uint32_t c = 0;
+        const uint32_t i0 = sl.first(tile);
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const uint32_t m = key[j] & mask;
+            if (i0 + j < sl.hi) c += m < prefix ? 1u : m == prefix ? 0x10000u : 0u;
+        }
+        return c;
+    };
+    uint32_t scan = 0, tile_total = 0, n_lt = 0, n_eq = 0;   // (counts of a tile fit 16 bits each: at most NT * E = 16384)
+    for (int tile = 0; tile < sl.tiles; ++tile) {
+        if (!resident) fetch(tile);
+        scan = block_scan<NT>(counts(tile), warp_sums, tile_total);
+        n_lt += tile_total & 0xffffu;
+        n_eq += tile_total >> 16;
+    }
+    uint32_t lt0 = 0, eq0 = 0;
+    if constexpr (CL > 1) {
+        if (threadIdx.x == 0) { totals[0] = n_lt; totals[1] = n_eq; }
+        cluster_sync();
+        lt0 = sum_over_cluster<CL>(smem_u32(&totals[0]), rank);
+        eq0 = sum_over_cluster<CL>(smem_u32(&totals[1]), rank);
+        smallq_cluster_arrive();                    // nobody leaves before its peers have read its counts
+    }
+    int* out_idx = indices + b * k;
+    float* out_val = values ? values + b * k : nullptr;
+    for (int tile = 0; tile < sl.tiles; ++tile) {
+        if (!resident) {
+            fetch(tile);
+            scan = block_scan<NT>(counts(tile), warp_sums, tile_total);
+        }
+        uint32_t lt = lt0 + (scan & 0xffffu), eq = eq0 + (scan >> 16);
+        const uint32_t i0 = sl.first(tile);
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const uint32_t m = key[j] & mask;
+            const bool in = i0 + j < sl.hi, below = in && m < prefix, equal = in && m == prefix;
+            if (below || (equal && eq < need)) {
+                const uint32_t pos = lt + (eq < need ? eq : need);
+                out_idx[pos] = (int)(i0 + j);
+                if (out_val) out_val[pos] = __uint_as_float(bits_of(key[j]));
+            }
+            lt += below ? 1u : 0u;
+            eq += equal ? 1u : 0u;
+        }
+        lt0 += tile_total & 0xffffu;
+        eq0 += tile_total >> 16;
+    }
+    if constexpr (CL > 1) smallq_cluster_wait();
+}
+
+// The threshold form: positions whose column mean is at least `threshold` (relative = 0) or at
+// least `threshold` times the row's mean value (relative = 1; the means of a row sum to one, so
+// that is threshold / S), ascending, in indices[row][0 .. counts[row]); the rest of the row of
+// `indices` is filled with -1.
+//
+// The row sum is added up in one fixed order whatever the cluster size -- 1024 strided partial
+// sums, each in index order, then a tree over 32 and a run over 32 -- so that a value that ties
+// with the threshold to the last bit is kept or not by the same arithmetic everywhere.
+constexpr int SUM_LANES = 1024;
+
+template <int NT, int E, int CL>
+__global__ void __launch_bounds__(NT)
+threshold_kernel(const float* __restrict__ colsum, long long ld, int S, float threshold, int relative,
+                 int* __restrict__ indices, int* __restrict__ counts_out) {
+    extern __shared__ __align__(16) uint32_t sel_smem[];
+    __shared__ uint32_t warp_sums[32];
+    __shared__ uint32_t totals[1];
+    __shared__ uint32_t part_sums[32];              // (bits) sums over 32 strided partial sums each
+    __shared__ float row_thr;
+    const uint32_t rank = smallq_cluster_rank();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long b = blockIdx.x / CL;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const float* row = colsum + b * ld;
+    Slice<NT, E> sl;
+    sl.init(row, sel_smem, S, CL, rank);
+    uint32_t v[E];
+    const bool resident = sl.tiles == 1;
+    if (resident) sl.load(0, v);
     float thr = threshold;
     if (relative) {
-        float part = 0.f;
-        for (int i = tid; i < S; i += TOPK_THREADS) part += row[i];
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) warp_sum[wid] = part;
+        // this CTA's share of the strided partial sums
+        const int lanes = SUM_LANES / CL, t0 = (int)rank * lanes;
+        for (int t = threadIdx.x; t < lanes; t += NT) {
+            float part = 0.f;
+            int i = t0 + t;
+            for (; i + 15 * SUM_LANES < S; i += 16 * SUM_LANES) {
+                float x[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] = row[i + j * SUM_LANES];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) part += x[j];
+            }
+            for (; i < S; i += SUM_LANES) part += row[i];
+            for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+            if (lane == 0) part_sums[t >> 5] = __float_as_uint(part);
+        }
+        if constexpr (CL > 1) cluster_sync(); else __syncthreads();
+        if (wid == 0) {
+            const int per = lanes / 32;             // part_sums per CTA
+            const float mine = __uint_as_float(ld_peer_u32(smem_u32(&part_sums[lane % per]), (uint32_t)(lane / per)));
+            float total = 0.f;
+            for (int w = 0; w < 32; ++w) total += __shfl_sync(0xffffffffu, mine, w);
+            if (lane == 0) row_thr = threshold * total / (float)S;
+        }
         __syncthreads();
-        float total = 0.f;
-        for (int w = 0; w < TOPK_THREADS / 32; ++w) total += warp_sum[w];
-        thr = threshold * total / (float)S;
+        thr = row_thr;
     }
-    if (tid == 0) run_out = 0;
-    __syncthreads();
-    for (int base = 0; base < S; base += TOPK_THREADS) {
-        const int i = base + tid;
-        const bool take = i < S && row[i] >= thr;
-        const unsigned m = __ballot_sync(0xffffffffu, take);
-        if (lane == 0) warp_n[wid] = __popc(m);
-        __syncthreads();
-        unsigned before = 0;
-        for (int w = 0; w < wid; ++w) before += warp_n[w];
-        before += __popc(m & ((1u << lane) - 1u));
-        if (take) out_idx[run_out + before] = i;
-        __syncthreads();
-        if (tid == TOPK_THREADS - 1) run_out += before + (take ? 1u : 0u);
-        __syncthreads();
+    auto counts = [&](int tile) {
+        uint32_t c = 0;
+        const uint32_t i0 = sl.first(tile);
+#pragma unroll
+        for (int j = 0; j < E; ++j) c += (i0 + j < sl.hi && __uint_as_float(v[j]) >= thr) ? 1u : 0u;
+        return c;
+    };
+    uint32_t scan = 0, tile_total = 0, n = 0;
+    for (int tile = 0; tile < sl.tiles; ++tile) {
+        if (!resident) sl.load(tile, v);
+        scan = block_scan<NT>(counts(tile), warp_sums, tile_total);
+        n += tile_total;
     }
-    const unsigned n = run_out;
-    for (int i = (int)n + tid; i < S; i += TOPK_THREADS) out_idx[i] = -1;
-    if (tid == 0) counts[blockIdx.x] = (int)n;
+    uint32_t before = 0, all = n;
+    if constexpr (CL > 1) {
+        if (threadIdx.x == 0) totals[0] = n;
+        cluster_sync();
+        before = sum_over_cluster<CL>(smem_u32(&totals[0]), rank);
+        all = sum_over_cluster<CL>(smem_u32(&totals[0]));
+        smallq_cluster_arrive();                    // nobody leaves before its peers have read its count
+    }
+    int* out_idx = indices + b * S;
+    for (int tile = 0; tile < sl.tiles; ++tile) {
+        if (!resident) {
+            sl.load(tile, v);
+            scan = block_scan<NT>(counts(tile), warp_sums, tile_total);
+        }
+        uint32_t pos = before + scan;
+        const uint32_t i0 = sl.first(tile);
+#pragma unroll
+        for (int j = 0; j < E; ++j)
+            if (i0 + j < sl.hi && __uint_as_float(v[j]) >= thr) out_idx[pos++] = (int)(i0 + j);
+        before += tile_total;
+    }
+    for (long long i = (long long)all + (long long)rank * NT + threadIdx.x; i < S; i += (long long)CL * NT) out_idx[i] = -1;
+    if (rank == 0 && threadIdx.x == 0) counts_out[b] = (int)all;
+    if constexpr (CL > 1) smallq_cluster_wait();
 }
 
+// CTAs per row: as many as it takes for 4096 elements each, at most eight -- or sixteen where that
+// keeps the slices in registers (more than 131072 elements; one row of 262144: 17.7 us against 38).
+// (Below that sixteen lose to eight, 12.3 against 10.7 us at 65536 elements: the cluster barriers
+// and the launch grow with the cluster.)
+inline int cluster_size(int S) {
+    const int most = S > 8 * 16384 ? MAX_CL : 8;
+    int cl = 1;
+    while (cl < most && (long long)cl * 4096 < S) cl *= 2;
+    return cl;
+}
+
+}  // namespace sel
 }  // namespace fcs
