@@ -24,8 +24,7 @@
 // The key blocks are fetched again for phase 2, last block first: what phase 1 read last is
 // what L2 still holds when the call's keys do not all fit it.  The copy warp runs ahead
 // across the exchange.  The output is
-// cleared by a small kernel in front, of which this kernel is a programmatic dependent:
-// it waits for it only before its first add.
+// cleared by a small kernel in front.
 //
 // Included by flash_colsum_sm100.cu below the streaming kernel, whose consumer-group
 // constants and per-tile functions (stats_tile, colsum_tile_ext, colsum_tile) it uses.
@@ -96,6 +95,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     float2* xch = reinterpret_cast<float2*>(smem + L::XCH_OFF);
     float* lse_buf = reinterpret_cast<float*>(smem + L::LSE_OFF);
 
+    if (clusters_pack(fp.CL)) grid_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t cr = smallq_cluster_rank();
@@ -142,6 +142,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     // every CTA of the cluster has set up its barriers once this completes; it is waited for
     // before the first store into another CTA's shared memory
     smallq_cluster_arrive();
+    grid_dependency_wait();     // the set-up is done; what follows reads the inputs and adds into the cleared output
 
     auto wait_all = [&](uint32_t bar, uint32_t parity, int code) -> bool {
         const bool ok = mbar_wait(bar, parity, abort_flag, p.status, code);
@@ -345,7 +346,6 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const int end = colsum_end_visible(p, 0) - q0;
         const float4* nl = reinterpret_cast<const float4*>(lse_buf) + q0 / 4;
         float* dst = p.out + (long long)b * p.out_ld;
-        bool out_clear = false;
         for (int i = 0; i < nblk; ++i, ++n) {
             const int kb = kb1 - 1 - i, buf = n & (NUM_TBUF - 1);
             ok = ok && mbar_wait(t_full(buf), (n >> 1) & 1, abort_flag, p.status, FCS_STATUS_WAIT_CONSUMER);
@@ -368,7 +368,6 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             }
             tc_fence_before();
             mbar_arrive(t_empty(buf));
-            if (!out_clear) { grid_dependency_wait(); out_clear = true; }   // the output has been cleared
             const int k_abs = ktg * TILE + row;
             const float v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
             // system scope: `out` may live on another GPU and take adds from several

@@ -195,15 +195,13 @@ __device__ __forceinline__ void smallq_merge(float& m, float& l, float mo, float
     m = mn;
 }
 
-// Zero the B x S valid entries of `out`; lets the kernel behind it in the stream start at once.
-__global__ void clear_rows_kernel(float* out, long long out_ld, int B, int S) {
+// Zero the B x S valid entries of `out`.
+__global__ void clear_rows_kernel(float* out, long long out_ld, long long B, long long S) {
     grid_launch_dependents();
-    const long long n = (long long)B * S;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const long long b = idx / S;
-        out[b * out_ld + (idx - b * S)] = 0.f;
-    }
+    grid_dependency_wait();
+    for (long long b = blockIdx.y; b < B; b += gridDim.y)
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < S; i += (long long)gridDim.x * blockDim.x)
+            out[b * out_ld + i] = 0.f;
 }
 
 // RMAX: compile-time bound on the query rows (1, 2 or 4); W: consumer warps (8, or 4 with four CTAs per SM;
@@ -245,10 +243,12 @@ colsum_small_q_kernel(const SmallQParams p) {
         *abort_flag = 0;
         mbar_fence_init();
     }
+    grid_launch_dependents();
     __syncthreads();
     // every CTA of the cluster has set up its barriers once this completes; it is waited for
     // before the first store into another CTA's shared memory
     smallq_cluster_arrive();
+    grid_dependency_wait();
 
     if (warp == W) {
         // ------------------------------------------------ copy issuer: runs ahead across units
@@ -300,7 +300,7 @@ colsum_small_q_kernel(const SmallQParams p) {
         // A wait that runs out raises the abort flag (later waits then give up at once) but does not
         // end the loops: all consumer warps keep meeting at the named barrier, the results are void and
         // the status word says so.
-        bool ok = true, peers_up = false, out_clear = false;
+        bool ok = true, peers_up = false;
 
         // unit `u` (the uc-th of this cluster) is finished one unit late, behind the scores of the
         // next one: by then every range's (maximum, sum) has long arrived
@@ -338,7 +338,6 @@ colsum_small_q_kernel(const SmallQParams p) {
                 }
             }
             }
-            if (!out_clear) { grid_dependency_wait(); out_clear = true; }   // the output has been cleared
             const float* sc = sc_base + (size_t)(p.bufs == 2 ? xb : 0) * sc_buf;
             float* ob = p.out + (long long)(unit / p.H) * p.out_ld + k0;
             for (int kl = threadIdx.x; kl < rows; kl += SMALLQ_CONSUMER_THREADS) {
