@@ -33,6 +33,7 @@
 #include "sm100_ptx.cuh"
 #include "schedule.h"
 #include "colsum_small_q.cuh"
+#include "colsum_few_rows.cuh"
 #include "colsum_math.cuh"
 
 #include <math.h>
@@ -910,6 +911,24 @@ static int make_tensor_map(CUtensorMap* m, const void* base, int dtype, int B, i
     return FCS_OK;
 }
 
+// The same view in boxes of `box_rows` whole rows, not swizzled: rows of D elements one after the
+// other in shared memory.
+static int make_plain_tensor_map(CUtensorMap* m, const void* base, int dtype, int B, int H, int S, int D,
+                                 int64_t sb, int64_t sh, int64_t ss, int box_rows) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return fail(FCS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)S, (cuuint64_t)H, (cuuint64_t)B};
+    cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
+    cuuint32_t box[4] = {(cuuint32_t)D, (cuuint32_t)box_rows, 1, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = enc(m, dtype == FCS_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                           4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(FCS_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+    return FCS_OK;
+}
+
 // Optional per-pass timing: when enabled, events are recorded on the caller's
 // stream around each kernel of a call.
 struct PassTimers {
@@ -1105,6 +1124,149 @@ static int launch_small_q(const void* q, const void* k, float* out, int64_t out_
                   : (bf16 ? launch_small_q_t<128, true>(sp, grid, smem, stream, clear_out)
                           : launch_small_q_t<128, false>(sp, grid, smem, stream, clear_out));
     if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "few-row kernel launch failed: %s", cudaGetErrorString(e));
+    return FCS_OK;
+}
+
+// At most four query rows with scratch to be had: the scores kernel and the columns kernel.
+template <int DK, int T, int R>
+static cudaError_t launch_few_rows_t(const CUtensorMap& tk, const few::Params& fp, int grid, cudaStream_t stream) {
+    static bool configured[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    auto kern = few::few_rows_scores_kernel<DK, T, R>;
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, few::SMEM_BYTES);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(few::THREADS);
+    cfg.dynamicSmemBytes = few::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap_previous() ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tk, fp);
+    if (e != cudaSuccess) return e;
+    const int B = fp.units / fp.H;
+    cfg.gridDim = dim3((unsigned)((fp.Sk + few::COLUMN_KEYS - 1) / few::COLUMN_KEYS), (unsigned)(B < 65535 ? B : 65535));
+    cfg.blockDim = dim3(few::COLUMN_THREADS);
+    cfg.dynamicSmemBytes = 0;
+    return cudaLaunchKernelEx(&cfg, few::few_rows_columns_kernel, fp);
+}
+template <int DK, int T, int R>
+static cudaError_t launch_few_rows_cluster_t(const CUtensorMap& tk, const few::Params& fp, int smem, cudaStream_t stream) {
+    static bool configured[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    auto kern = few::few_rows_cluster_kernel<DK, T, R>;
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, few::CLUSTER_SMEM_LIMIT);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)fp.units);
+    cfg.blockDim = dim3(few::THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = (unsigned)fp.H;
+    attrs[0].val.clusterDim.y = 1;
+    attrs[0].val.clusterDim.z = 1;
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = overlap_previous() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, tk, fp);
+}
+
+// Which form takes a call with at most four query rows.  Measured back to back on a B200, us per call in
+// clusters per batch entry / in two kernels / in clusters over key ranges (colsum_small_q.cuh; "-": it
+// does not take the call or is far behind), one CLS row over B x H x keys of 64 columns unless said:
+//     2 x 4 x 128            4.3 /  6.6 /  6.1       38 x 4 x 185           5.3 /  8.3 /  -
+//     8 x 12 x 577 strided   7.7 /  7.9 / 34         32 x 12 x 257 of 128   8.1 / 12.0 /  9.5
+//     32 x 16 x 577         18.7 / 15.2 / 12.1       64 x 12 x 197         12.0 / 12.8 /  9.9
+//     16 x 16 x 700 of 80   14.8 / 12.6 /  -         8 x 16 x 2048, 3 rows 20.7 / 16.6 / 18.0
+//     8 x 2000 of 128          - /  8.1 /  6.7       32 x 4096 of 128         - / 12.0 / 12.2
+//     32 x 32768 of 128        - / 50.4 / 60.4       the same, 4 rows         - / 64.6 / 98.6
+enum : int { FEW_CLUSTER = 0, FEW_TWO_KERNELS = 1, FEW_KEY_RANGES = 2 };
+static int few_rows_form(int B, int H, int R, int keys, int D, int row_bytes, bool dense, bool fp32, int smem, int sms) {
+    const long long units = (long long)B * H, unit_bytes = (long long)keys * row_bytes;
+    // many short units keep four CTAs on every SM busy; few bytes in all are over before two launches are
+    const bool ranges_ok = !fp32 && dense && (D == 64 || D == 128);
+    const bool many_short = units >= 2 * sms && unit_bytes <= 80 * 1024;
+    const bool one_wave = H <= few::CLUSTER_MAX && units <= 2 * sms && smem <= few::CLUSTER_SMEM_LIMIT;
+    if (one_wave && unit_bytes <= 80 * 1024) return FEW_CLUSTER;
+    if (ranges_ok && R <= 2 && (many_short || units * unit_bytes <= (6ll << 20))) return FEW_KEY_RANGES;
+    return FEW_TWO_KERNELS;
+}
+
+static int launch_few_rows(const void* q, const void* k, float* out, int64_t out_ld, int B, int H, int R, int Sk, int D,
+                           int dtype, int64_t qsb, int64_t qsh, int64_t qss, int64_t ksb, int64_t ksh, int64_t kss,
+                           float scale, int causal, int k_past, int h_norm, int* status, cudaStream_t stream,
+                           void* (*alloc)(void*, size_t), void* alloc_ctx) {
+    few::Params fp;
+    memset(&fp, 0, sizeof(fp));
+    fp.q = q; fp.out = out; fp.out_ld = out_ld;
+    fp.H = H; fp.R = R; fp.D = D; fp.Sk = Sk;
+    fp.units = B * H;
+    // keys past the last query's horizon are seen by no row: not read, their columns are zero
+    fp.keys = causal && (long long)k_past + R < Sk ? k_past + R : Sk;
+    fp.qsb = qsb; fp.qsh = qsh; fp.qss = qss;
+    fp.c = scale * 1.4426950408889634f;
+    fp.causal = causal;
+    fp.k_past = causal ? k_past : 0;
+    fp.inv_norm = 1.0f / ((float)h_norm * (float)R);
+    fp.status = status;
+    const int sms = num_sms();
+    const bool bf16 = dtype == FCS_DTYPE_BF16;
+    CUtensorMap tk;
+    memset(&tk, 0, sizeof(tk));
+    int rc;
+    cudaError_t e;
+    const int smem = D <= 64 ? few::cluster_smem<64, few::T_FP16>(R, fp.keys) : few::cluster_smem<128, few::T_FP16>(R, fp.keys);
+    const int form = few_rows_form(B, H, R, fp.keys, D, D * 2, kss == D, false, smem, sms);
+    if (form == FEW_KEY_RANGES)
+        return launch_small_q(q, k, out, out_ld, B, H, R, Sk, D, dtype, qsb, qsh, qss, ksb, ksh, kss, scale, causal,
+                              k_past, h_norm, true, status, stream);
+    if (form == FEW_CLUSTER) {
+        const int rows = D <= 64 ? few::ClusterStage<64, few::T_FP16>::ROWS : few::ClusterStage<128, few::T_FP16>::ROWS;
+        if ((rc = make_plain_tensor_map(&tk, k, dtype, B, H, Sk, D, ksb, ksh, kss, rows)) != FCS_OK) return rc;
+        e = D <= 64 ? (bf16 ? launch_few_rows_cluster_t<64, few::T_BF16, 4>(tk, fp, smem, stream)
+                            : launch_few_rows_cluster_t<64, few::T_FP16, 4>(tk, fp, smem, stream))
+                    : (bf16 ? launch_few_rows_cluster_t<128, few::T_BF16, 4>(tk, fp, smem, stream)
+                            : launch_few_rows_cluster_t<128, few::T_FP16, 4>(tk, fp, smem, stream));
+        if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "few-row cluster form launch failed: %s", cudaGetErrorString(e));
+        return FCS_OK;
+    }
+    const long long total = (long long)fp.units * fp.keys;
+    long long share = (total + sms - 1) / sms;
+    if (share < few::MIN_SHARE) share = few::MIN_SHARE;
+    share = (share + 31) / 32 * 32;
+    fp.share = (int)share;
+    fp.slots = (int)((fp.keys + share - 2) / share) + 1;
+    fp.score_ld = (fp.keys + 3) / 4 * 4;
+    const size_t part_bytes = align_up((size_t)fp.units * fp.slots * few::CONSUMER_WARPS * few::MAX_ROWS * sizeof(float2), 256);
+    uint8_t* ws = static_cast<uint8_t*>(alloc(alloc_ctx, part_bytes + (size_t)fp.units * R * fp.score_ld * sizeof(float)));
+    if (!ws) return fail(FCS_ERR_WORKSPACE, "no scratch memory for the few-row form");
+    fp.part = reinterpret_cast<float2*>(ws);
+    fp.scores = reinterpret_cast<float*>(ws + part_bytes);
+    const int rows = D <= 64 ? few::Stage<64, few::T_FP16>::ROWS : few::Stage<128, few::T_FP16>::ROWS;
+    if ((rc = make_plain_tensor_map(&tk, k, dtype, B, H, Sk, D, ksb, ksh, kss, rows)) != FCS_OK) return rc;
+    const int grid = (int)((total + share - 1) / share);
+    e = D <= 64 ? (bf16 ? launch_few_rows_t<64, few::T_BF16, 4>(tk, fp, grid, stream)
+                        : launch_few_rows_t<64, few::T_FP16, 4>(tk, fp, grid, stream))
+                : (bf16 ? launch_few_rows_t<128, few::T_BF16, 4>(tk, fp, grid, stream)
+                        : launch_few_rows_t<128, few::T_FP16, 4>(tk, fp, grid, stream));
+    if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "few-row form launch failed: %s", cudaGetErrorString(e));
     return FCS_OK;
 }
 
@@ -1396,6 +1558,18 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
     if (causal && k_past < 0) k_past = Sk > Sq ? Sk - Sq : 0;
 
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+    if (passes == PASSES_BOTH && !sig && alloc && clear_out && Sq <= few::MAX_ROWS) {
+        // reported as a call whose statistics and merge passes take no time
+        PassTimers* tms = g_profiling ? timers_for_current_device() : nullptr;
+        if (tms) {
+            tms->recorded = false;
+            for (int i = 0; i < 3; ++i) cudaEventRecord(tms->ev[i], stream);
+        }
+        rc = launch_few_rows(q, k, out, out_ld, B, H, Sq, Sk, D, dtype, qsb, qsh, qss, ksb, ksh, kss, scale, causal,
+                             k_past, h_norm, status, stream, alloc, alloc_ctx);
+        if (rc == FCS_OK && tms) { cudaEventRecord(tms->ev[3], stream); tms->recorded = true; }
+        return rc;
+    }
     if (sig && passes == PASSES_BOTH && smallq_fits(Sq, Sk, D, B * H, num_sms()))
         return fail(FCS_ERR_UNSUPPORTED, "calls with at most four query rows take the few-row kernel, which does not "
                                          "signal other GPUs; order them with a barrier");
