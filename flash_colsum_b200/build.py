@@ -21,7 +21,8 @@ LIB_DIR = os.path.join(PKG, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libflash_colsum_b200.so")
 SOURCES = [os.path.join(CSRC, "flash_colsum_sm100.cu")]
 HEADERS = [os.path.join(CSRC, "sm100_ptx.cuh"), os.path.join(CSRC, "schedule.h"),
-           os.path.join(CSRC, "colsum_small_q.cuh"), os.path.join(CSRC, "colsum_few_rows.cuh"), os.path.join(CSRC, "colsum_math.cuh"),
+           os.path.join(CSRC, "colsum_small_q.cuh"), os.path.join(CSRC, "colsum_few_rows.cuh"),
+           os.path.join(CSRC, "round_fp32.cuh"), os.path.join(CSRC, "colsum_math.cuh"),
            os.path.join(CSRC, "colsum_single_pass.cuh"), os.path.join(CSRC, "select_topk.cuh"),
            os.path.join(CSRC, "colsum_fused_short.cuh"), os.path.join(CSRC, "host_api.h"),
            os.path.join(os.path.dirname(PKG), "include", "flash_colsum_b200.h")]

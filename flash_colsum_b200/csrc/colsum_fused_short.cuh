@@ -118,15 +118,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         // every CTA of the cluster sends its 128 (maximum, sum) pairs here
         mbar_arrive_expect_tx(xch_bar, (uint32_t)fp.CL * TILE * 8);
     }
-    {
-        // the key-side constant of the extra columns: every 16-byte piece is (k, k, k, 0, 0, 0, 0, 0),
-        // which reads the same under any swizzle of the pieces
-        const uint32_t k16 = p.ext_bf16 ? 0x3F80u : 0x5C00u;   // bf16 1.0 / fp16 256.0
-        uint4* ones = reinterpret_cast<uint4*>(smem + L::EXTA_OFF);
-        for (int i = threadIdx.x; i < EXT_A_BYTES / 16; i += THREADS)
-            ones[i] = make_uint4(k16 | (k16 << 16), k16, 0u, 0u);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
+    fill_ext_constant(smem + L::EXTA_OFF, p.ext_bf16 != 0);
     if (warp == PRODUCER_WARP && lane == 0) {
         prefetch_tensormap(&tm_q);
         prefetch_tensormap(&tm_k);
@@ -143,6 +135,10 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     // before the first store into another CTA's shared memory
     smallq_cluster_arrive();
     grid_dependency_wait();     // the set-up is done; what follows reads the inputs and adds into the cleared output
+    if (p.fmt) {                // the element type was decided by a kernel of this call
+        fill_ext_constant(smem + L::EXTA_OFF, *p.fmt != 0);
+        __syncthreads();
+    }
 
     auto wait_all = [&](uint32_t bar, uint32_t parity, int code) -> bool {
         const bool ok = mbar_wait(bar, parity, abort_flag, p.status, code);
@@ -175,6 +171,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         smallq_cluster_wait();      // (pairs with the arrive above; this warp stores nothing into other CTAs)
     } else if (warp == MMA_WARP) {
         // -------------------------------------------- MMA issuer
+        const uint32_t fmt_bits = p.fmt && *p.fmt ? IDESC_BF16 : 0u;
         bool ok = wait_all(q_full, 0, FCS_STATUS_WAIT_MMA);
         const uint64_t dq = umma_desc_k_sw128(q_smem);
         int n = 0;
@@ -190,7 +187,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint64_t oq = (uint64_t)(((ks >> 2) * L::Q_SLAB_BYTES + (ks & 3) * 32) >> 4);
                     const uint64_t ok_ = (uint64_t)(((ks >> 2) * L::K_SLAB_BYTES + (ks & 3) * 32) >> 4);
-                    umma_f16(d_tmem, dq + oq, dk + ok_, fp.idesc_scores, ks > 0 ? 1u : 0u);
+                    umma_f16(d_tmem, dq + oq, dk + ok_, fp.idesc_scores | fmt_bits, ks > 0 ? 1u : 0u);
                 }
                 umma_commit(k_empty(stage));
                 umma_commit(t_full(buf));
@@ -211,7 +208,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint64_t oq = (uint64_t)(((ks >> 2) * L::Q_SLAB_BYTES + (ks & 3) * 32) >> 4);
                     const uint64_t ok_ = (uint64_t)(((ks >> 2) * L::K_SLAB_BYTES + (ks & 3) * 32) >> 4);
-                    umma_f16(d_tmem, dk + ok_, dq + oq, fp.idesc_cols, ks > 0 ? 1u : 0u);
+                    umma_f16(d_tmem, dk + ok_, dq + oq, fp.idesc_cols | fmt_bits, ks > 0 ? 1u : 0u);
                 }
             }
         };
@@ -220,7 +217,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 #pragma unroll
             for (int t = 0; t < 2; ++t)
                 umma_f16(tmem_base + buf * BLOCK + t * (BLOCK / 2), umma_desc_k_sw32(smem_base + L::EXTA_OFF),
-                         umma_desc_k_sw32(smem_base + L::EXTB_OFF), fp.idesc_cols, 1u);
+                         umma_desc_k_sw32(smem_base + L::EXTB_OFF), fp.idesc_cols | fmt_bits, 1u);
         };
         const int early = nblk < NUM_TBUF ? nblk : NUM_TBUF;
         for (int e = 0; ok && e < early; ++e) {
@@ -326,7 +323,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             lse_buf[row] = nlv;
             lse_buf[TILE + row] = -INFINITY;
             uint4 e0, e1;
-            make_ext_row(nlv, p.inv_c, p.ext_bf16 != 0, e0, e1);
+            make_ext_row(nlv, p.inv_c, p.fmt ? *p.fmt != 0 : p.ext_bf16 != 0, e0, e1);
             // rows of 32 bytes under the 32-byte swizzle: the two 16-byte halves of a row
             // change places in rows 4..7 of every eight
             const int sw = (row >> 2) & 1;

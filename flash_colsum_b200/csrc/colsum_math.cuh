@@ -10,6 +10,9 @@
 
 namespace fcs {
 
+// The MMA instruction descriptor for 16-bit operands given as fp16, for bf16 ones.
+constexpr uint32_t IDESC_BF16 = (1u << 7) | (1u << 10);
+
 // Of every 16 pairs of exps on fully visible tiles, this many are evaluated by
 // the polynomial on the FMA pipe instead of the special-function unit (which
 // issues 16 results per clock per SM and is the busiest unit of both passes).

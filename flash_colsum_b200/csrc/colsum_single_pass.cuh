@@ -47,6 +47,7 @@ struct SinglePassParams {
     long long out_ld;
     int* status;
     uint32_t idesc_scores;  // 128 x 256 x 16, K-major operands
+    const int* fmt;         // NULL, or where a kernel of this call has written the operands' type (1: bf16)
     uint32_t idesc_colsum;  // 128 x 16 x 16, A = P~ (M-major), B = W (K-major), fp16
 };
 
@@ -435,6 +436,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         // in which their inputs become ready: scores(i+1) when the consumers have read scores(i)
         // out of tensor memory, column sums(i-1) only after the statistics of tile i-1 have gone
         // around the cluster.
+        const uint32_t idesc_scores = p.idesc_scores | (p.fmt && *p.fmt ? IDESC_BF16 : 0u);
         int i = 0, uc = 0, fc = 0;
         int first = 0;                // first tile of the current batch entry on this CTA
         bool ok = true, fresh = true; // fresh: the next column-sum MMAs start a new accumulation
@@ -482,7 +484,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 #pragma unroll
                         for (int ks = 0; ks < 4; ++ks)
                             umma_f16(tmem_base, dq + (uint64_t)((ks * 32) >> 4),
-                                     dk + (uint64_t)((ks * 32) >> 4), p.idesc_scores, ks > 0 ? 1u : 0u);
+                                     dk + (uint64_t)((ks * 32) >> 4), idesc_scores, ks > 0 ? 1u : 0u);
                         umma_commit(s_full);
                         umma_commit(q_empty(qs));
                         if (t + 1 == t_end) umma_commit(k_empty);

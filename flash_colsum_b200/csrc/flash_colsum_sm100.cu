@@ -35,6 +35,7 @@
 #include "colsum_small_q.cuh"
 #include "colsum_few_rows.cuh"
 #include "colsum_math.cuh"
+#include "round_fp32.cuh"
 
 #include <math.h>
 #include <stdarg.h>
@@ -160,6 +161,15 @@ __device__ __forceinline__ void colsum_tile(uint32_t taddr, const float4* nl, in
     }
 }
 
+// The key-side constant of the extension: every 16-byte piece is (k, k, k, 0, 0, 0, 0, 0), which reads
+// the same under any swizzle of the pieces.
+__device__ __forceinline__ void fill_ext_constant(uint8_t* dst, bool bf16) {
+    const uint32_t k16 = bf16 ? 0x3F80u : 0x5C00u;   // bf16 1.0 / fp16 256.0
+    uint4* ones = reinterpret_cast<uint4*>(dst);
+    for (int i = threadIdx.x; i < EXT_A_BYTES / 16; i += THREADS) ones[i] = make_uint4(k16 | (k16 << 16), k16, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // Release stores at system scope, kept out of line: with a system-scope fence or release store
 // in its own body the streaming kernel's adds into another GPU's memory run markedly slower
 // (measured on the long-context shape: 0.363 against 0.289 ms for the column pass of a rank that
@@ -228,15 +238,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         *abort_flag = 0;
         mbar_fence_init();
     }
-    if constexpr (EXT) {
-        // the key-side constant of the extension: every 16-byte piece is (k, k, k, 0, 0, 0, 0, 0),
-        // which reads the same under any swizzle of the pieces
-        const uint32_t k16 = p.ext_bf16 ? 0x3F80u : 0x5C00u;   // bf16 1.0 / fp16 256.0
-        uint4* ones = reinterpret_cast<uint4*>(smem + L::EXTA_OFF);
-        for (int i = threadIdx.x; i < EXT_A_BYTES / 16; i += THREADS)
-            ones[i] = make_uint4(k16 | (k16 << 16), k16, 0u, 0u);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
+    if constexpr (EXT) fill_ext_constant(smem + L::EXTA_OFF, p.ext_bf16 != 0);
     if (warp == PRODUCER_WARP && lane == 0) {
         prefetch_tensormap(&tm_a);
         prefetch_tensormap(&tm_b);
@@ -253,6 +255,13 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     // everything above touched only this CTA's shared and tensor memory; from here on the
     // results of the kernels before this one in the stream are read
     grid_dependency_wait();
+    if (p.fmt) {
+        // the element type was decided by a kernel of this call
+        const int bf16 = *p.fmt;
+        if constexpr (EXT) fill_ext_constant(smem + L::EXTA_OFF, bf16 != 0);
+        if (threadIdx.x == 0 && bf16) { ps.ext_bf16 = 1; ps.idesc |= IDESC_BF16; }
+        __syncthreads();
+    }
     if (MODE != MODE_STATS && (p.sig_wait || p.sig_post_n > 0)) {
         // head shards on several GPUs adding into one buffer: nothing is added before the owner of
         // the buffer has said that it is clear (a flag in this GPU's memory, written over NVLink;
@@ -400,6 +409,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             // -------------------------------------------- MMA issuer
             Items it;
             it.init(ps, blockIdx.x, gridDim.x);
+            const uint32_t idesc = ps.idesc;
             int a_cnt = 0, stage = 0, n = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -432,10 +442,10 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                                 for (int ks = 0; ks < D / 16; ++ks) {
                                     const uint64_t oa = (uint64_t)(((ks >> 2) * L::A_SLAB_BYTES + (ks & 3) * 32) >> 4);
                                     const uint64_t ob = (uint64_t)(((ks >> 2) * L::B_SLAB_BYTES + (ks & 3) * 32) >> 4);
-                                    umma_f16(d_tmem, da + oa, db + ob, p.idesc, ks > 0 ? 1u : 0u);
+                                    umma_f16(d_tmem, da + oa, db + ob, idesc, ks > 0 ? 1u : 0u);
                                 }
                                 umma_f16(d_tmem, umma_desc_k_sw32(smem_base + L::EXTA_OFF),
-                                         umma_desc_k_sw32(b_smem + st * L::B_STAGE_BYTES + L::B_BYTES), p.idesc, 1u);
+                                         umma_desc_k_sw32(b_smem + st * L::B_STAGE_BYTES + L::B_BYTES), idesc, 1u);
                                 umma_commit(t_full(buf));
                                 if (st + 1 == it.s1) umma_commit(a_empty(ab));
                             }
@@ -459,10 +469,10 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                             for (int ks = 0; ks < D / 16; ++ks) {
                                 const uint64_t oa = (uint64_t)(((ks >> 2) * L::A_SLAB_BYTES + (ks & 3) * 32) >> 4);
                                 const uint64_t ob = (uint64_t)(((ks >> 2) * L::B_SLAB_BYTES + (ks & 3) * 32) >> 4);
-                                umma_f16(d_tmem, da + oa, db + ob, p.idesc, ks > 0 ? 1u : 0u);
+                                umma_f16(d_tmem, da + oa, db + ob, idesc, ks > 0 ? 1u : 0u);
                             }
                             umma_f16(d_tmem, umma_desc_k_sw32(smem_base + L::EXTA_OFF),
-                                     umma_desc_k_sw32(b_smem + L::B_BYTES), p.idesc, 1u);
+                                     umma_desc_k_sw32(b_smem + L::B_BYTES), idesc, 1u);
                             umma_commit(a_empty(ab));
                             if (t + 1 == it.nt) umma_commit(t_full(buf));
                         }
@@ -488,11 +498,11 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                             // 32 bytes per 16-element step inside a slab
                             const uint64_t oa = (uint64_t)(((ks >> 2) * L::A_SLAB_BYTES + (ks & 3) * 32) >> 4);
                             const uint64_t ob = (uint64_t)(((ks >> 2) * L::B_SLAB_BYTES + (ks & 3) * 32) >> 4);
-                            umma_f16(d_tmem, da + oa, db + ob, p.idesc, ks > 0 ? 1u : 0u);
+                            umma_f16(d_tmem, da + oa, db + ob, idesc, ks > 0 ? 1u : 0u);
                         }
                         if constexpr (EXT)   // + (key-side constant) x (-(lse)/c parts of the queries)
                             umma_f16(d_tmem, umma_desc_k_sw32(smem_base + L::EXTA_OFF),
-                                     umma_desc_k_sw32(b_smem + stage * L::B_STAGE_BYTES + L::B_BYTES), p.idesc, 1u);
+                                     umma_desc_k_sw32(b_smem + stage * L::B_STAGE_BYTES + L::B_BYTES), idesc, 1u);
                         umma_commit(b_empty(stage));
                         umma_commit(t_full(buf));
                         if (st + 1 == it.s1) umma_commit(a_empty(ab));
@@ -561,7 +571,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 const float nlv = (q_abs < p.Sq) ? -(mm + log2f(ll) + p.log2_norm) : -INFINITY;
                 p.neg_lse[bh * p.lse_rows + q_abs] = nlv;
                 uint4 e0, e1;
-                make_ext_row(nlv, p.inv_c, p.ext_bf16 != 0, e0, e1);
+                make_ext_row(nlv, p.inv_c, ps.ext_bf16 != 0, e0, e1);
                 uint4* er = reinterpret_cast<uint4*>(p.ext) + (bh * p.lse_rows + q_abs) * 2;
                 er[0] = e0;
                 er[1] = e1;
@@ -802,7 +812,7 @@ __global__ void merge_stats_kernel(const Problem p) {
         }
         p.neg_lse[bh * p.lse_rows + q_abs] = v;
         uint4 e0, e1;
-        make_ext_row(v, p.inv_c, p.ext_bf16 != 0, e0, e1);
+        make_ext_row(v, p.inv_c, p.fmt ? *p.fmt != 0 : p.ext_bf16 != 0, e0, e1);
         uint4* er = reinterpret_cast<uint4*>(p.ext) + (bh * p.lse_rows + q_abs) * 2;
         er[0] = e0;
         er[1] = e1;
@@ -918,10 +928,13 @@ static int make_plain_tensor_map(CUtensorMap* m, const void* base, int dtype, in
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return fail(FCS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)S, (cuuint64_t)H, (cuuint64_t)B};
-    cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
+    const int es = dtype == FCS_DTYPE_FP32 ? 4 : 2;
+    cuuint64_t strides[3] = {(cuuint64_t)ss * es, (cuuint64_t)sh * es, (cuuint64_t)sb * es};
     cuuint32_t box[4] = {(cuuint32_t)D, (cuuint32_t)box_rows, 1, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
-    const CUresult r = enc(m, dtype == FCS_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+    const CUresult r = enc(m, dtype == FCS_DTYPE_FP32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                              : dtype == FCS_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                        : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                            4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1029,13 +1042,13 @@ static int launch_clear(float* out, long long out_ld, long long B, long long S, 
 // 64-column slabs.
 static bool head_dim_ok(int D) { return D >= 8 && D <= 128 && D % 8 == 0; }
 
-static int check_operand(const char* name, const void* ptr, int64_t sb, int64_t sh, int64_t ss) {
+static int check_operand(const char* name, const void* ptr, int64_t sb, int64_t sh, int64_t ss, int granule = 8) {
     if (!ptr) return fail(FCS_ERR_INVALID_ARGUMENT, "%s is NULL", name);
     if (reinterpret_cast<uintptr_t>(ptr) % 16)
         return fail(FCS_ERR_INVALID_ARGUMENT, "%s must be 16-byte aligned", name);
-    if (sb <= 0 || sh <= 0 || ss <= 0 || sb % 8 || sh % 8 || ss % 8)
+    if (sb <= 0 || sh <= 0 || ss <= 0 || sb % granule || sh % granule || ss % granule)
         return fail(FCS_ERR_INVALID_ARGUMENT,
-                    "%s strides must be positive multiples of 8 elements (got b=%lld h=%lld s=%lld)", name,
+                    "%s strides must be positive multiples of %d elements (got b=%lld h=%lld s=%lld)", name, granule,
                     (long long)sb, (long long)sh, (long long)ss);
     return FCS_OK;
 }
@@ -1227,20 +1240,29 @@ static int launch_few_rows(const void* q, const void* k, float* out, int64_t out
     fp.inv_norm = 1.0f / ((float)h_norm * (float)R);
     fp.status = status;
     const int sms = num_sms();
-    const bool bf16 = dtype == FCS_DTYPE_BF16;
+    const bool bf16 = dtype == FCS_DTYPE_BF16, fp32 = dtype == FCS_DTYPE_FP32;
     CUtensorMap tk;
     memset(&tk, 0, sizeof(tk));
     int rc;
     cudaError_t e;
-    const int smem = D <= 64 ? few::cluster_smem<64, few::T_FP16>(R, fp.keys) : few::cluster_smem<128, few::T_FP16>(R, fp.keys);
-    const int form = few_rows_form(B, H, R, fp.keys, D, D * 2, kss == D, false, smem, sms);
+    const int smem = fp32 ? (D <= 64 ? few::cluster_smem<64, few::T_FP32>(R, fp.keys) : few::cluster_smem<128, few::T_FP32>(R, fp.keys))
+                     : D <= 64 ? few::cluster_smem<64, few::T_FP16>(R, fp.keys) : few::cluster_smem<128, few::T_FP16>(R, fp.keys);
+    const int form = few_rows_form(B, H, R, fp.keys, D, D * (fp32 ? 4 : 2), kss == D, fp32, smem, sms);
     if (form == FEW_KEY_RANGES)
         return launch_small_q(q, k, out, out_ld, B, H, R, Sk, D, dtype, qsb, qsh, qss, ksb, ksh, kss, scale, causal,
                               k_past, h_norm, true, status, stream);
     if (form == FEW_CLUSTER) {
-        const int rows = D <= 64 ? few::ClusterStage<64, few::T_FP16>::ROWS : few::ClusterStage<128, few::T_FP16>::ROWS;
+        const int rows = fp32      ? few::ClusterStage<64, few::T_FP32>::ROWS
+                         : D <= 64 ? few::ClusterStage<64, few::T_FP16>::ROWS
+                                   : few::ClusterStage<128, few::T_FP16>::ROWS;
         if ((rc = make_plain_tensor_map(&tk, k, dtype, B, H, Sk, D, ksb, ksh, kss, rows)) != FCS_OK) return rc;
-        e = D <= 64 ? (bf16 ? launch_few_rows_cluster_t<64, few::T_BF16, 4>(tk, fp, smem, stream)
+        if (fp32)
+            e = D <= 64 ? (R == 1 ? launch_few_rows_cluster_t<64, few::T_FP32, 1>(tk, fp, smem, stream)
+                                  : launch_few_rows_cluster_t<64, few::T_FP32, 4>(tk, fp, smem, stream))
+                        : (R == 1 ? launch_few_rows_cluster_t<128, few::T_FP32, 1>(tk, fp, smem, stream)
+                                  : launch_few_rows_cluster_t<128, few::T_FP32, 4>(tk, fp, smem, stream));
+        else
+            e = D <= 64 ? (bf16 ? launch_few_rows_cluster_t<64, few::T_BF16, 4>(tk, fp, smem, stream)
                             : launch_few_rows_cluster_t<64, few::T_FP16, 4>(tk, fp, smem, stream))
                     : (bf16 ? launch_few_rows_cluster_t<128, few::T_BF16, 4>(tk, fp, smem, stream)
                             : launch_few_rows_cluster_t<128, few::T_FP16, 4>(tk, fp, smem, stream));
@@ -1259,10 +1281,18 @@ static int launch_few_rows(const void* q, const void* k, float* out, int64_t out
     if (!ws) return fail(FCS_ERR_WORKSPACE, "no scratch memory for the few-row form");
     fp.part = reinterpret_cast<float2*>(ws);
     fp.scores = reinterpret_cast<float*>(ws + part_bytes);
-    const int rows = D <= 64 ? few::Stage<64, few::T_FP16>::ROWS : few::Stage<128, few::T_FP16>::ROWS;
+    const int rows = fp32      ? few::Stage<64, few::T_FP32>::ROWS
+                     : D <= 64 ? few::Stage<64, few::T_FP16>::ROWS
+                               : few::Stage<128, few::T_FP16>::ROWS;
     if ((rc = make_plain_tensor_map(&tk, k, dtype, B, H, Sk, D, ksb, ksh, kss, rows)) != FCS_OK) return rc;
     const int grid = (int)((total + share - 1) / share);
-    e = D <= 64 ? (bf16 ? launch_few_rows_t<64, few::T_BF16, 4>(tk, fp, grid, stream)
+    if (fp32)
+        e = D <= 64 ? (R == 1 ? launch_few_rows_t<64, few::T_FP32, 1>(tk, fp, grid, stream)
+                              : launch_few_rows_t<64, few::T_FP32, 4>(tk, fp, grid, stream))
+                    : (R == 1 ? launch_few_rows_t<128, few::T_FP32, 1>(tk, fp, grid, stream)
+                              : launch_few_rows_t<128, few::T_FP32, 4>(tk, fp, grid, stream));
+    else
+        e = D <= 64 ? (bf16 ? launch_few_rows_t<64, few::T_BF16, 4>(tk, fp, grid, stream)
                         : launch_few_rows_t<64, few::T_FP16, 4>(tk, fp, grid, stream))
                 : (bf16 ? launch_few_rows_t<128, few::T_BF16, 4>(tk, fp, grid, stream)
                         : launch_few_rows_t<128, few::T_FP16, 4>(tk, fp, grid, stream));
@@ -1327,7 +1357,7 @@ static int single_pass_max_clusters(int cl) {
 
 static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, float* out, int64_t out_ld, int B,
                               int H, int Sq, int Sk, float scale, int h_norm, int dtype, bool clear_out,
-                              int max_clusters, int* status, cudaStream_t stream) {
+                              int max_clusters, int* status, const int* fmt_word, cudaStream_t stream) {
     if (clear_out) {
         const int rc = launch_clear(out, out_ld, B, Sk, stream);
         if (rc != FCS_OK) return rc;
@@ -1350,6 +1380,7 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
     sp_.out = out;
     sp_.out_ld = out_ld;
     sp_.status = status;
+    sp_.fmt = fmt_word;
     const uint32_t fmt = dtype == FCS_DTYPE_BF16 ? 1u : 0u;
     // one score MMA covers the 256 keys of the slice: M = 128, N = 256
     sp_.idesc_scores = (1u << 4) | (fmt << 7) | (fmt << 10) | ((scale < 0.f ? 1u : 0u) << 13) |
@@ -1499,6 +1530,44 @@ static int launch_fused_short(const CUtensorMap& tq, const CUtensorMap& tk, cons
     return FCS_OK;
 }
 
+// fp32 operands rounded into `q16` / `k16` (dense [B][H][rows][D]); `fmt` receives the type.
+static int launch_round_fp32(const float* q, const float* k, void* q16, void* k16, int* notes, int n_notes, int* fmt, int B,
+                             int H, int Sq, int Sk, int D, int64_t qsb, int64_t qsh, int64_t qss, int64_t ksb, int64_t ksh,
+                             int64_t kss, cudaStream_t stream) {
+    rnd::Params rp;
+    memset(&rp, 0, sizeof(rp));
+    auto operand = [&](rnd::Operand& o, const float* src, void* dst, int rows, int64_t sb, int64_t sh, int64_t ss) {
+        o.src = src;
+        o.dst = static_cast<uint16_t*>(dst);
+        o.rows = (unsigned)rows;
+        o.H = (unsigned)H;
+        o.d8 = (unsigned)(D / 8);
+        o.pieces = (unsigned)((long long)B * H * rows * (D / 8));
+        o.sb = sb; o.sh = sh; o.ss = ss;
+        o.dense = ss == D && sh == (int64_t)rows * D && sb == (int64_t)H * rows * D;
+        return (long long)B * H * rows * (D / 8) <= 0xffffffffll;
+    };
+    if (!operand(rp.op[0], q, q16, Sq, qsb, qsh, qss) || !operand(rp.op[1], k, k16, Sk, ksb, ksh, kss))
+        return fail(FCS_ERR_UNSUPPORTED, "fp32 operands of more than 2^35 elements are not supported");
+    rp.notes = notes;
+    rp.n_notes = n_notes;
+    rp.fmt = fmt;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)n_notes);
+    cfg.blockDim = dim3(rnd::THREADS);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap_previous() ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, rnd::round_kernel, rp);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, rnd::settle_kernel, rp);
+    if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "rounding fp32 operands failed: %s", cudaGetErrorString(e));
+    return FCS_OK;
+}
+
 enum : int { PASSES_BOTH = 0, PASSES_STATS = 1, PASSES_COLUMNS = 2 };
 
 // -(log-sum-exp) per query row -> the 16 extension columns the column pass contracts with.
@@ -1532,7 +1601,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
         return fail(FCS_ERR_INVALID_ARGUMENT, "sizes must be positive (B=%d H=%d Sq=%d Sk=%d)", B, H, Sq_full, Sk);
     if (!head_dim_ok(D))
         return fail(FCS_ERR_UNSUPPORTED, "head dimension must be a multiple of 8 from 8 to 128, got %d", D);
-    if (dtype != FCS_DTYPE_FP16 && dtype != FCS_DTYPE_BF16)
+    if (dtype != FCS_DTYPE_FP16 && dtype != FCS_DTYPE_BF16 && !(dtype == FCS_DTYPE_FP32 && alloc))
         return fail(FCS_ERR_UNSUPPORTED, "dtype must be FCS_DTYPE_FP16 or FCS_DTYPE_BF16, got %d", dtype);
     const int DK = D <= 64 ? 64 : 128;   // columns the streaming kernels contract (zero-filled beyond D)
     if (passes != PASSES_STATS) {
@@ -1549,8 +1618,9 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
     if (!causal && cls_n != -1 && cls_n <= 0)
         return fail(FCS_ERR_INVALID_ARGUMENT, "cls_n must be -1 or positive, got %d", cls_n);
     int rc;
-    if ((rc = check_operand("q", q, qsb, qsh, qss)) != FCS_OK) return rc;
-    if ((rc = check_operand("k", k, ksb, ksh, kss)) != FCS_OK) return rc;
+    const int granule = dtype == FCS_DTYPE_FP32 ? 4 : 8;   // 16 bytes
+    if ((rc = check_operand("q", q, qsb, qsh, qss, granule)) != FCS_OK) return rc;
+    if ((rc = check_operand("k", k, ksb, ksh, kss, granule)) != FCS_OK) return rc;
     if (h_norm <= 0) h_norm = H;
 
     int Sq = Sq_full;                       // rows that enter the mean
@@ -1569,6 +1639,28 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
                              k_past, h_norm, status, stream, alloc, alloc_ctx);
         if (rc == FCS_OK && tms) { cudaEventRecord(tms->ev[3], stream); tms->recorded = true; }
         return rc;
+    }
+    const int* fmt_word = nullptr;
+    if (dtype == FCS_DTYPE_FP32) {
+        // one allocation: the type, the notes, both operands
+        const long long pieces = (long long)B * H * ((long long)Sq + Sk) * (D / 8);
+        long long notes = (pieces + rnd::THREADS - 1) / rnd::THREADS;
+        if (notes > 8ll * num_sms()) notes = 8ll * num_sms();
+        const size_t head = align_up((size_t)(notes + 1) * sizeof(int), 256);
+        const size_t q_bytes = align_up((size_t)B * H * Sq * D * 2, 256), k_bytes = (size_t)B * H * Sk * D * 2;
+        uint8_t* ws = static_cast<uint8_t*>(alloc(alloc_ctx, head + q_bytes + k_bytes));
+        if (!ws) return fail(FCS_ERR_WORKSPACE, "no scratch memory for the rounded fp32 operands");
+        int* words = reinterpret_cast<int*>(ws);
+        rc = launch_round_fp32(static_cast<const float*>(q), static_cast<const float*>(k), ws + head, ws + head + q_bytes,
+                               words + 1, (int)notes, words, B, H, Sq, Sk, D, qsb, qsh, qss, ksb, ksh, kss, stream);
+        if (rc != FCS_OK) return rc;
+        q = ws + head;
+        k = ws + head + q_bytes;
+        qss = kss = D;
+        qsh = (int64_t)Sq * D; qsb = qsh * H;
+        ksh = (int64_t)Sk * D; ksb = ksh * H;
+        dtype = FCS_DTYPE_FP16;
+        fmt_word = words;
     }
     if (sig && passes == PASSES_BOTH && smallq_fits(Sq, Sk, D, B * H, num_sms()))
         return fail(FCS_ERR_UNSUPPORTED, "calls with at most four query rows take the few-row kernel, which does not "
@@ -1595,6 +1687,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
     memset(&p, 0, sizeof(p));
     plan(p, B, H, Sq, Sk, causal, k_past, sms, COL_INTERLEAVE_MIN_ROWS, /*head_major_ok=*/use_ext);
     p.ext_bf16 = dtype == FCS_DTYPE_BF16 ? 1 : 0;
+    p.fmt = fmt_word;
     p.out = out;
     p.out_ld = out_ld;
     p.clear_out = (clear_out && passes == PASSES_BOTH) ? 1 : 0;   // (the statistics pass does the clearing)
@@ -1631,7 +1724,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
                 for (int i = 0; i < 3; ++i) cudaEventRecord(tms->ev[i], stream);
             }
             rc = launch_single_pass(tq_a, tk_b, out, out_ld, B, H, Sq, Sk, scale, h_norm, dtype, clear_out,
-                                    max_clusters, status, stream);
+                                    max_clusters, status, fmt_word, stream);
             if (rc == FCS_OK && tms) { cudaEventRecord(tms->ev[3], stream); tms->recorded = true; }
             return rc;
         }

@@ -7,7 +7,12 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "../../include/flash_colsum_b200.h"
+
 extern "C" {
+
+// Operands that the library rounds itself (round_fp32.cuh); needs an allocator.
+enum { FCS_DTYPE_FP32 = 2 };
 
 typedef struct FcsCall {
     const void* q;
@@ -15,7 +20,7 @@ typedef struct FcsCall {
     float* out;
     int64_t out_ld;
     int B, H, Sq, Sk, D;          // Sq: query rows of the tensor
-    int dtype;                    // FCS_DTYPE_*
+    int dtype;                    // FCS_DTYPE_FP16 / _BF16 / _FP32
     int64_t q_stride[3], k_stride[3];   // batch, head, row; in elements
     float scale;
     int causal, k_past, cls_n, h_norm;  // as in fcs_colsum_causal_batched / fcs_colsum_batched

@@ -61,7 +61,8 @@ struct Problem {
     float* neg_lse;     // [B*H][lse_rows]   -(lse2 + log2_norm)
     void* ext;          // [B*H][lse_rows][16] 16-bit: neg_lse / c split into three parts (see make_ext_row)
     float inv_c;        // 1 / c
-    int ext_bf16;       // element type of `ext` (that of the inputs)
+    int ext_bf16;       // element type of the operands and of `ext`: 1 bf16, 0 fp16
+    const int* fmt;     // NULL, or where a kernel of this call has written that type (fp32 inputs, rounded on the way in)
     void* part;         // float2 [nsplit][B*H][NQ*128]   (max, sum) per key range
     float* out;
     long long out_ld;

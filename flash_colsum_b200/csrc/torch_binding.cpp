@@ -63,7 +63,7 @@ struct Scratch {
 };
 
 int dtype_code(at::ScalarType t) {
-    return t == at::kHalf ? FCS_DTYPE_FP16 : t == at::kBFloat16 ? FCS_DTYPE_BF16 : -1;
+    return t == at::kHalf ? FCS_DTYPE_FP16 : t == at::kBFloat16 ? FCS_DTYPE_BF16 : t == at::kFloat ? FCS_DTYPE_FP32 : -1;
 }
 
 // Unit inner stride, positive outer strides in multiples of 16 bytes, 16-byte aligned base.  The
@@ -78,7 +78,8 @@ void kernel_strides(const at::Tensor& t, int64_t (&st)[3]) {
 bool kernel_ready(const at::Tensor& t) {
     int64_t st[3];
     kernel_strides(t, st);
-    return t.stride(3) == 1 && st[0] > 0 && st[1] > 0 && st[2] > 0 && ((st[0] | st[1] | st[2]) & 7) == 0 &&
+    const int64_t granule = 16 / t.element_size();
+    return t.stride(3) == 1 && st[0] > 0 && st[1] > 0 && st[2] > 0 && ((st[0] | st[1] | st[2]) & (granule - 1)) == 0 &&
            (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0;
 }
 

@@ -92,30 +92,30 @@ def _round_fp32(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, t
     """fp32 inputs are rounded to 16 bits before the tensor cores see them: to fp16, whose ten
     mantissa bits are those of the TF32 format the reference's ``tl.dot`` gives fp32 operands
     (kernel_noncausal_batched.py:37,54), or to bf16 when a value lies outside fp16's range.
-    The range check reads one number back from the device (the call synchronises)."""
+    Whole calls do this on the device (csrc/round_fp32.cuh); the entry points that run a part of one
+    do it here, where the range check reads one number back (they synchronise)."""
     limit = 60000.0
     big = max(float(query.abs().max()), float(key.abs().max())) if query.numel() and key.numel() else 0.0
     dt = torch.float16 if big < limit else torch.bfloat16
     return query.to(dt), key.to(dt)
 
 
-def _prepare_types(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
-    """The operands in a type the kernels take; raises for what they do not."""
+def _check_types(query: torch.Tensor, key: torch.Tensor) -> None:
+    """Raises for operands whose types, devices or head dimension the kernels do not take."""
     if key.dtype != query.dtype:
         raise ValueError(f"query and key must have the same dtype, got {query.dtype} and {key.dtype}")
     if key.device != query.device:
         raise ValueError(f"query and key must be on the same device, got {query.device} and {key.device}")
-    if query.dtype == torch.float32:
-        query, key = _round_fp32(query, key)
-    if query.dtype not in _DTYPE_CODE:
+    if query.dtype not in _DTYPE_CODE and query.dtype != torch.float32:
         raise ValueError(f"flash_colsum supports float16, bfloat16 and float32 inputs, got {query.dtype}")
     if query.shape[3] % 8 or not 8 <= query.shape[3] <= 128:
         raise ValueError(f"head_dim must be a multiple of 8 from 8 to 128, got {query.shape[3]}")
-    return query, key
 
 
 def _prepare(query: torch.Tensor, key: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, int]:
-    query, key = _prepare_types(query, key)
+    _check_types(query, key)
+    if query.dtype == torch.float32:
+        query, key = _round_fp32(query, key)
     return _tma_ready(query), _tma_ready(key), _DTYPE_CODE[query.dtype]
 
 
@@ -155,7 +155,7 @@ def _launch(Q: torch.Tensor, K: torch.Tensor, scale: float, is_causal: bool, k_p
             h_norm: int) -> torch.Tensor:
     """One call on operands of valid shape: (B, S_k) fp32.  ``k_past`` / ``cls_n`` -1 and ``h_norm`` 0
     stand for the defaults."""
-    Q, K = _prepare_types(Q, K)
+    _check_types(Q, K)
     out = _load_native(Q.device).launch(Q, K, float(scale), is_causal, k_past, cls_n, h_norm)
     if out is None:
         raise ValueError(f"unsupported operands: query {tuple(Q.shape)}, key {tuple(K.shape)}")
