@@ -514,7 +514,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const int w4 = warp & 3;                   // 32-row block of the tile
         const int row = (w4 << 5) | lane;          // tensor-memory lane = query row of the tile
         const uint32_t lane_base = tmem_base + ((uint32_t)(w4 << 5) << 16);
-        const float c = p.c;
+        const float c = fmaxf(p.c, 1.0e-30f);      // (a scale of zero: every visible score still counts as 2^0)
         const int keys_valid = p.Sk - (256 * (int)rank + 64 * wg);   // >= 64: the whole group is real keys
         // this thread's 128-byte line of P~ (one line per query row and 64-key group)
         const uint32_t p_line = (uint32_t)(hf * P_TILE_BYTES + half64 * P_ATOM_COL_BYTES + (row >> 3) * 1024 +
@@ -540,8 +540,8 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 
                 // ---- P~ = exp2(c*s - m_g) as packed fp16
                 uint32_t h[32];
-                float m_g, l_g;
-                if (keys_valid >= 64) {
+                float m_g = -INFINITY, l_g = 0.f;
+                auto exps = [&]() {
                     m_g = fmaxf(max_of_32(sa), max_of_32(sb)) * c;
                     const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_g, -m_g);
                     f32x2 sum0 = pack2(0.f, 0.f), sum1 = sum0;
@@ -553,30 +553,18 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     float x0, x1;
                     unpack2(add2(sum0, sum1), x0, x1);
                     l_g = x0 + x1;
-                } else {
-                    // ragged end of the key axis: keys past S_k (zero rows of the TMA box) are excluded
-                    float cm = -INFINITY;
+                };
+                if (keys_valid >= 64) {
+                    exps();
+                } else if (keys_valid > 0) {
+                    // ragged end of the key axis: keys past S_k (zero rows of the TMA box) get a score whose exp
+                    // is zero for any scale
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        if (j < keys_valid) cm = fmaxf(cm, __uint_as_float(sa[j]));
-                        if (j + 32 < keys_valid) cm = fmaxf(cm, __uint_as_float(sb[j]));
+                        sa[j] = j < keys_valid ? sa[j] : __float_as_uint(-3.0e38f);
+                        sb[j] = j + 32 < keys_valid ? sb[j] : __float_as_uint(-3.0e38f);
                     }
-                    m_g = (cm == -INFINITY) ? -INFINITY : cm * c;
-                    const float m_safe = (m_g == -INFINITY) ? 0.f : m_g;
-                    float acc = 0.f;
-#pragma unroll
-                    for (int pr = 0; pr < 32; ++pr) {
-                        const int j = 2 * pr;
-                        const float s0 = __uint_as_float(pr < 16 ? sa[j & 31] : sb[j & 31]);
-                        const float s1 = __uint_as_float(pr < 16 ? sa[(j + 1) & 31] : sb[(j + 1) & 31]);
-                        float ta = fmaf(s0, c, -m_safe), tb = fmaf(s1, c, -m_safe);
-                        ta = (j < keys_valid) ? ta : -INFINITY;       // c may be 0: select after the multiply
-                        tb = (j + 1 < keys_valid) ? tb : -INFINITY;
-                        const float ea = ex2_approx(ta), eb = ex2_approx(tb);
-                        acc += ea + eb;
-                        h[pr] = pack_half2(ea, eb);
-                    }
-                    l_g = acc;
+                    exps();
                 }
                 // ---- tile i-2 is through: its column-sum MMA has read P~(i-2), and (before that)
                 // the exchange warps have read its statistics -- both slots are free
@@ -586,12 +574,14 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 // ---- this group's (max, sum), for the exchange warps
                 lstats[(slot * CONSUMER_GROUPS + wg) * 128 + row] = make_float2(m_g, l_g);
                 mbar_arrive(stats_bar(slot));
-                {
-                    const uint32_t line = p_smem + slot * P_BYTES + p_line;
+                const uint32_t line = p_smem + slot * P_BYTES + p_line;
+                if (keys_valid > 0) {
 #pragma unroll
                     for (int j8 = 0; j8 < 8; ++j8)
                         st_shared_v4(line + ((((uint32_t)j8) ^ sw) << 4), h[4 * j8], h[4 * j8 + 1], h[4 * j8 + 2],
                                      h[4 * j8 + 3]);
+                } else if (i < 2) {      // a group without keys: its exps are zero in both buffers, for good
+                    for (int j8 = 0; j8 < 8; ++j8) st_shared_v4(line + 16 * j8, 0u, 0u, 0u, 0u);
                 }
                 // (the MMA warp makes these stores visible to the tensor core: it fences after its wait)
                 mbar_arrive(p_ready(slot, hf));

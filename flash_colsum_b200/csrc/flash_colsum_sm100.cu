@@ -626,10 +626,12 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                     if (full) {
                         stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
                     } else {
+                        // what the rows of this warp see of the group's columns: everything, nothing, or some
                         const int lim = stats_last_visible(p, it.qt, st, row) - col0;
-                        // skip the block when no row of the tile sees any of its columns
-                        const int lim_last_row = stats_last_visible(p, it.qt, st, TILE - 1) - col0;
-                        if (lim_last_row >= 0) stats_tile<true>(taddr, lim, c, m_run, l_run);
+                        const int lim_first = stats_last_visible(p, it.qt, st, row & ~31) - col0;
+                        const int lim_last = stats_last_visible(p, it.qt, st, (row | 31)) - col0;
+                        if (lim_first >= GROUP_COLS - 1) stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
+                        else if (lim_last >= 0) stats_tile<true>(taddr, lim, c, m_run, l_run);
                     }
                 } else if constexpr (EXT) {
                     // the accumulator already holds s - lse/c
@@ -648,8 +650,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                                     const int q0 = (wg & 1) * GROUP_COLS;
                                     const int end = colsum_end_visible(p, st) - q0;
                                     const int thr = colsum_first_visible(p, ktg, st, row) - q0;
-                                    const int thr_first_row = colsum_first_visible(p, ktg, st, 0) - q0;
-                                    const int thr_last_row = colsum_first_visible(p, ktg, st, TILE - 1) - q0;
+                                    const int thr_first_row = colsum_first_visible(p, ktg, st, row & ~31) - q0;
+                                    const int thr_last_row = colsum_first_visible(p, ktg, st, (row | 31)) - q0;
                                     if (end > 0 && thr_first_row < GROUP_COLS) {
                                         if (end >= GROUP_COLS && thr_last_row <= 0)
                                             colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
@@ -664,8 +666,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                                 const int c0 = wg * (GROUP_COLS / 2);
                                 const int end = colsum_end_visible(p, st) - c0;
                                 const int thr = colsum_first_visible(p, it.kt, st, row) - c0;
-                                const int thr_first_row = colsum_first_visible(p, it.kt, st, 0) - c0;
-                                const int thr_last_row = colsum_first_visible(p, it.kt, st, TILE - 1) - c0;
+                                const int thr_first_row = colsum_first_visible(p, it.kt, st, row & ~31) - c0;
+                                const int thr_last_row = colsum_first_visible(p, it.kt, st, (row | 31)) - c0;
                                 if (end > 0 && thr_first_row < GROUP_COLS / 2) {
                                     uint32_t r[32];
                                     tmem_ld_x32(taddr - col0 + c0, r);
@@ -678,9 +680,13 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                         if (!done_short) {
                             const int thr = colsum_first_visible(p, it.kt, st, row) - col0;
                             const int end = colsum_end_visible(p, st) - col0;
-                            // skip the block when no key of the tile is seen by any of its queries
-                            const int thr_first_row = colsum_first_visible(p, it.kt, st, 0) - col0;
-                            if (end > 0 && thr_first_row < GROUP_COLS) colsum_tile_ext<true>(taddr, thr, end, c, acc);
+                            // what the block's queries see of this warp's keys: nothing, everything, or some
+                            const int thr_first_row = colsum_first_visible(p, it.kt, st, row & ~31) - col0;
+                            const int thr_last_row = colsum_first_visible(p, it.kt, st, (row | 31)) - col0;
+                            if (end > 0 && thr_first_row < GROUP_COLS) {
+                                if (end >= GROUP_COLS && thr_last_row <= 0) colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
+                                else colsum_tile_ext<true>(taddr, thr, end, c, acc);
+                            }
                         }
                     }
                 } else {
@@ -695,7 +701,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                         const int thr = colsum_first_visible(p, it.kt, st, row) - col0;
                         const int end = colsum_end_visible(p, st) - col0;
                         // skip the block when no key of the tile is seen by any of its queries
-                        const int thr_first_row = colsum_first_visible(p, it.kt, st, 0) - col0;
+                        const int thr_first_row = colsum_first_visible(p, it.kt, st, row & ~31) - col0;
                         if (end > 0 && thr_first_row < GROUP_COLS) colsum_tile<true>(taddr, nl, thr, end, c, acc);
                     }
                     mbar_arrive(l_empty(ls));

@@ -1,0 +1,35 @@
+"""Masks decided per warp and ragged key groups: diagonals, groups without keys, extreme scores."""
+
+import pytest
+import torch
+
+from conftest import REL_L2_TOL
+from flash_colsum_b200.inputs import Workload, make_inputs
+from oracle import c_oracle
+from oracle.naive_colsum import parity_errors
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,D,causal", [
+    (1, 2, 900, 900, 64, False),       # statistics and column passes
+    (1, 2, 900, 900, 128, True),       # ... with a causal diagonal
+    (2, 2, 577, 577, 64, False),       # single-pass cluster kernel: groups of 64, 1 and no keys
+    (1, 2, 128, 1500, 64, True),       # one-kernel form
+])
+@pytest.mark.parametrize("jump,scale", [(30.0, None), (1.0e4, None), (1.0, 0.0)])
+def test_extreme_scores_and_a_scale_of_zero(B, H, Sq, Sk, D, causal, jump, scale):
+    """Keys further on that lift the scores by hundreds and by hundreds of thousands of powers of two, and a
+    scale of zero (every visible key counts the same)."""
+    if not torch.cuda.is_available():
+        pytest.fail("the gpu-marked tests need a CUDA device")
+    import flash_colsum_b200 as fc
+    w = Workload("jump", B, H, Sq, Sk, D, "bf16", is_causal=causal, seed=Sk + D)
+    q, k = make_inputs(w)
+    k[:, :, Sk // 3::7] *= jump
+    got = fc.flash_colsum(q.cuda(), k.cuda(), scale=scale, is_causal=causal).cpu().numpy()
+    assert fc.device_status() == 0
+    want = c_oracle.colsum_c(q, k, scale=scale, is_causal=causal)
+    rel, mx = parity_errors(got, want)
+    # (scores in the hundreds of thousands: an fp32 score has no more than a percent of a unit)
+    assert rel <= (REL_L2_TOL if jump <= 30 else 0.1), (jump, rel, mx)
