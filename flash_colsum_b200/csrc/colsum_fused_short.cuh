@@ -283,8 +283,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
                 } else {
                     const int lim = stats_last_visible(p, 0, kb, row) - col0;
-                    const int lim_first = stats_last_visible(p, 0, kb, row & ~31) - col0;
-                    const int lim_last = stats_last_visible(p, 0, kb, (row | 31)) - col0;
+                    const int lim_first = __shfl_sync(0xffffffffu, lim, 0), lim_last = __shfl_sync(0xffffffffu, lim, 31);
                     if (lim_first >= GROUP_COLS - 1) stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
                     else if (lim_last >= 0) stats_tile<true>(taddr, lim, c, m_run, l_run);
                 }
@@ -353,8 +352,8 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             const uint32_t taddr = lane_addr + buf * BLOCK;
             const int ktg = kb * 2 + tg;
             const int thr = colsum_first_visible(p, ktg, 0, row) - q0;
-            const int thr_first_row = colsum_first_visible(p, ktg, 0, row & ~31) - q0;
-            const int thr_last_row = colsum_first_visible(p, ktg, 0, (row | 31)) - q0;
+            const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
+            const int thr_last_row = __shfl_sync(0xffffffffu, thr, 31);
             if (ok && end > 0 && thr_first_row < GROUP_COLS) {
                 const bool whole = end >= GROUP_COLS && thr_last_row <= 0;
                 if (fp.use_ext) {

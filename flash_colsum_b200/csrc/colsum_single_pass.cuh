@@ -247,6 +247,8 @@ __device__ __forceinline__ void exp8_packed(int pair0, const uint32_t* s, f32x2 
 //                      result to every CTA of the cluster, and when all CTAs' values are in,
 //                      write the weights W of the four groups.
 // ---------------------------------------------------------------------------
+// WHOLE: every CTA's slice is full (the masks cost registers that the loop is short of: 12 % at 1024 keys).
+template <bool WHOLE>
 __global__ void __launch_bounds__(sp::THREADS, 1)
 colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const SinglePassParams p) {
@@ -514,7 +516,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const int w4 = warp & 3;                   // 32-row block of the tile
         const int row = (w4 << 5) | lane;          // tensor-memory lane = query row of the tile
         const uint32_t lane_base = tmem_base + ((uint32_t)(w4 << 5) << 16);
-        const float c = fmaxf(p.c, 1.0e-30f);      // (a scale of zero: every visible score still counts as 2^0)
+        const float c = WHOLE ? p.c : fmaxf(p.c, 1.0e-30f);      // (a scale of zero: every visible score still counts as 2^0)
         const int keys_valid = p.Sk - (256 * (int)rank + 64 * wg);   // >= 64: the whole group is real keys
         // this thread's 128-byte line of P~ (one line per query row and 64-key group)
         const uint32_t p_line = (uint32_t)(hf * P_TILE_BYTES + half64 * P_ATOM_COL_BYTES + (row >> 3) * 1024 +
@@ -541,7 +543,16 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 // ---- P~ = exp2(c*s - m_g) as packed fp16
                 uint32_t h[32];
                 float m_g = -INFINITY, l_g = 0.f;
-                auto exps = [&]() {
+                if (WHOLE || keys_valid > 0) {
+                    if (!WHOLE && keys_valid < 64) {
+                        // ragged end of the key axis: keys past S_k (zero rows of the TMA box) get a score whose
+                        // exp is zero for any scale, and everything after this is the common path
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            sa[j] = j < keys_valid ? sa[j] : __float_as_uint(-3.0e38f);
+                            sb[j] = j + 32 < keys_valid ? sb[j] : __float_as_uint(-3.0e38f);
+                        }
+                    }
                     m_g = fmaxf(max_of_32(sa), max_of_32(sb)) * c;
                     const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_g, -m_g);
                     f32x2 sum0 = pack2(0.f, 0.f), sum1 = sum0;
@@ -553,18 +564,6 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     float x0, x1;
                     unpack2(add2(sum0, sum1), x0, x1);
                     l_g = x0 + x1;
-                };
-                if (keys_valid >= 64) {
-                    exps();
-                } else if (keys_valid > 0) {
-                    // ragged end of the key axis: keys past S_k (zero rows of the TMA box) get a score whose exp
-                    // is zero for any scale
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        sa[j] = j < keys_valid ? sa[j] : __float_as_uint(-3.0e38f);
-                        sb[j] = j + 32 < keys_valid ? sb[j] : __float_as_uint(-3.0e38f);
-                    }
-                    exps();
                 }
                 // ---- tile i-2 is through: its column-sum MMA has read P~(i-2), and (before that)
                 // the exchange warps have read its statistics -- both slots are free
@@ -575,7 +574,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 lstats[(slot * CONSUMER_GROUPS + wg) * 128 + row] = make_float2(m_g, l_g);
                 mbar_arrive(stats_bar(slot));
                 const uint32_t line = p_smem + slot * P_BYTES + p_line;
-                if (keys_valid > 0) {
+                if (WHOLE || keys_valid > 0) {
 #pragma unroll
                     for (int j8 = 0; j8 < 8; ++j8)
                         st_shared_v4(line + ((((uint32_t)j8) ^ sw) << 4), h[4 * j8], h[4 * j8 + 1], h[4 * j8 + 2],

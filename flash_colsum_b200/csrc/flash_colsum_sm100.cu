@@ -628,8 +628,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                     } else {
                         // what the rows of this warp see of the group's columns: everything, nothing, or some
                         const int lim = stats_last_visible(p, it.qt, st, row) - col0;
-                        const int lim_first = stats_last_visible(p, it.qt, st, row & ~31) - col0;
-                        const int lim_last = stats_last_visible(p, it.qt, st, (row | 31)) - col0;
+                        const int lim_first = __shfl_sync(0xffffffffu, lim, 0), lim_last = __shfl_sync(0xffffffffu, lim, 31);
                         if (lim_first >= GROUP_COLS - 1) stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
                         else if (lim_last >= 0) stats_tile<true>(taddr, lim, c, m_run, l_run);
                     }
@@ -650,8 +649,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                                     const int q0 = (wg & 1) * GROUP_COLS;
                                     const int end = colsum_end_visible(p, st) - q0;
                                     const int thr = colsum_first_visible(p, ktg, st, row) - q0;
-                                    const int thr_first_row = colsum_first_visible(p, ktg, st, row & ~31) - q0;
-                                    const int thr_last_row = colsum_first_visible(p, ktg, st, (row | 31)) - q0;
+                                    const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
+                                    const int thr_last_row = __shfl_sync(0xffffffffu, thr, 31);
                                     if (end > 0 && thr_first_row < GROUP_COLS) {
                                         if (end >= GROUP_COLS && thr_last_row <= 0)
                                             colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
@@ -666,8 +665,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                                 const int c0 = wg * (GROUP_COLS / 2);
                                 const int end = colsum_end_visible(p, st) - c0;
                                 const int thr = colsum_first_visible(p, it.kt, st, row) - c0;
-                                const int thr_first_row = colsum_first_visible(p, it.kt, st, row & ~31) - c0;
-                                const int thr_last_row = colsum_first_visible(p, it.kt, st, (row | 31)) - c0;
+                                const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
+                                const int thr_last_row = __shfl_sync(0xffffffffu, thr, 31);
                                 if (end > 0 && thr_first_row < GROUP_COLS / 2) {
                                     uint32_t r[32];
                                     tmem_ld_x32(taddr - col0 + c0, r);
@@ -681,8 +680,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                             const int thr = colsum_first_visible(p, it.kt, st, row) - col0;
                             const int end = colsum_end_visible(p, st) - col0;
                             // what the block's queries see of this warp's keys: nothing, everything, or some
-                            const int thr_first_row = colsum_first_visible(p, it.kt, st, row & ~31) - col0;
-                            const int thr_last_row = colsum_first_visible(p, it.kt, st, (row | 31)) - col0;
+                            const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
+                            const int thr_last_row = __shfl_sync(0xffffffffu, thr, 31);
                             if (end > 0 && thr_first_row < GROUP_COLS) {
                                 if (end >= GROUP_COLS && thr_last_row <= 0) colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
                                 else colsum_tile_ext<true>(taddr, thr, end, c, acc);
@@ -701,7 +700,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                         const int thr = colsum_first_visible(p, it.kt, st, row) - col0;
                         const int end = colsum_end_visible(p, st) - col0;
                         // skip the block when no key of the tile is seen by any of its queries
-                        const int thr_first_row = colsum_first_visible(p, it.kt, st, row & ~31) - col0;
+                        const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
                         if (end > 0 && thr_first_row < GROUP_COLS) colsum_tile<true>(taddr, nl, thr, end, c, acc);
                     }
                     mbar_arrive(l_empty(ls));
@@ -1336,7 +1335,10 @@ static int single_pass_max_clusters(int cl) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || cl < 1 || cl > sp::MAX_CL) return 0;
     const int idx = cl;
     if (cached[dev][idx] == 0) {
-        if (cudaFuncSetAttribute(colsum_single_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        // (both instances: the same block, shared memory and registers)
+        if (cudaFuncSetAttribute(colsum_single_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 sp::DYN_BYTES) != cudaSuccess ||
+            cudaFuncSetAttribute(colsum_single_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  sp::DYN_BYTES) != cudaSuccess)
             return 0;
         cudaLaunchConfig_t cfg;
@@ -1352,7 +1354,7 @@ static int single_pass_max_clusters(int cl) {
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, colsum_single_pass_kernel, &cfg) != cudaSuccess || n <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, colsum_single_pass_kernel<true>, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
             return 0;
         }
@@ -1408,7 +1410,8 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = overlap_previous() ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, colsum_single_pass_kernel, tq, tk, sp_);
+    auto kern = Sk % 256 == 0 ? colsum_single_pass_kernel<true> : colsum_single_pass_kernel<false>;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tq, tk, sp_);
     if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "single-pass kernel launch failed: %s", cudaGetErrorString(e));
     return FCS_OK;
 }
