@@ -227,6 +227,10 @@ __device__ __forceinline__ void exp8_packed(int pair0, const uint32_t* s, f32x2 
     }
 }
 
+// what of a consumer group's 64 keys is real
+enum : int { NO_KEYS, SOME_KEYS, ALL_KEYS };
+template <int V> struct Kind { static constexpr int value = V; };
+
 }  // namespace sp
 
 // ---------------------------------------------------------------------------
@@ -247,7 +251,7 @@ __device__ __forceinline__ void exp8_packed(int pair0, const uint32_t* s, f32x2 
 //                      result to every CTA of the cluster, and when all CTAs' values are in,
 //                      write the weights W of the four groups.
 // ---------------------------------------------------------------------------
-// WHOLE: every CTA's slice is full (the masks cost registers that the loop is short of: 12 % at 1024 keys).
+// WHOLE: every CTA's slice is full.
 template <bool WHOLE>
 __global__ void __launch_bounds__(sp::THREADS, 1)
 colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -522,6 +526,10 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const uint32_t p_line = (uint32_t)(hf * P_TILE_BYTES + half64 * P_ATOM_COL_BYTES + (row >> 3) * 1024 +
                                            (row & 7) * 128);
         const uint32_t sw = (uint32_t)(row & 7);
+        // The loop over the tiles, apart for groups whose 64 keys are all real, some of them, or none: the
+        // masks cost registers that the loop is short of (in one copy, 12 % at 1024 keys).
+        auto consume = [&](auto kind) {
+        constexpr int KEYS = decltype(kind)::value;
         int i = 0, fc = 0;
         bool ok = true;
         for (int u = u0; ok && u < u1; ++u) {
@@ -533,18 +541,20 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t sa[32], sb[32];   // columns 0..31 and 32..63 of the group
-                tmem_ld_x32(lane_base + 64 * wg, sa);
-                tmem_ld_x32(lane_base + 64 * wg + 32, sb);
-                tmem_ld_wait(sa);
-                tmem_ld_wait(sb);
+                if constexpr (KEYS != NO_KEYS) {
+                    tmem_ld_x32(lane_base + 64 * wg, sa);
+                    tmem_ld_x32(lane_base + 64 * wg + 32, sb);
+                    tmem_ld_wait(sa);
+                    tmem_ld_wait(sb);
+                }
                 tc_fence_before();
                 mbar_arrive(s_empty);
 
                 // ---- P~ = exp2(c*s - m_g) as packed fp16
                 uint32_t h[32];
                 float m_g = -INFINITY, l_g = 0.f;
-                if (WHOLE || keys_valid > 0) {
-                    if (!WHOLE && keys_valid < 64) {
+                if constexpr (KEYS != NO_KEYS) {
+                    if constexpr (KEYS == SOME_KEYS) {
                         // ragged end of the key axis: keys past S_k (zero rows of the TMA box) get a score whose
                         // exp is zero for any scale, and everything after this is the common path
 #pragma unroll
@@ -571,10 +581,10 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 // ---- this group's (max, sum), for the exchange warps
-                lstats[(slot * CONSUMER_GROUPS + wg) * 128 + row] = make_float2(m_g, l_g);
+                lstats[(slot * sp::CONSUMER_GROUPS + wg) * 128 + row] = make_float2(m_g, l_g);
                 mbar_arrive(stats_bar(slot));
                 const uint32_t line = p_smem + slot * P_BYTES + p_line;
-                if (WHOLE || keys_valid > 0) {
+                if constexpr (KEYS != NO_KEYS) {
 #pragma unroll
                     for (int j8 = 0; j8 < 8; ++j8)
                         st_shared_v4(line + ((((uint32_t)j8) ^ sw) << 4), h[4 * j8], h[4 * j8 + 1], h[4 * j8 + 2],
@@ -607,6 +617,15 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 mbar_arrive(d2_empty(hf));
                 ++fc;
             }
+        }
+    
+        };
+        if constexpr (WHOLE) {
+            consume(Kind<ALL_KEYS>{});
+        } else {
+            if (keys_valid >= 64) consume(Kind<ALL_KEYS>{});
+            else if (keys_valid > 0) consume(Kind<SOME_KEYS>{});
+            else consume(Kind<NO_KEYS>{});
         }
     }
 
