@@ -227,9 +227,15 @@ __device__ __forceinline__ void exp8_packed(int pair0, const uint32_t* s, f32x2 
     }
 }
 
-// what of a consumer group's 64 keys is real
-enum : int { NO_KEYS, SOME_KEYS, ALL_KEYS };
-template <int V> struct Kind { static constexpr int value = V; };
+// Writes `value` into `n` columns of this warp's 32 tensor-memory lanes.
+__device__ __forceinline__ void tmem_fill(uint32_t taddr, int n, uint32_t value) {
+    for (; n >= 8; n -= 8, taddr += 8)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(value) : "memory");
+    for (; n > 0; --n, ++taddr)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(value) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+template <bool V> struct Flag { static constexpr bool value = V; };
 
 }  // namespace sp
 
@@ -251,8 +257,9 @@ template <int V> struct Kind { static constexpr int value = V; };
 //                      result to every CTA of the cluster, and when all CTAs' values are in,
 //                      write the weights W of the four groups.
 // ---------------------------------------------------------------------------
-// WHOLE: every CTA's slice is full.
-template <bool WHOLE>
+// PADDED: the key axis ends inside a group of 64 keys.  (An instance of its own: the test for it in the
+// loop costs 4 % at 512 and 1024 keys.)
+template <bool PADDED>
 __global__ void __launch_bounds__(sp::THREADS, 1)
 colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const SinglePassParams p) {
@@ -520,16 +527,19 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const int w4 = warp & 3;                   // 32-row block of the tile
         const int row = (w4 << 5) | lane;          // tensor-memory lane = query row of the tile
         const uint32_t lane_base = tmem_base + ((uint32_t)(w4 << 5) << 16);
-        const float c = WHOLE ? p.c : fmaxf(p.c, 1.0e-30f);      // (a scale of zero: every visible score still counts as 2^0)
+        const float c = PADDED ? fmaxf(p.c, 1.0e-30f) : p.c;      // (a scale of zero: every visible score still counts as 2^0)
         const int keys_valid = p.Sk - (256 * (int)rank + 64 * wg);   // >= 64: the whole group is real keys
         // this thread's 128-byte line of P~ (one line per query row and 64-key group)
         const uint32_t p_line = (uint32_t)(hf * P_TILE_BYTES + half64 * P_ATOM_COL_BYTES + (row >> 3) * 1024 +
                                            (row & 7) * 128);
         const uint32_t sw = (uint32_t)(row & 7);
-        // The loop over the tiles, apart for groups whose 64 keys are all real, some of them, or none: the
-        // masks cost registers that the loop is short of (in one copy, 12 % at 1024 keys).
-        auto consume = [&](auto kind) {
-        constexpr int KEYS = decltype(kind)::value;
+        // columns of the group past S_k (zero rows of the TMA box): their scores are overwritten in tensor
+        // memory, so that the loop knows no masks -- in registers they cost it spills (12 % at 1024 keys), and a
+        // second copy of it for the ragged group does not fit the instruction cache next to the first
+        // (385-447 keys: 89 us a call against 62)
+        const int padding = keys_valid < 64 ? 64 - keys_valid : 0;
+        auto consume = [&](auto keys) {
+        constexpr bool KEYS = decltype(keys)::value;     // false: nothing but padding
         int i = 0, fc = 0;
         bool ok = true;
         for (int u = u0; ok && u < u1; ++u) {
@@ -541,7 +551,8 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t sa[32], sb[32];   // columns 0..31 and 32..63 of the group
-                if constexpr (KEYS != NO_KEYS) {
+                if constexpr (KEYS) {
+                    if (PADDED && padding > 0) tmem_fill(lane_base + 64 * wg + keys_valid, padding, __float_as_uint(-3.0e38f));
                     tmem_ld_x32(lane_base + 64 * wg, sa);
                     tmem_ld_x32(lane_base + 64 * wg + 32, sb);
                     tmem_ld_wait(sa);
@@ -553,16 +564,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 // ---- P~ = exp2(c*s - m_g) as packed fp16
                 uint32_t h[32];
                 float m_g = -INFINITY, l_g = 0.f;
-                if constexpr (KEYS != NO_KEYS) {
-                    if constexpr (KEYS == SOME_KEYS) {
-                        // ragged end of the key axis: keys past S_k (zero rows of the TMA box) get a score whose
-                        // exp is zero for any scale, and everything after this is the common path
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            sa[j] = j < keys_valid ? sa[j] : __float_as_uint(-3.0e38f);
-                            sb[j] = j + 32 < keys_valid ? sb[j] : __float_as_uint(-3.0e38f);
-                        }
-                    }
+                if constexpr (KEYS) {
                     m_g = fmaxf(max_of_32(sa), max_of_32(sb)) * c;
                     const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_g, -m_g);
                     f32x2 sum0 = pack2(0.f, 0.f), sum1 = sum0;
@@ -584,7 +586,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 lstats[(slot * sp::CONSUMER_GROUPS + wg) * 128 + row] = make_float2(m_g, l_g);
                 mbar_arrive(stats_bar(slot));
                 const uint32_t line = p_smem + slot * P_BYTES + p_line;
-                if constexpr (KEYS != NO_KEYS) {
+                if constexpr (KEYS) {
 #pragma unroll
                     for (int j8 = 0; j8 < 8; ++j8)
                         st_shared_v4(line + ((((uint32_t)j8) ^ sw) << 4), h[4 * j8], h[4 * j8 + 1], h[4 * j8 + 2],
@@ -620,13 +622,8 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         }
     
         };
-        if constexpr (WHOLE) {
-            consume(Kind<ALL_KEYS>{});
-        } else {
-            if (keys_valid >= 64) consume(Kind<ALL_KEYS>{});
-            else if (keys_valid > 0) consume(Kind<SOME_KEYS>{});
-            else consume(Kind<NO_KEYS>{});
-        }
+        if (keys_valid > 0) consume(Flag<true>{});
+        else consume(Flag<false>{});
     }
 
     // ---------------------------------------------------- teardown

@@ -1354,7 +1354,7 @@ static int single_pass_max_clusters(int cl) {
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, colsum_single_pass_kernel<true>, &cfg) != cudaSuccess || n <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, colsum_single_pass_kernel<false>, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
             return 0;
         }
@@ -1410,7 +1410,7 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = overlap_previous() ? 2 : 1;
-    auto kern = Sk % 256 == 0 ? colsum_single_pass_kernel<true> : colsum_single_pass_kernel<false>;
+    auto kern = Sk % 64 ? colsum_single_pass_kernel<true> : colsum_single_pass_kernel<false>;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tq, tk, sp_);
     if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "single-pass kernel launch failed: %s", cudaGetErrorString(e));
     return FCS_OK;
