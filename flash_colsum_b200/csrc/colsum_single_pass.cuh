@@ -21,11 +21,9 @@
 // the column-sum MMA of tile i runs while the consumers work on tiles i+1 and i+2,
 // which is the time the statistics of tile i have to go around the cluster.
 //
-// Measured against the two-pass kernels (fp16, B = 32, H = 16): 1.2-1.3x at 400-1024
-// keys, 1.07-1.14x at 1152-1536, 0.84x / 0.95x at 1792 / 2048 (only 15 clusters of seven
-// or eight CTAs are resident at a time: 105 / 120 of the 148 SMs); key lengths that fill
-// less than ~75 % of their cluster's slices lose to the padding.  The host side picks
-// accordingly.
+// A tile takes a CTA the same time whatever the number of real keys in its slice; keys past S_k are
+// overwritten in tensor memory.  us per call (B = 32, H = 16) with the padding masked in registers and here:
+// 400 keys 71 -> 63, 577 137 -> 117; the rule for which calls come here is with the launcher.
 #pragma once
 
 #include "colsum_math.cuh"

@@ -1318,11 +1318,14 @@ static bool single_pass_applies(int B, int H, int Sq, int Sk, int D, int causal)
     if (g_single_pass == 1 || causal || D > 64 || Sk > 256 * sp::MAX_CL) return false;   // (D < 64: zero-filled columns)
     if (g_single_pass == 2) return true;
     const int cl = single_pass_cluster_size(Sk);
-    // measured at B=32 H=16 against the two passes: 1.2-1.3x at 400-1024 keys, 1.07-1.14x at
-    // 1152-1536, 1.02x at 577 (75 % of three slices); clusters of 7 and 8 fit only 15 at a time
-    // (105 / 120 of 148 SMs) and lose on large calls (0.84x / 0.95x) but win on small ones,
-    // where the fixed costs of two launches and partial waves weigh more
-    if (cl <= 6) return (long long)Sk * 100 >= (long long)cl * 256 * 75;
+    // us per call, this form / the two passes, at 32 x 16 pairs and at 2 x 8: 96 keys 19/23 9/9, 150 27/34
+    // 8/13, 320 50/54 9/14, 520 118/133 13/20, 640 114/139 12/20, 1030 342/381 21/23, 1400 489/544 24/38 -- the
+    // time goes by whole slices of 256 keys, and up to six of them it wins at any fill from 60 %
+    // (one slice: at any length); clusters of 7 and 8 fit only 15 at a time (105 / 120 of 148 SMs) and lose
+    // on large calls (2048 keys: 1046/998) but win on small ones (41/50), where the fixed costs of two
+    // launches and partial waves weigh more
+    if (cl == 1) return true;
+    if (cl <= 6) return (long long)Sk * 100 >= (long long)cl * 256 * 60;
     if ((long long)Sk * 100 < (long long)cl * 256 * 85) return false;
     const long long tiles = (long long)B * H * ((Sq + TILE - 1) / TILE);
     return tiles <= 512;
