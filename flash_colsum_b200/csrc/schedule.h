@@ -163,6 +163,8 @@ FCS_HD inline void colsum_full_range(const Problem& p, int kt, int& lo, int& hi)
 // tile index, and the longest items may come last: the busiest CTA had 1.2 times the average at 2000 x
 // 2000 and 128 heads, 1.5 at 4000 x 4000 and 16.  Longest first over all heads brings that to 1.06 / 1.29 --
 // over as many heads at a time as have their keys in L2 together (every head is read by all SMs at once).
+// us per call, plain / longest first: 4000 x 4000, 16 heads 99 / 93; 6000, 8 heads 122 / 110; 8000, 32 heads
+// 682 / 664 -- but 700 x 700, 256 heads 83 / 89, 1500, 32 heads 42.7 / 43.5, 20000, 32 heads 3745 / 3768.
 struct StatsItems {
     bool done;
     int b, h, qt, sp, s0, s1, grid;   // steps = key blocks s0..s1-1
@@ -510,7 +512,9 @@ inline void plan(Problem& p, int B, int H, int Sq, int Sk, int causal, int k_pas
     p.nsplit = best;
     p.stats_items = base_items * p.nsplit;
     p.stats_heads = 0;
-    if (causal && p.nsplit == 1 && p.NQ > 1 && base_items <= 0x7fffffffLL) {
+    // (long items and few of them: with short ones a head's keys come from memory for one item at a time, with
+    // many the plain order evens out)
+    if (causal && p.nsplit == 1 && p.NQ >= 24 && base_items < 16ll * sms) {
         const long long fit = STATS_ROUND_ROWS / Sk;
         p.stats_heads = (int)(fit < 1 ? 1 : fit < (long long)B * H ? fit : (long long)B * H);
     }
