@@ -30,10 +30,25 @@ typedef struct FcsCall {
     void* alloc_ctx;
 } FcsCall;
 
+// A call whose query, key and result live in host memory (contiguous; pinned for copies that overlap).
+// `call` describes the operands as they will lie on the device: q, k and out are device buffers of the whole
+// operands' size, the strides dense.
+typedef struct FcsHostCall {
+    FcsCall call;
+    const void* host_q;
+    const void* host_k;
+    float* host_out;
+    int batch_chunk;              // batch entries per chunk, or 0: chunks that shrink towards the end
+} FcsHostCall;
+
 typedef int (*FcsRunCallFn)(const FcsCall*);
+typedef int (*FcsRunHostCallFn)(const FcsHostCall*);
 typedef int (*FcsSelectTopkFn)(const float*, int64_t, int, int, int, int*, float*, void*);
 typedef int (*FcsSelectThresholdFn)(const float*, int64_t, int, int, float, int, int*, int*, void*);
 typedef const char* (*FcsLastErrorFn)(void);
 
 int fcs_run_call(const FcsCall* call);
+
+// Copies in, computes, copies the result out; returns when the result is there.
+int fcs_run_host_call(const FcsHostCall* call);
 }

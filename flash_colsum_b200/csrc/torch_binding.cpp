@@ -25,6 +25,7 @@
 namespace {
 
 FcsRunCallFn g_run_call = nullptr;
+FcsRunHostCallFn g_run_host_call = nullptr;
 FcsSelectTopkFn g_select_topk = nullptr;
 FcsSelectThresholdFn g_select_threshold = nullptr;
 FcsLastErrorFn g_last_error = nullptr;
@@ -185,6 +186,78 @@ PyObject* py_launch(PyObject*, PyObject* const* args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// host(query, key, scale, is_causal, cls_len, device index, batch_chunk or 0) -> host tensor
+PyObject* py_host(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 7 || !g_run_host_call || !usable(args[0]) || !usable(args[1])) Py_RETURN_NONE;
+    const at::Tensor& q = THPVariable_Unpack(args[0]);
+    const at::Tensor& k = THPVariable_Unpack(args[1]);
+    const int causal = PyObject_IsTrue(args[3]);
+    const long idx = PyLong_AsLong(args[5]), batch_chunk = PyLong_AsLong(args[6]);
+    if (PyErr_Occurred()) return nullptr;
+    if (idx < 0 || idx >= MAX_DEVICES || !g_status[idx] || batch_chunk < 0) Py_RETURN_NONE;
+    if (q.dim() != 4 || k.dim() != 4 || !q.is_cpu() || !k.is_cpu() || !q.is_contiguous() || !k.is_contiguous()) Py_RETURN_NONE;
+    if (q.scalar_type() != k.scalar_type() || dtype_code(q.scalar_type()) < 0) Py_RETURN_NONE;
+    const auto a = q.sizes(), b = k.sizes();
+    if (a[0] != b[0] || a[1] != b[1] || a[3] != b[3] || a[3] < 8 || a[3] > 128 || a[3] % 8) Py_RETURN_NONE;
+    for (int i = 0; i < 4; ++i)
+        if (a[i] <= 0 || b[i] <= 0 || a[i] > 0x7fffffffLL || b[i] > 0x7fffffffLL) Py_RETURN_NONE;
+    if (causal ? a[0] != 1 : a[2] != b[2]) Py_RETURN_NONE;
+    int cls_n = -1;
+    if (args[4] != Py_None) {
+        if (causal || !PyLong_CheckExact(args[4])) Py_RETURN_NONE;
+        int overflow = 0;
+        const long long v = PyLong_AsLongLongAndOverflow(args[4], &overflow);
+        if (overflow || v <= 0 || v > 0x7fffffffLL) Py_RETURN_NONE;
+        cls_n = (int)v;
+    }
+    const double scale = scale_or_default(args[2], q);
+    if (PyErr_Occurred()) return nullptr;
+    at::Tensor host_out;
+    int rc;
+    {
+        WithoutGil nogil;
+        const c10::Device dev(c10::kCUDA, (c10::DeviceIndex)idx);
+        const c10::DeviceGuard guard(dev);
+        const at::Tensor dq = at::detail::empty_cuda(a, q.scalar_type(), dev, std::nullopt);
+        const at::Tensor dk = at::detail::empty_cuda(b, k.scalar_type(), dev, std::nullopt);
+        const at::Tensor out = empty_f32(a[0], b[2], dev);
+        host_out = at::empty({a[0], b[2]}, at::TensorOptions().dtype(at::kFloat).device(at::kCPU));
+        FcsHostCall hc;
+        FcsCall& c = hc.call;
+        c.B = (int)a[0];
+        c.H = (int)a[1];
+        c.Sq = (int)a[2];
+        c.Sk = (int)b[2];
+        c.D = (int)a[3];
+        c.q = dq.const_data_ptr();
+        c.k = dk.const_data_ptr();
+        c.out = static_cast<float*>(out.mutable_data_ptr());
+        c.out_ld = c.Sk;
+        c.dtype = dtype_code(q.scalar_type());
+        kernel_strides(dq, c.q_stride);
+        kernel_strides(dk, c.k_stride);
+        c.scale = (float)scale;
+        c.causal = causal;
+        c.k_past = -1;
+        c.cls_n = cls_n;
+        c.h_norm = 0;
+        c.status = g_status[idx];
+        c.stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)idx).stream();
+        Scratch scratch{dev, {}};
+        c.alloc = &Scratch::alloc;
+        c.alloc_ctx = &scratch;
+        hc.host_q = q.const_data_ptr();
+        hc.host_k = k.const_data_ptr();
+        hc.host_out = static_cast<float*>(host_out.mutable_data_ptr());
+        hc.batch_chunk = (int)(batch_chunk < 0x7fffffffL ? batch_chunk : 0x7fffffffL);
+        rc = g_run_host_call(&hc);
+    }
+    if (rc != FCS_OK) return raise_library_error(rc);
+    return THPVariable_Wrap(std::move(host_out));
+    END_HANDLE_TH_ERRORS
+}
+
 bool means_ok(const at::Tensor& t) {
     return t.dim() == 2 && t.scalar_type() == at::kFloat && t.is_cuda();
 }
@@ -265,7 +338,8 @@ PyObject* py_bind(PyObject*, PyObject* arg) {
     g_select_topk = reinterpret_cast<FcsSelectTopkFn>(sym("fcs_select_topk"));
     g_select_threshold = reinterpret_cast<FcsSelectThresholdFn>(sym("fcs_select_threshold"));
     g_run_call = reinterpret_cast<FcsRunCallFn>(sym("fcs_run_call"));
-    if (!g_last_error || !g_select_topk || !g_select_threshold || !g_run_call) {
+    g_run_host_call = reinterpret_cast<FcsRunHostCallFn>(sym("fcs_run_host_call"));
+    if (!g_last_error || !g_select_topk || !g_select_threshold || !g_run_call || !g_run_host_call) {
         PyErr_SetString(PyExc_RuntimeError, "flash_colsum_b200: the CUDA library lacks an entry point of this binding");
         return nullptr;
     }
@@ -288,6 +362,7 @@ constexpr PyCFunction fast(F f) { return reinterpret_cast<PyCFunction>(reinterpr
 PyMethodDef g_methods[] = {
     {"colsum", fast(py_colsum), METH_FASTCALL, nullptr},
     {"launch", fast(py_launch), METH_FASTCALL, nullptr},
+    {"host", fast(py_host), METH_FASTCALL, nullptr},
     {"topk", fast(py_topk), METH_FASTCALL, nullptr},
     {"threshold", fast(py_threshold), METH_FASTCALL, nullptr},
     {"bind", py_bind, METH_O, nullptr},

@@ -455,24 +455,6 @@ def threshold_columns(colsum: torch.Tensor, threshold: float, relative: bool = F
     return _load_native(colsum.device).threshold(colsum, float(threshold), bool(relative))
 
 
-_copy_streams: Dict[int, torch.cuda.Stream] = {}
-
-
-def _host_chunks(B: int, batch_chunk: Optional[int]):
-    """(first entry, entries) of the chunks a host-memory call is copied and computed in."""
-    if batch_chunk is not None:
-        if batch_chunk <= 0:
-            raise ValueError(f"batch_chunk must be positive, got {batch_chunk}")
-        return [(b0, min(batch_chunk, B - b0)) for b0 in range(0, B, batch_chunk)]
-    out, b0 = [], 0
-    while b0 < B:
-        left = B - b0
-        n = left - max(1, left // 4) if left > 2 else 1
-        out.append((b0, n))
-        b0 += n
-    return out
-
-
 def flash_colsum_host(
     query: torch.Tensor,
     key: torch.Tensor,
@@ -486,48 +468,27 @@ def flash_colsum_host(
     """``flash_colsum`` for inputs that live in host memory; returns a host tensor.
 
     Same arguments as :func:`flash_colsum`, but ``query`` and ``key`` are CPU
-    tensors (pinned memory makes the copies asynchronous).  A batched call is cut
-    along the batch into chunks whose host-to-device copies run on a second stream
-    while the chunk before is being computed, so the call costs about the copy time
-    of the inputs plus the compute of the last chunk.  By default the chunks shrink
-    towards the end (three quarters of what is left, then single entries): few large
-    copies, and only one entry's compute behind the last copy; ``batch_chunk`` asks
-    for uniform chunks of that many entries instead.
-    Causal and single-sample calls are copied in one piece.
+    tensors (pinned memory makes the copies asynchronous).  The call is cut into chunks
+    whose host-to-device copies run on a second stream while the chunk before is being
+    computed, so it costs about the copy time of the inputs.  By default the chunks shrink
+    towards the end (three quarters of the batch entries that are left, the last entry by
+    heads): few large copies, and little compute behind the last one; ``batch_chunk`` asks
+    for uniform chunks of that many batch entries instead.
     """
     if query.ndim != 4 or key.ndim != 4:
         raise ValueError(f"Expected 4D tensors, got query.ndim={query.ndim}, key.ndim={key.ndim}")
     if query.device.type != "cpu" or key.device.type != "cpu":
         raise ValueError("flash_colsum_host takes host tensors; use flash_colsum for CUDA tensors")
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    B = query.shape[0]
-    if is_causal or B == 1 or key.shape[0] != B:
-        out = flash_colsum(query.to(dev, non_blocking=True), key.to(dev, non_blocking=True), scale,
-                           is_causal, cls_len)
-        return out.cpu()
+    if batch_chunk is not None and batch_chunk <= 0 and not is_causal and query.shape[0] > 1:
+        raise ValueError(f"batch_chunk must be positive, got {batch_chunk}")
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    with torch.cuda.device(dev):
-        copy_stream = _copy_streams.get(idx)
-        if copy_stream is None:
-            copy_stream = _copy_streams[idx] = torch.cuda.Stream(device=dev)
-        main = torch.cuda.current_stream(dev)
-        out = torch.empty((B, key.shape[2]), dtype=torch.float32, device=dev)
-        copy_stream.wait_stream(main)
-        staged = []
-        for b0, n in _host_chunks(B, batch_chunk):
-            with torch.cuda.stream(copy_stream):
-                qd = query[b0:b0 + n].to(dev, non_blocking=True)
-                kd = key[b0:b0 + n].to(dev, non_blocking=True)
-                ready = torch.cuda.Event()
-                ready.record(copy_stream)
-            staged.append((b0, qd, kd, ready))
-        for b0, qd, kd, ready in staged:
-            main.wait_event(ready)
-            # a one-entry chunk takes the single-sample entry point, a longer one the batched one
-            out[b0:b0 + qd.shape[0]] = flash_colsum(qd, kd, scale, False, cls_len)
-            qd.record_stream(main)
-            kd.record_stream(main)
-        return out.cpu()
+    chunk = 0 if batch_chunk is None or is_causal else int(batch_chunk)
+    out = _load_native(torch.device("cuda", idx)).host(query.contiguous(), key.contiguous(), scale, is_causal, cls_len,
+                                                       idx, chunk)
+    if out is None:      # what is wrong with the arguments, or nothing to compute
+        out = flash_colsum(query.to(dev), key.to(dev), scale, is_causal, cls_len).cpu()
+    return out
 
 
 __all__ = ["flash_colsum", "flash_colsum_causal", "flash_colsum_host", "topk_columns", "threshold_columns",
