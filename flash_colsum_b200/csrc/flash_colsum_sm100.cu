@@ -1944,10 +1944,10 @@ static cudaError_t launch_threshold(const float* colsum, long long ld, int B, in
 // Host-memory calls: the operands are copied in chunks on a stream of their own while the chunk before is
 // computed.  The copies bound the call (64 MiB at 54 GB/s: 1.23 ms, against 0.27 ms of kernels), so that the
 // chunks are few and large at first and small at the end: three quarters of the batch entries that are left,
-// and the last entry by heads (whose sums are added up on the device), until less than half a MiB of it is
-// behind the last copy -- about what a launch takes to get going.
+// and the last entry by heads (whose sums are added up on the device), down to chunks of 2 MiB (40 us; 1 MiB
+// and 4 MiB: the 8 x 16 x 2048 call 1335 and 1304 us against 1303, 64 x 16 x 512 2518 and 2523 against 2509).
 // ---------------------------------------------------------------------------
-constexpr size_t HOST_CHUNK_MIN_BYTES = 1u << 20;
+constexpr size_t HOST_CHUNK_MIN_BYTES = 2u << 20;
 
 static cudaStream_t host_copy_stream() {
     static cudaStream_t streams[64] = {nullptr};
@@ -1989,16 +1989,19 @@ static int run_host_call(const FcsHostCall* hc) {
     const FcsCall& c = hc->call;
     const size_t es = c.dtype == FCS_DTYPE_FP32 ? 4 : 2;
     const size_t q_pair = (size_t)c.Sq * c.D * es, k_pair = (size_t)c.Sk * c.D * es;
-    cudaStream_t copy = host_copy_stream(), main = reinterpret_cast<cudaStream_t>(c.stream);
-    if (!copy) return fail(FCS_ERR_CUDA, "no stream for the copies");
+    cudaStream_t main = reinterpret_cast<cudaStream_t>(c.stream);
     const std::vector<HostChunk> chunks = host_chunks(c.B, c.H, q_pair + k_pair, hc->batch_chunk);
-    std::vector<cudaEvent_t> events(chunks.size() + 1, nullptr);
+    // (one chunk: nothing to overlap, everything goes on the caller's stream)
+    const bool overlap = chunks.size() > 1;
+    cudaStream_t copy = overlap ? host_copy_stream() : main;
+    if (overlap && !copy) return fail(FCS_ERR_CUDA, "no stream for the copies");
+    std::vector<cudaEvent_t> events(overlap ? chunks.size() + 1 : 0, nullptr);
     cudaError_t e = cudaSuccess;
     for (auto& ev : events)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     // the device buffers may still be in use by earlier work of the caller's stream
-    if (e == cudaSuccess) e = cudaEventRecord(events.back(), main);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(copy, events.back(), 0);
+    if (overlap && e == cudaSuccess) e = cudaEventRecord(events.back(), main);
+    if (overlap && e == cudaSuccess) e = cudaStreamWaitEvent(copy, events.back(), 0);
     auto copy_in = [&](size_t i) {
         const HostChunk& ch = chunks[i];
         const size_t first = (size_t)ch.b0 * c.H + ch.h0, n = (size_t)ch.nb * ch.nh;
@@ -2009,13 +2012,13 @@ static int run_host_call(const FcsHostCall* hc) {
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(const_cast<uint8_t*>(bytes(c.k, first * k_pair)), bytes(hc->host_k, first * k_pair), n * k_pair,
                                 cudaMemcpyHostToDevice, copy);
-        if (e == cudaSuccess) e = cudaEventRecord(events[i], copy);
+        if (overlap && e == cudaSuccess) e = cudaEventRecord(events[i], copy);
     };
     int rc = FCS_OK;
     if (e == cudaSuccess) copy_in(0);
     for (size_t i = 0; i < chunks.size() && e == cudaSuccess && rc == FCS_OK; ++i) {
         if (i + 1 < chunks.size()) copy_in(i + 1);     // (queued before the kernels of this chunk are)
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(main, events[i], 0);
+        if (overlap && e == cudaSuccess) e = cudaStreamWaitEvent(main, events[i], 0);
         if (e != cudaSuccess) break;
         const HostChunk& ch = chunks[i];
         const size_t first = (size_t)ch.b0 * c.H + ch.h0;
@@ -2028,7 +2031,7 @@ static int run_host_call(const FcsHostCall* hc) {
     if (e == cudaSuccess && rc == FCS_OK)
         e = cudaMemcpyAsync(hc->host_out, c.out, (size_t)c.B * c.Sk * sizeof(float), cudaMemcpyDeviceToHost, main);
     // (also on the way out of an error: nothing of this call is left in flight over the caller's buffers)
-    const cudaError_t e2 = cudaStreamSynchronize(copy), e3 = cudaStreamSynchronize(main);
+    const cudaError_t e2 = overlap ? cudaStreamSynchronize(copy) : cudaSuccess, e3 = cudaStreamSynchronize(main);
     for (auto ev : events)
         if (ev) cudaEventDestroy(ev);
     if (rc != FCS_OK) return rc;
