@@ -451,36 +451,35 @@ template <int DK, int T>
 struct ClusterStage {
     static constexpr int ROWS = T == T_FP32 ? 32 : 64 * 64 / DK;
     static constexpr int BYTES = ROWS * DK * (T == T_FP32 ? 4 : 2);
-    static constexpr int RING = CONSUMER_WARPS * BYTES;
 };
-constexpr int CLUSTER_FIXED = 2 * CONSUMER_WARPS * 8 + 16 + CONSUMER_WARPS * MAX_ROWS * 8;
 // a stage per warp, [R][keys] scores, barriers and the warps' statistics
-template <int DK, int T>
+template <int DK, int T, int W>
 constexpr int cluster_smem(int R, int keys) {
-    return ClusterStage<DK, T>::RING + R * ((keys + 3) / 4 * 4) * 4 + CLUSTER_FIXED + 128;
+    return W * ClusterStage<DK, T>::BYTES + R * ((keys + 3) / 4 * 4) * 4 + 2 * W * 8 + 16 + W * MAX_ROWS * 8 + 128;
 }
 
-template <int DK, int T, int R>
-__global__ void __launch_bounds__(THREADS, 2)
+// W: consumer warps, eight with two CTAs per SM or four with four.
+template <int DK, int T, int R, int W>
+__global__ void __launch_bounds__(32 * (W + 1), 16 / W)
 few_rows_cluster_kernel(const __grid_constant__ CUtensorMap tm_k, const Params p) {
     using S = ClusterStage<DK, T>;
     using Dots = typename DotsOf<DK, T, R>::type;
     extern __shared__ uint8_t few_smem[];
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(few_smem) + 127) & ~static_cast<uintptr_t>(127));
     const int pitch = (p.keys + 3) / 4 * 4;
-    float* score = reinterpret_cast<float*>(ring + S::RING);        // [R][pitch]; row 0 becomes the head's columns
+    float* score = reinterpret_cast<float*>(ring + W * S::BYTES);        // [R][pitch]; row 0 becomes the head's columns
     uint8_t* fixed = reinterpret_cast<uint8_t*>(score + p.R * pitch);
     const uint32_t bars = smem_u32(fixed);
     auto full_bar = [&](int w) { return bars + 8u * w; };
-    auto empty_bar = [&](int w) { return bars + 8u * (CONSUMER_WARPS + w); };
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(fixed + 2 * CONSUMER_WARPS * 8);
-    float2* red = reinterpret_cast<float2*>(fixed + 2 * CONSUMER_WARPS * 8 + 16);     // [warps][MAX_ROWS]
+    auto empty_bar = [&](int w) { return bars + 8u * (W + w); };
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(fixed + 2 * W * 8);
+    float2* red = reinterpret_cast<float2*>(fixed + 2 * W * 8 + 16);     // [warps][MAX_ROWS]
 
     if (clusters_pack(p.H)) grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = (int)smallq_cluster_rank(), b = (int)blockIdx.x / p.H;
     if (threadIdx.x == 0) {
-        for (int w = 0; w < CONSUMER_WARPS; ++w) { mbar_init(full_bar(w), 1); mbar_init(empty_bar(w), 1); }
+        for (int w = 0; w < W; ++w) { mbar_init(full_bar(w), 1); mbar_init(empty_bar(w), 1); }
         *abort_flag = 0;
         mbar_fence_init();
         prefetch_tensormap(&tm_k);
@@ -490,10 +489,10 @@ few_rows_cluster_kernel(const __grid_constant__ CUtensorMap tm_k, const Params p
     const int stages = (p.keys + S::ROWS - 1) / S::ROWS;
     bool ok = true;
 
-    if (warp == CONSUMER_WARPS) {
+    if (warp == W) {
         // ------------------------------------------------ copies (whole tiles: rows past the keys read as zero)
         for (int n = 0; n < stages && ok; ++n) {
-            const int w = n % CONSUMER_WARPS, m = n / CONSUMER_WARPS;
+            const int w = n % W, m = n / W;
             if (m > 0) {
                 ok = mbar_wait(empty_bar(w), (m & 1) ^ 1, abort_flag, p.status, FCS_STATUS_WAIT_PRODUCER);
                 ok = __all_sync(0xffffffffu, ok);
@@ -514,7 +513,7 @@ few_rows_cluster_kernel(const __grid_constant__ CUtensorMap tm_k, const Params p
         float tm[COLS], tl[COLS];
 #pragma unroll
         for (int j = 0; j < COLS; ++j) { tm[j] = -INFINITY; tl[j] = 0.f; }
-        for (int n = warp, m = 0; n < stages; n += CONSUMER_WARPS, ++m) {
+        for (int n = warp, m = 0; n < stages; n += W, ++m) {
             ok = ok && mbar_wait(full_bar(warp), m & 1, abort_flag, p.status, FCS_STATUS_WAIT_CONSUMER);
             ok = __all_sync(0xffffffffu, ok);
             float v[NV][COLS];
@@ -537,27 +536,27 @@ few_rows_cluster_kernel(const __grid_constant__ CUtensorMap tm_k, const Params p
             }
             if (lane < Dots::LANE_STEP && col0 + j < p.R) red[warp * MAX_ROWS + col0 + j] = make_float2(tm[j], tl[j]);
         }
-        smallq_consumer_sync<CONSUMER_WARPS>();          // scores and statistics are in
-        float M[R], W[R];
+        smallq_consumer_sync<W>();          // scores and statistics are in
+        float M[R], weight[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            M[r] = 0.f; W[r] = 0.f;
+            M[r] = 0.f; weight[r] = 0.f;
             if (r < p.R) {
-                float2 t[CONSUMER_WARPS];
+                float2 t[W];
                 float mm = -INFINITY, ll = 0.f;
 #pragma unroll
-                for (int w = 0; w < CONSUMER_WARPS; ++w) { t[w] = red[w * MAX_ROWS + r]; mm = fmaxf(mm, t[w].x); }
+                for (int w = 0; w < W; ++w) { t[w] = red[w * MAX_ROWS + r]; mm = fmaxf(mm, t[w].x); }
 #pragma unroll
-                for (int w = 0; w < CONSUMER_WARPS; ++w) ll += t[w].y * ex2_approx(t[w].x - mm);
+                for (int w = 0; w < W; ++w) ll += t[w].y * ex2_approx(t[w].x - mm);
                 M[r] = mm;
-                W[r] = ok ? p.inv_norm / ll : 0.f;
+                weight[r] = ok ? p.inv_norm / ll : 0.f;
             }
         }
-        for (int k = threadIdx.x; k < p.keys; k += CONSUMER_THREADS) {
+        for (int k = threadIdx.x; k < p.keys; k += 32 * W) {
             float v = 0.f;
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                if (r < p.R) v += ex2_approx(score[r * pitch + k] - M[r]) * W[r];
+                if (r < p.R) v += ex2_approx(score[r * pitch + k] - M[r]) * weight[r];
             score[k] = v;
         }
     }
@@ -566,7 +565,7 @@ few_rows_cluster_kernel(const __grid_constant__ CUtensorMap tm_k, const Params p
     smallq_cluster_arrive();
     smallq_cluster_wait();
     const int per = (p.Sk + p.H - 1) / p.H, k1 = (h + 1) * per < p.Sk ? (h + 1) * per : p.Sk;
-    for (int k = h * per + (int)threadIdx.x; k < k1; k += THREADS) {
+    for (int k = h * per + (int)threadIdx.x; k < k1; k += 32 * (W + 1)) {
         float v = 0.f;
         if (k < p.keys) {
             float x[CLUSTER_MAX];

@@ -1179,12 +1179,12 @@ static cudaError_t launch_few_rows_t(const CUtensorMap& tk, const few::Params& f
     cfg.dynamicSmemBytes = 0;
     return cudaLaunchKernelEx(&cfg, few::few_rows_columns_kernel, fp);
 }
-template <int DK, int T, int R>
-static cudaError_t launch_few_rows_cluster_t(const CUtensorMap& tk, const few::Params& fp, int smem, cudaStream_t stream) {
+template <int DK, int T, int R, int W>
+static cudaError_t launch_few_rows_cluster_w(const CUtensorMap& tk, const few::Params& fp, cudaStream_t stream) {
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
-    auto kern = few::few_rows_cluster_kernel<DK, T, R>;
+    auto kern = few::few_rows_cluster_kernel<DK, T, R, W>;
     if (dev >= 0 && dev < 64 && !configured[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, few::CLUSTER_SMEM_LIMIT);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -1194,8 +1194,8 @@ static cudaError_t launch_few_rows_cluster_t(const CUtensorMap& tk, const few::P
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)fp.units);
-    cfg.blockDim = dim3(few::THREADS);
-    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.blockDim = dim3(32 * (W + 1));
+    cfg.dynamicSmemBytes = (size_t)few::cluster_smem<DK, T, W>(fp.R, fp.keys);
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
     attrs[0].id = cudaLaunchAttributeClusterDimension;
@@ -1209,6 +1209,11 @@ static cudaError_t launch_few_rows_cluster_t(const CUtensorMap& tk, const few::P
     return cudaLaunchKernelEx(&cfg, kern, tk, fp);
 }
 
+template <int DK, int T, int R>
+static cudaError_t launch_few_rows_cluster_t(const CUtensorMap& tk, const few::Params& fp, bool narrow, cudaStream_t stream) {
+    return narrow ? launch_few_rows_cluster_w<DK, T, R, 4>(tk, fp, stream) : launch_few_rows_cluster_w<DK, T, R, 8>(tk, fp, stream);
+}
+
 // Which form takes a call with at most four query rows.  Measured back to back on a B200, us per call in
 // clusters per batch entry / in two kernels / in clusters over key ranges (colsum_small_q.cuh; "-": it
 // does not take the call or is far behind), one CLS row over B x H x keys of 64 columns unless said:
@@ -1218,14 +1223,21 @@ static cudaError_t launch_few_rows_cluster_t(const CUtensorMap& tk, const few::P
 //     16 x 16 x 700 of 80   14.8 / 12.6 /  -         8 x 16 x 2048, 3 rows 20.7 / 16.6 / 18.0
 //     8 x 2000 of 128          - /  8.1 /  6.7       32 x 4096 of 128         - / 12.0 / 12.2
 //     32 x 32768 of 128        - / 50.4 / 60.4       the same, 4 rows         - / 64.6 / 98.6
-enum : int { FEW_CLUSTER = 0, FEW_TWO_KERNELS = 1, FEW_KEY_RANGES = 2 };
-static int few_rows_form(int B, int H, int R, int keys, int D, int row_bytes, bool dense, bool fp32, int smem, int sms) {
+// and in clusters with four CTAs per SM: 25 x 16 x 577, 4 rows 10.2 (two kernels 17.9), 40 x 12 x 300 of 80
+// 7.0 (12.7), 32 x 12 x 257 of 128 7.4 (key ranges 9.5), 64 x 8 x 577 11.5 (12.3), but 32 x 16 x 577 16.5 (12.1).
+enum : int { FEW_CLUSTER = 0, FEW_CLUSTER_NARROW = 3, FEW_TWO_KERNELS = 1, FEW_KEY_RANGES = 2 };
+static int few_rows_form(int B, int H, int R, int keys, int D, int row_bytes, bool dense, bool fp32, int smem, int smem_narrow, int sms) {
     const long long units = (long long)B * H, unit_bytes = (long long)keys * row_bytes;
     // many short units keep four CTAs on every SM busy; few bytes in all are over before two launches are
     const bool ranges_ok = !fp32 && dense && (D == 64 || D == 128);
     const bool many_short = units >= 2 * sms && unit_bytes <= 80 * 1024;
-    const bool one_wave = H <= few::CLUSTER_MAX && units <= 2 * sms && smem <= few::CLUSTER_SMEM_LIMIT;
-    if (one_wave && unit_bytes <= 80 * 1024) return FEW_CLUSTER;
+    if (H <= few::CLUSTER_MAX && unit_bytes <= 80 * 1024) {
+        if (units <= 2 * sms && smem <= few::CLUSTER_SMEM_LIMIT) return FEW_CLUSTER;
+        // four CTAs of four consumer warps per SM, as long as all clusters run at once (large ones do not fill
+        // every SM); where the alternative is two kernels, in two rounds as well
+        const long long at_once = H <= 8 ? 4ll * sms : 13ll * sms / 4;
+        if (smem_narrow <= 55 * 1024 && units <= (ranges_ok ? at_once : 6ll * sms)) return FEW_CLUSTER_NARROW;
+    }
     if (ranges_ok && R <= 2 && (many_short || units * unit_bytes <= (6ll << 20))) return FEW_KEY_RANGES;
     return FEW_TWO_KERNELS;
 }
@@ -1253,27 +1265,29 @@ static int launch_few_rows(const void* q, const void* k, float* out, int64_t out
     memset(&tk, 0, sizeof(tk));
     int rc;
     cudaError_t e;
-    const int smem = fp32 ? (D <= 64 ? few::cluster_smem<64, few::T_FP32>(R, fp.keys) : few::cluster_smem<128, few::T_FP32>(R, fp.keys))
-                     : D <= 64 ? few::cluster_smem<64, few::T_FP16>(R, fp.keys) : few::cluster_smem<128, few::T_FP16>(R, fp.keys);
-    const int form = few_rows_form(B, H, R, fp.keys, D, D * (fp32 ? 4 : 2), kss == D, fp32, smem, sms);
+    auto cluster_bytes = [&](int w) {
+        const int stages = w * (fp32 ? 32 * (D <= 64 ? 64 : 128) * 4 : 8192);
+        return stages + few::cluster_smem<64, few::T_FP16, 1>(R, fp.keys) - few::ClusterStage<64, few::T_FP16>::BYTES + w * 48;
+    };
+    const int form = few_rows_form(B, H, R, fp.keys, D, D * (fp32 ? 4 : 2), kss == D, fp32, cluster_bytes(8), cluster_bytes(4), sms);
     if (form == FEW_KEY_RANGES)
         return launch_small_q(q, k, out, out_ld, B, H, R, Sk, D, dtype, qsb, qsh, qss, ksb, ksh, kss, scale, causal,
                               k_past, h_norm, true, status, stream);
-    if (form == FEW_CLUSTER) {
+    if (form == FEW_CLUSTER || form == FEW_CLUSTER_NARROW) {
         const int rows = fp32      ? few::ClusterStage<64, few::T_FP32>::ROWS
                          : D <= 64 ? few::ClusterStage<64, few::T_FP16>::ROWS
                                    : few::ClusterStage<128, few::T_FP16>::ROWS;
         if ((rc = make_plain_tensor_map(&tk, k, dtype, B, H, Sk, D, ksb, ksh, kss, rows)) != FCS_OK) return rc;
         if (fp32)
-            e = D <= 64 ? (R == 1 ? launch_few_rows_cluster_t<64, few::T_FP32, 1>(tk, fp, smem, stream)
-                                  : launch_few_rows_cluster_t<64, few::T_FP32, 4>(tk, fp, smem, stream))
-                        : (R == 1 ? launch_few_rows_cluster_t<128, few::T_FP32, 1>(tk, fp, smem, stream)
-                                  : launch_few_rows_cluster_t<128, few::T_FP32, 4>(tk, fp, smem, stream));
+            e = D <= 64 ? (R == 1 ? launch_few_rows_cluster_t<64, few::T_FP32, 1>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
+                                  : launch_few_rows_cluster_t<64, few::T_FP32, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream))
+                        : (R == 1 ? launch_few_rows_cluster_t<128, few::T_FP32, 1>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
+                                  : launch_few_rows_cluster_t<128, few::T_FP32, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream));
         else
-            e = D <= 64 ? (bf16 ? launch_few_rows_cluster_t<64, few::T_BF16, 4>(tk, fp, smem, stream)
-                            : launch_few_rows_cluster_t<64, few::T_FP16, 4>(tk, fp, smem, stream))
-                    : (bf16 ? launch_few_rows_cluster_t<128, few::T_BF16, 4>(tk, fp, smem, stream)
-                            : launch_few_rows_cluster_t<128, few::T_FP16, 4>(tk, fp, smem, stream));
+            e = D <= 64 ? (bf16 ? launch_few_rows_cluster_t<64, few::T_BF16, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
+                            : launch_few_rows_cluster_t<64, few::T_FP16, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream))
+                    : (bf16 ? launch_few_rows_cluster_t<128, few::T_BF16, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
+                            : launch_few_rows_cluster_t<128, few::T_FP16, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream));
         if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "few-row cluster form launch failed: %s", cudaGetErrorString(e));
         return FCS_OK;
     }

@@ -22,6 +22,7 @@ CASES = [  # B, H, Sq, Sk, D, causal, cls
     (2, 5, 500, 500, 40, False, 3),
     (1, 4, 4, 9000, 128, True, None),       # four rows: two kernels
     (1, 20, 1, 3000, 96, True, None),
+    (50, 8, 60, 60, 64, False, 2),          # many pairs: four CTAs of a cluster per SM
 ]
 
 

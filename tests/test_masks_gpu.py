@@ -33,3 +33,19 @@ def test_extreme_scores_and_a_scale_of_zero(B, H, Sq, Sk, D, causal, jump, scale
     rel, mx = parity_errors(got, want)
     # (scores in the hundreds of thousands: an fp32 score has no more than a percent of a unit)
     assert rel <= (REL_L2_TOL if jump <= 30 else 0.1), (jump, rel, mx)
+
+
+@pytest.mark.parametrize("B,H,S,D,cls", [(50, 8, 150, 64, 1), (38, 12, 33, 128, 4), (45, 10, 280, 40, 3), (20, 16, 300, 64, 2)])
+def test_few_rows_over_many_pairs(B, H, S, D, cls):
+    """Clusters per batch entry with four CTAs per SM, contiguous and strided."""
+    if not torch.cuda.is_available():
+        pytest.fail("the gpu-marked tests need a CUDA device")
+    import flash_colsum_b200 as fc
+    q, k = make_inputs(Workload("few", B, H, S, S, D, "bf16", cls_len=cls, seed=B + S))
+    want = c_oracle.colsum_c(q, k, cls_len=cls)
+    for strided in (False, True):
+        a, b = (t.transpose(1, 2).contiguous().cuda().transpose(1, 2) if strided else t.cuda() for t in (q, k))
+        got = fc.flash_colsum(a, b, cls_len=cls).cpu().numpy()
+        assert fc.device_status() == 0
+        rel, mx = parity_errors(got, want)
+        assert rel <= REL_L2_TOL and mx <= REL_L2_TOL, (strided, rel, mx)
