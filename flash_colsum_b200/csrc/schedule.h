@@ -225,7 +225,7 @@ struct StatsItems {
     }
     FCS_HD void next(const Problem& p) {
         item += grid;
-        if (grid != p.stats_grid || p.stats_heads > 0) { load(p); return; }    // (no digits for this grid or order: decode afresh)
+        if (grid != p.stats_grid) { load(p); return; }    // (no digits for this grid or order: decode afresh)
         if (item >= p.stats_items) { done = true; return; }
         // add the grid's digits, with carries
         sp += p.stats_d_sp;
@@ -247,7 +247,7 @@ struct StatsItems {
 
 // The digits of `grid` (the statistics pass's CTA count) for StatsItems::next; call before launching it.
 inline void stats_set_grid(Problem& p, int grid) {
-    p.stats_grid = grid;
+    p.stats_grid = p.stats_heads > 0 ? 0 : grid;      // (rounds of heads have no digits)
     long long g = grid;
     p.stats_d_sp = (int)(g % p.nsplit);
     g /= p.nsplit;
