@@ -19,8 +19,8 @@ constexpr uint32_t IDESC_BF16 = (1u << 7) | (1u << 10);
 #ifndef FCS_POLY_PAIRS
 #define FCS_POLY_PAIRS 5
 #endif
-__host__ __device__ constexpr bool pair_uses_polynomial(int pair) {
-    return ((pair * FCS_POLY_PAIRS) % 16) < FCS_POLY_PAIRS;
+__host__ __device__ constexpr bool pair_uses_polynomial(int pair, int of_16 = FCS_POLY_PAIRS) {
+    return ((pair * of_16) % 16) < of_16;
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;

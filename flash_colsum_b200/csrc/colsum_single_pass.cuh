@@ -204,6 +204,8 @@ __device__ __forceinline__ float max_of_32(const uint32_t (&r)[32]) {
 
 // exp2(c*s - m) of 8 scores -> four packed fp16 pairs; adds the fp32 values to `sum`.
 // `pair0` is the index (mod 16) of the first pair in the exp-unit / polynomial pattern.
+// POLY: pairs of 16 that the polynomial takes.
+template <int POLY>
 __device__ __forceinline__ void exp8_packed(int pair0, const uint32_t* s, f32x2 c2, f32x2 nm2, f32x2& sum0,
                                             f32x2& sum1, uint32_t* h) {
 #pragma unroll
@@ -211,7 +213,7 @@ __device__ __forceinline__ void exp8_packed(int pair0, const uint32_t* s, f32x2 
         const f32x2 t = fma2(pack2(__uint_as_float(s[2 * pr]), __uint_as_float(s[2 * pr + 1])), c2, nm2);
         f32x2 e;
         float e0, e1;
-        if (pair_uses_polynomial((pair0 + pr) & 15)) {
+        if (pair_uses_polynomial((pair0 + pr) & 15, POLY)) {
             e = ex2_poly2(t);
             unpack2(e, e0, e1);
         } else {
@@ -536,6 +538,9 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         // second copy of it for the ragged group does not fit the instruction cache next to the first
         // (385-447 keys: 89 us a call against 62)
         const int padding = keys_valid < 64 ? 64 - keys_valid : 0;
+        // (5 of 16 pairs on the FMA pipe, where it is short of time; a cluster that waits for its ragged CTA is not:
+        // 577 keys 117.3 us with 5, 113.0 with 3, 115.2 with 2; 1024 keys 232.7 / 234.6 / 232.6)
+        constexpr int POLY = PADDED ? 3 : FCS_POLY_PAIRS;
         auto consume = [&](auto keys) {
         constexpr bool KEYS = decltype(keys)::value;     // false: nothing but padding
         int i = 0, fc = 0;
@@ -567,10 +572,10 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_g, -m_g);
                     f32x2 sum0 = pack2(0.f, 0.f), sum1 = sum0;
 #pragma unroll
-                    for (int j8 = 0; j8 < 4; ++j8) exp8_packed(j8 * 4, &sa[8 * j8], c2, nm2, sum0, sum1, &h[4 * j8]);
+                    for (int j8 = 0; j8 < 4; ++j8) exp8_packed<POLY>(j8 * 4, &sa[8 * j8], c2, nm2, sum0, sum1, &h[4 * j8]);
 #pragma unroll
                     for (int j8 = 0; j8 < 4; ++j8)
-                        exp8_packed(j8 * 4, &sb[8 * j8], c2, nm2, sum0, sum1, &h[16 + 4 * j8]);
+                        exp8_packed<POLY>(j8 * 4, &sb[8 * j8], c2, nm2, sum0, sum1, &h[16 + 4 * j8]);
                     float x0, x1;
                     unpack2(add2(sum0, sum1), x0, x1);
                     l_g = x0 + x1;
