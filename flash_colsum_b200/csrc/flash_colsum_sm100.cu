@@ -1655,6 +1655,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
     int Sq = Sq_full;                       // rows that enter the mean
     if (!causal && cls_n > 0 && cls_n < Sq_full) Sq = cls_n;
     if (causal && k_past < 0) k_past = Sk > Sq ? Sk - Sq : 0;
+    if (causal && k_past > Sk) k_past = Sk;   // (every row sees every key; the kernels add the row index in 32 bits)
 
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
     if (passes == PASSES_BOTH && !sig && alloc && clear_out && Sq <= few::MAX_ROWS) {
