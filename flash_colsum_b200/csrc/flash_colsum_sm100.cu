@@ -1695,7 +1695,8 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
     if (sig && passes == PASSES_BOTH && smallq_fits(Sq, Sk, D, B * H, num_sms()))
         return fail(FCS_ERR_UNSUPPORTED, "calls with at most four query rows take the few-row kernel, which does not "
                                          "signal other GPUs; order them with a barrier");
-    if (passes == PASSES_BOTH && smallq_fits(Sq, Sk, D, B * H, num_sms())) {
+    // (a type that is decided on the device is known to the kernels below this one only)
+    if (passes == PASSES_BOTH && !fmt_word && smallq_fits(Sq, Sk, D, B * H, num_sms())) {
         // reported as a call whose statistics and merge passes take no time
         PassTimers* tms = g_profiling ? timers_for_current_device() : nullptr;
         if (tms) {
@@ -1976,7 +1977,9 @@ static cudaStream_t host_copy_stream() {
 
 struct HostChunk { int b0, nb, h0, nh; };
 
-static std::vector<HostChunk> host_chunks(int B, int H, size_t pair_bytes, int batch_chunk) {
+// (`whole`: no entry is cut -- calls with at most four query rows, whose kernels take a hundredth of the copies'
+// time and write the columns instead of adding to them)
+static std::vector<HostChunk> host_chunks(int B, int H, size_t pair_bytes, int batch_chunk, bool whole) {
     std::vector<HostChunk> out;
     if (batch_chunk > 0) {
         for (int b = 0; b < B; b += batch_chunk) out.push_back({b, B - b < batch_chunk ? B - b : batch_chunk, 0, H});
@@ -1989,6 +1992,10 @@ static std::vector<HostChunk> host_chunks(int B, int H, size_t pair_bytes, int b
         const int n = left - (left / 4 > 1 ? left / 4 : 1);
         out.push_back({b, n, 0, H});
         b += n;
+    }
+    if (whole) {
+        out.push_back({b, 1, 0, H});
+        return out;
     }
     for (int h = 0; h < H;) {
         const int left = H - h;
@@ -2005,7 +2012,8 @@ static int run_host_call(const FcsHostCall* hc) {
     const size_t es = c.dtype == FCS_DTYPE_FP32 ? 4 : 2;
     const size_t q_pair = (size_t)c.Sq * c.D * es, k_pair = (size_t)c.Sk * c.D * es;
     cudaStream_t main = reinterpret_cast<cudaStream_t>(c.stream);
-    const std::vector<HostChunk> chunks = host_chunks(c.B, c.H, q_pair + k_pair, hc->batch_chunk);
+    const int rows = !c.causal && c.cls_n > 0 && c.cls_n < c.Sq ? c.cls_n : c.Sq;
+    const std::vector<HostChunk> chunks = host_chunks(c.B, c.H, q_pair + k_pair, hc->batch_chunk, rows <= few::MAX_ROWS);
     // (one chunk: nothing to overlap, everything goes on the caller's stream)
     const bool overlap = chunks.size() > 1;
     cudaStream_t copy = overlap ? host_copy_stream() : main;

@@ -31,3 +31,22 @@ def test_the_largest_k_past_shows_every_key(fc, Sq, D, dtype):
         assert fc.device_status() == 0
         rel, mx = parity_errors(got, want)
         assert rel <= REL_L2_TOL, (k_past, rel, mx)
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,D,causal,cls", [
+    (2, 16, 2000, 2000, 64, False, 1),      # 16 MB an entry: several chunks
+    (1, 12, 1500, 1500, 128, False, 4),
+    (1, 16, 2, 9000, 64, True, None),
+])
+def test_host_calls_with_few_rows_outside_the_range_of_fp16(fc, B, H, Sq, Sk, D, causal, cls):
+    """Every chunk of an fp32 call takes the few-row forms, which leave values past fp16's range as they are."""
+    q, k = make_inputs(Workload("host_fp32", B, H, Sq, Sk, D, "fp32", is_causal=causal, cls_len=cls, seed=Sk))
+    q = q * 1e5
+    scale = D ** -0.5 / 1e5
+    rows = cls or Sq
+    ref = [torch.where(t.abs() < 60000, t.half().float(), t) for t in (q[:, :, :rows], k)]
+    want = naive_colsum_f64(*ref, scale=scale, is_causal=causal)
+    got = fc.flash_colsum_host(q.pin_memory(), k.pin_memory(), scale=scale, is_causal=causal, cls_len=cls)
+    assert fc.device_status() == 0
+    rel, mx = parity_errors(got.numpy(), want)
+    assert rel <= REL_L2_TOL, (rel, mx)
