@@ -17,6 +17,7 @@
 #include <dlfcn.h>
 
 #include <cmath>
+#include <exception>
 #include <vector>
 
 #include "../../include/flash_colsum_b200.h"
@@ -51,15 +52,25 @@ at::Tensor empty_f32(int64_t rows, int64_t cols, c10::Device dev) {
 }
 
 // Scratch of one call; freed when the call returns (the caching allocator hands it out again in
-// stream order only).
+// stream order only).  What the allocator throws does not pass through the library, which has copies
+// in flight to wait for: it is kept, and thrown again by `rethrow` once the library has returned.
 struct Scratch {
     c10::Device dev;
     std::vector<at::Tensor> held;
-    static void* alloc(void* ctx, size_t bytes) {
+    std::exception_ptr error;
+    static void* alloc(void* ctx, size_t bytes) noexcept {
         Scratch* s = static_cast<Scratch*>(ctx);
-        const int64_t size[1] = {static_cast<int64_t>(bytes)};
-        s->held.push_back(at::detail::empty_cuda(c10::IntArrayRef(size, 1), at::kByte, s->dev, std::nullopt));
-        return s->held.back().mutable_data_ptr();
+        try {
+            const int64_t size[1] = {static_cast<int64_t>(bytes)};
+            s->held.push_back(at::detail::empty_cuda(c10::IntArrayRef(size, 1), at::kByte, s->dev, std::nullopt));
+            return s->held.back().mutable_data_ptr();
+        } catch (...) {
+            s->error = std::current_exception();
+            return nullptr;
+        }
+    }
+    void rethrow() const {
+        if (error) std::rethrow_exception(error);
     }
 };
 
@@ -117,10 +128,11 @@ PyObject* run(at::Tensor q, at::Tensor k, double scale, bool causal, int k_past,
         c.h_norm = h_norm;
         c.status = g_status[dev.index()];
         c.stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-        Scratch scratch{dev, {}};
+        Scratch scratch{dev, {}, nullptr};
         c.alloc = &Scratch::alloc;
         c.alloc_ctx = &scratch;
         rc = g_run_call(&c);
+        scratch.rethrow();
     }
     if (rc != FCS_OK) return raise_library_error(rc);
     return THPVariable_Wrap(std::move(out));
@@ -244,7 +256,7 @@ PyObject* py_host(PyObject*, PyObject* const* args, Py_ssize_t n) {
         c.h_norm = 0;
         c.status = g_status[idx];
         c.stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)idx).stream();
-        Scratch scratch{dev, {}};
+        Scratch scratch{dev, {}, nullptr};
         c.alloc = &Scratch::alloc;
         c.alloc_ctx = &scratch;
         hc.host_q = q.const_data_ptr();
@@ -252,6 +264,7 @@ PyObject* py_host(PyObject*, PyObject* const* args, Py_ssize_t n) {
         hc.host_out = static_cast<float*>(host_out.mutable_data_ptr());
         hc.batch_chunk = (int)(batch_chunk < 0x7fffffffL ? batch_chunk : 0x7fffffffL);
         rc = g_run_host_call(&hc);
+        scratch.rethrow();
     }
     if (rc != FCS_OK) return raise_library_error(rc);
     return THPVariable_Wrap(std::move(host_out));

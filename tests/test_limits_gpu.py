@@ -1,9 +1,12 @@
 """Calls at the limits of what the operator takes, against the plain float64 evaluation."""
 
+import subprocess
+import sys
+
 import pytest
 import torch
 
-from conftest import REL_L2_TOL
+from conftest import REL_L2_TOL, ROOT
 from flash_colsum_b200.inputs import Workload, make_inputs
 from oracle.naive_colsum import naive_colsum_f64, parity_errors
 
@@ -50,3 +53,37 @@ def test_host_calls_with_few_rows_outside_the_range_of_fp16(fc, B, H, Sq, Sk, D,
     assert fc.device_status() == 0
     rel, mx = parity_errors(got.numpy(), want)
     assert rel <= REL_L2_TOL, (rel, mx)
+
+
+OUT_OF_MEMORY = """
+import torch
+import flash_colsum_b200 as fc
+from flash_colsum_b200.inputs import Workload, make_inputs
+q, k = (t.pin_memory() for t in make_inputs(Workload("oom", 8, 16, 2048, 2048, 64, "fp16", seed=5)))
+want = fc.flash_colsum_host(q, k)                   # (32 MB an operand; the first chunk's scratch is 7 MB)
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+total = torch.cuda.get_device_properties(0).total_memory
+torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (70 << 20)) / total)
+try:
+    fc.flash_colsum_host(q, k)
+    raise SystemExit("the call found memory after all")
+except torch.OutOfMemoryError:
+    pass
+# the operands' memory comes back for these, and nothing writes to it any more
+again = [torch.full((8 << 20,), 1.0, device="cuda") for _ in range(2)]
+torch.cuda.synchronize()
+torch.cuda.set_per_process_memory_fraction(1.0)
+assert all(bool((t == 1.0).all()) for t in again)
+del again
+torch.testing.assert_close(fc.flash_colsum_host(q, k), want, rtol=3e-4, atol=1e-8)
+assert fc.device_status() == 0
+"""
+
+
+def test_a_host_call_that_runs_out_of_memory_leaves_nothing_in_flight(fc):
+    """The scratch of the first chunk cannot be had while two chunks are being copied: the call raises torch's
+    error after the copies have ended, so that the memory they went to can be used at once.  (In a process of its
+    own, whose allocator holds nothing that would serve after all.)"""
+    done = subprocess.run([sys.executable, "-c", OUT_OF_MEMORY], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stdout + done.stderr
