@@ -320,7 +320,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 const float2 o = xch[i * TILE + row];
                 ll += o.y * exp2f(o.x - ms);
             }
-            const float nlv = (ok && row < p.Sq) ? -(mm + log2f(ll) + p.log2_norm) : -INFINITY;
+            const float nlv = (ok && row < p.Sq) ? negative_lse(mm, ll, p.log2_norm) : -INFINITY;
             lse_buf[row] = nlv;
             lse_buf[TILE + row] = -INFINITY;
             uint4 e0, e1;

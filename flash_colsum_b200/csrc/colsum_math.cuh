@@ -4,6 +4,7 @@
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <float.h>
 #include <math.h>
 
 #include "sm100_ptx.cuh"
@@ -58,8 +59,8 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
         m_safe = (m_new == -INFINITY) ? 0.f : m_new;
         l *= ex2_approx(m - m_safe);
         m = m_new;
-    } else {        // all 32 scores are finite
-        m_safe = fmaxf(m, cm * c);
+    } else {        // (the floor: where all of them are -inf -- masked keys -- their exps are zero)
+        m_safe = max3(m, cm * c, -FLT_MAX);
         l *= ex2_approx(m - m_safe);
         m = m_safe;
     }
@@ -98,6 +99,12 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
         }
         l += (a0 + a1) + (a2 + a3);
     }
+}
+
+// -(log2-sum-exp + log2_norm) of a row from its (maximum, sum); NaN, as the softmax has it, for a row whose
+// scores are all -inf (a maximum at the floor above, or none).
+__device__ __forceinline__ float negative_lse(float m, float l, float log2_norm) {
+    return m > -FLT_MAX ? -(m + log2f(l) + log2_norm) : nanf("");
 }
 
 // Add exp2(c*s - lse[q]) of 32 query columns into a key's accumulators.  `nl`

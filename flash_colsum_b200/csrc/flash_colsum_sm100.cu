@@ -571,7 +571,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             const long long bh = (long long)pend_b * p.H + pend_h;
             const int q_abs = pend_qt * TILE + row;
             if (p.nsplit == 1) {
-                const float nlv = (q_abs < p.Sq) ? -(mm + log2f(ll) + p.log2_norm) : -INFINITY;
+                const float nlv = (q_abs < p.Sq) ? negative_lse(mm, ll, p.log2_norm) : -INFINITY;
                 p.neg_lse[bh * p.lse_rows + q_abs] = nlv;
                 uint4 e0, e1;
                 make_ext_row(nlv, p.inv_c, ps.ext_bf16 != 0, e0, e1);
@@ -816,7 +816,7 @@ __global__ void merge_stats_kernel(const Problem p) {
                 const float2 t = part[s * n + idx];
                 ll += t.y * exp2f(t.x - mm);
             }
-            v = -(mm + log2f(ll) + p.log2_norm);
+            v = negative_lse(mm, ll, p.log2_norm);
         }
         p.neg_lse[bh * p.lse_rows + q_abs] = v;
         uint4 e0, e1;

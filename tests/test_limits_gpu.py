@@ -87,3 +87,44 @@ def test_a_host_call_that_runs_out_of_memory_leaves_nothing_in_flight(fc):
     own, whose allocator holds nothing that would serve after all.)"""
     done = subprocess.run([sys.executable, "-c", OUT_OF_MEMORY], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stdout + done.stderr
+
+
+def masked_inputs(B, H, Sq, Sk, D, dtype, causal, where, value):
+    """Keys that a mask in the first feature takes out: the query's is 1 there, theirs `value`, the others' 0."""
+    q, k = make_inputs(Workload("masked", B, H, Sq, Sk, D, dtype, is_causal=causal, seed=Sq + Sk + D))
+    q[..., 0], k[..., 0] = 1.0, 0.0
+    value = torch.finfo(q.dtype).min if value == "lowest" else float("-inf")
+    if where == "tail":
+        k[:, :, Sk * 2 // 3:, 0] = value
+    elif where == "group":
+        k[:, :, 64:128, 0] = value
+    else:
+        k[:, :, -1, 0] = value
+    return q, k
+
+
+@pytest.mark.parametrize("Sq,Sk,causal", [
+    (128, 128, False), (150, 150, False), (200, 200, False), (330, 330, False), (700, 700, False),   # non-causal
+    (128, 200, True), (128, 700, True), (60, 1500, True),                # one-kernel form
+    (200, 200, True), (129, 130, True), (900, 900, True), (300, 5000, True),      # streaming passes
+])
+@pytest.mark.parametrize("D,dtype,scale", [(128, "fp16", None), (72, "bf16", 1.0)])
+@pytest.mark.parametrize("where,value", [("tail", "-inf"), ("group", "-inf"), ("last", "-inf"), ("tail", "lowest")])
+def test_masked_keys(fc, Sq, Sk, causal, D, dtype, scale, where, value):
+    """Scores of -inf weigh nothing, wherever a tile's visible columns begin with a run of them."""
+    q, k = masked_inputs(2 if not causal else 1, 3, Sq, Sk, D, dtype, causal, where, value)
+    got = fc.flash_colsum(q.cuda(), k.cuda(), scale=scale, is_causal=causal).cpu().numpy()
+    assert fc.device_status() == 0
+    rel, mx = parity_errors(got, naive_colsum_f64(q, k, scale=scale, is_causal=causal))
+    assert rel <= REL_L2_TOL and mx <= REL_L2_TOL, (rel, mx)
+
+
+@pytest.mark.parametrize("S,D", [(200, 128), (700, 128)])
+def test_a_head_without_a_key_left_gives_nan(fc, S, D):
+    """The softmax of nothing but -inf: the batch entry's means are NaN, the other entry's are not."""
+    q, k = masked_inputs(2, 3, S, S, D, "fp16", False, "tail", "-inf")
+    k[0, 1, :, 0] = float("-inf")
+    got = fc.flash_colsum(q.cuda(), k.cuda()).cpu()
+    assert torch.isnan(got[0]).all()
+    rel, _ = parity_errors(got[1:].numpy(), naive_colsum_f64(q[1:], k[1:]))
+    assert rel <= REL_L2_TOL
