@@ -39,7 +39,7 @@ struct SinglePassParams {
     int units;              // B * H
     int clusters;           // gridDim.x / CL
     int flush_units;        // most (batch, head) pairs accumulated in tensor memory before a flush
-    float c;                // |scale| * log2(e)
+    float c;                // |scale| * log2(e), never zero
     float out_scale;        // 1 / (h_norm * R * 2^10): the weights are stored times 2^10
     float* out;
     long long out_ld;
@@ -527,7 +527,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const int w4 = warp & 3;                   // 32-row block of the tile
         const int row = (w4 << 5) | lane;          // tensor-memory lane = query row of the tile
         const uint32_t lane_base = tmem_base + ((uint32_t)(w4 << 5) << 16);
-        const float c = PADDED ? fmaxf(p.c, 1.0e-30f) : p.c;      // (a scale of zero: every visible score still counts as 2^0)
+        const float c = p.c;
         const int keys_valid = p.Sk - (256 * (int)rank + 64 * wg);   // >= 64: the whole group is real keys
         // this thread's 128-byte line of P~ (one line per query row and 64-key group)
         const uint32_t p_line = (uint32_t)(hf * P_TILE_BYTES + half64 * P_ATOM_COL_BYTES + (row >> 3) * 1024 +
@@ -555,7 +555,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 tc_fence_after();
                 uint32_t sa[32], sb[32];   // columns 0..31 and 32..63 of the group
                 if constexpr (KEYS) {
-                    if (PADDED && padding > 0) tmem_fill(lane_base + 64 * wg + keys_valid, padding, __float_as_uint(-3.0e38f));
+                    if (PADDED && padding > 0) tmem_fill(lane_base + 64 * wg + keys_valid, padding, __float_as_uint(-INFINITY));
                     tmem_ld_x32(lane_base + 64 * wg, sa);
                     tmem_ld_x32(lane_base + 64 * wg + 32, sb);
                     tmem_ld_wait(sa);

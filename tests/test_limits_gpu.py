@@ -128,3 +128,15 @@ def test_a_head_without_a_key_left_gives_nan(fc, S, D):
     assert torch.isnan(got[0]).all()
     rel, _ = parity_errors(got[1:].numpy(), naive_colsum_f64(q[1:], k[1:]))
     assert rel <= REL_L2_TOL
+
+
+@pytest.mark.parametrize("S", [150, 256, 577, 1000])
+@pytest.mark.parametrize("scale", [1e-36, -1e-36, 0.0])
+def test_scales_at_the_end_of_the_range(fc, S, scale):
+    """bf16 scores of 1e36 under a scale of 1e-36 are ordinary; under a scale of zero every key counts the same."""
+    q, k = make_inputs(Workload("scale", 2, 3, S, S, 64, "fp32", seed=S))
+    q, k = (q * 1e18).bfloat16(), (k * 1e17).bfloat16()
+    got = fc.flash_colsum(q.cuda(), k.cuda(), scale=scale).cpu().numpy()
+    assert fc.device_status() == 0
+    rel, mx = parity_errors(got, naive_colsum_f64(q, k, scale=scale))
+    assert rel <= REL_L2_TOL, (rel, mx)
