@@ -26,6 +26,8 @@
 // 400 keys 71 -> 63, 577 137 -> 117; the rule for which calls come here is with the launcher.
 #pragma once
 
+#include <float.h>
+
 #include "colsum_math.cuh"
 #include "schedule.h"
 #include "sm100_ptx.cuh"
@@ -427,7 +429,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 float L = 0.f;
 #pragma unroll
                 for (int r = 0; r < MAX_CL; ++r) L = fmaf(o[r].y, ex2_approx(o[r].x - M), L);
-                const float base = W_SCALE_LOG2 - M - __log2f(L);
+                const float base = M > -FLT_MAX ? W_SCALE_LOG2 - M - __log2f(L) : nanf("");   // (a row without a key left)
                 const bool live = t * 128 + row < p.Sq;   // rows past the end of the query axis weigh nothing
                 // columns 2a (hi), 2a + 1 (lo) of half hf's operand belong to group 2*hf + a
                 const uint32_t w_row = w_smem + (row >> 4) * 512 + (row & 15) * 2;
@@ -568,7 +570,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 uint32_t h[32];
                 float m_g = -INFINITY, l_g = 0.f;
                 if constexpr (KEYS) {
-                    m_g = fmaxf(max_of_32(sa), max_of_32(sb)) * c;
+                    m_g = max3(max_of_32(sa) * c, max_of_32(sb) * c, -FLT_MAX);   // (nothing but -inf -- masked keys -- has exps of zero)
                     const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_g, -m_g);
                     f32x2 sum0 = pack2(0.f, 0.f), sum1 = sum0;
 #pragma unroll
@@ -590,6 +592,10 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 mbar_arrive(stats_bar(slot));
                 const uint32_t line = p_smem + slot * P_BYTES + p_line;
                 if constexpr (KEYS) {
+                    if (t * 128 + row >= p.Sq) {   // past the query axis: weighs zero, but zero times a masked key is NaN
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) h[j] = 0u;
+                    }
 #pragma unroll
                     for (int j8 = 0; j8 < 8; ++j8)
                         st_shared_v4(line + ((((uint32_t)j8) ^ sw) << 4), h[4 * j8], h[4 * j8 + 1], h[4 * j8 + 2],

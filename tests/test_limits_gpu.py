@@ -104,11 +104,12 @@ def masked_inputs(B, H, Sq, Sk, D, dtype, causal, where, value):
 
 
 @pytest.mark.parametrize("Sq,Sk,causal", [
-    (128, 128, False), (150, 150, False), (200, 200, False), (330, 330, False), (700, 700, False),   # non-causal
+    (128, 128, False), (150, 150, False), (200, 200, False), (330, 330, False), (700, 700, False),
+    (513, 513, False), (577, 577, False), (1024, 1024, False),           # non-causal (to 64 columns: the single pass)
     (128, 200, True), (128, 700, True), (60, 1500, True),                # one-kernel form
     (200, 200, True), (129, 130, True), (900, 900, True), (300, 5000, True),      # streaming passes
 ])
-@pytest.mark.parametrize("D,dtype,scale", [(128, "fp16", None), (72, "bf16", 1.0)])
+@pytest.mark.parametrize("D,dtype,scale", [(128, "fp16", None), (72, "bf16", 1.0), (64, "fp16", None), (40, "bf16", 1.0)])
 @pytest.mark.parametrize("where,value", [("tail", "-inf"), ("group", "-inf"), ("last", "-inf"), ("tail", "lowest")])
 def test_masked_keys(fc, Sq, Sk, causal, D, dtype, scale, where, value):
     """Scores of -inf weigh nothing, wherever a tile's visible columns begin with a run of them."""
@@ -119,7 +120,7 @@ def test_masked_keys(fc, Sq, Sk, causal, D, dtype, scale, where, value):
     assert rel <= REL_L2_TOL and mx <= REL_L2_TOL, (rel, mx)
 
 
-@pytest.mark.parametrize("S,D", [(200, 128), (700, 128)])
+@pytest.mark.parametrize("S,D", [(200, 128), (700, 128), (150, 64), (577, 64), (1024, 64)])
 def test_a_head_without_a_key_left_gives_nan(fc, S, D):
     """The softmax of nothing but -inf: the batch entry's means are NaN, the other entry's are not."""
     q, k = masked_inputs(2, 3, S, S, D, "fp16", False, "tail", "-inf")
