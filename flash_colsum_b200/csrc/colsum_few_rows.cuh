@@ -243,7 +243,7 @@ __device__ __forceinline__ void keep_scores(const Params& p, const float (&v)[NV
         const bool seen = kl < rows && (!p.causal || lo + kl <= p.k_past + col);
         s[x] = seen ? v[x][j] * p.c : -INFINITY;
         if (kl < rows) dst[kl] = s[x];
-        m = fmaxf(m, s[x]);
+        m = max_or_nan(m, s[x]);
     }
     if (m != -INFINITY) {
         float l = tl * ex2_approx(tm - m);

@@ -263,6 +263,13 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
+// The larger of two values, NaN if one of them is (fmaxf drops it).
+__device__ __forceinline__ float max_or_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // Two fp32 values in one 64-bit register, for the packed fp32 instructions.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) {

@@ -141,3 +141,27 @@ def test_scales_at_the_end_of_the_range(fc, S, scale):
     assert fc.device_status() == 0
     rel, mx = parity_errors(got, naive_colsum_f64(q, k, scale=scale))
     assert rel <= REL_L2_TOL, (rel, mx)
+
+
+def with_nan(q, k, what, at):
+    t = (q if what == "query" else k).clone()
+    t[0, 0, at, 3] = float("nan")
+    return (t, k) if what == "query" else (q, t)
+
+
+@pytest.mark.parametrize("B,H,Sk,D,R,dtype", [
+    (2, 4, 577, 64, 1, "fp16"),        # a cluster per batch entry
+    (1, 20, 577, 104, 4, "bf16"),      # two kernels
+    (2, 4, 5000, 128, 2, "fp16"),
+    (50, 8, 60, 64, 2, "fp16"),        # four CTAs of a cluster per SM
+    (2, 4, 700, 80, 3, "fp32"),
+])
+def test_few_rows_pass_nan_on(fc, B, H, Sk, D, R, dtype):
+    """A NaN in a key makes its head's rows NaN, and so the batch entry's means; the other entries' stay."""
+    q, k = make_inputs(Workload("nan", B, H, R, Sk, D, dtype, is_causal=True, seed=Sk + D))
+    want = fc.flash_colsum_causal(q.cuda(), k.cuda(), k_past=Sk).cpu()
+    for at in (0, 1, 7, Sk // 2, Sk - 2, Sk - 1):
+        qn, kn = with_nan(q, k, "key", at)
+        got = fc.flash_colsum_causal(qn.cuda(), kn.cuda(), k_past=Sk).cpu()
+        assert torch.isnan(got[0]).all(), at
+        torch.testing.assert_close(got[1:], want[1:])
