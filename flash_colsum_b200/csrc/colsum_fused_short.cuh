@@ -367,7 +367,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             tc_fence_before();
             mbar_arrive(t_empty(buf));
             const int k_abs = ktg * TILE + row;
-            const float v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+            const float v = column_sum(acc);
             // system scope: `out` may live on another GPU and take adds from several
             if (ok && k_abs < p.Sk && v != 0.f) atomicAdd_system(dst + k_abs, v);
             acc[0] = acc[1] = acc[2] = acc[3] = 0.f;

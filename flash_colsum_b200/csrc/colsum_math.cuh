@@ -23,9 +23,10 @@ constexpr uint32_t IDESC_BF16 = (1u << 7) | (1u << 10);
 __host__ __device__ constexpr bool pair_uses_polynomial(int pair, int of_16 = FCS_POLY_PAIRS) {
     return ((pair * of_16) % 16) < of_16;
 }
+// The largest of three values, NaN if one of them is.
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
 
@@ -51,7 +52,7 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
     }
     m0 = max3(m0, s[28], s[29]);
     m1 = max3(m1, s[30], s[31]);
-    const float cm = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+    const float cm = max_or_nan(max_or_nan(m0, m1), max_or_nan(m2, m3));
     float m_safe;
     if (MASKED) {   // a row may see nothing of this block (or nothing yet): keep -inf out of the arithmetic
         const float scaled = (cm == -INFINITY) ? -INFINITY : cm * c;
@@ -101,10 +102,17 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
     }
 }
 
-// -(log2-sum-exp + log2_norm) of a row from its (maximum, sum); NaN, as the softmax has it, for a row whose
-// scores are all -inf (a maximum at the floor above, or none).
+// -(log2-sum-exp + log2_norm) of a row from its (maximum, sum); NaN, as the softmax has it, for a row with a
+// score of +inf, and for one whose scores are all -inf (a maximum at the floor above, or none).
 __device__ __forceinline__ float negative_lse(float m, float l, float log2_norm) {
-    return m > -FLT_MAX ? -(m + log2f(l) + log2_norm) : nanf("");
+    return fabsf(m) < FLT_MAX ? -(m + log2f(l) + log2_norm) : nanf("");
+}
+
+// The sum a thread has collected for its key.  The polynomial turns a NaN (a row whose statistics are) into
+// FLT_MAX; no sum of shares of one comes near that.
+__device__ __forceinline__ float column_sum(const float (&acc)[4]) {
+    const float v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    return v < 1.0e38f ? v : nanf("");
 }
 
 // Add exp2(c*s - lse[q]) of 32 query columns into a key's accumulators.  `nl`

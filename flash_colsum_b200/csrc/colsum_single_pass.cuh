@@ -201,7 +201,7 @@ __device__ __forceinline__ float max_of_32(const uint32_t (&r)[32]) {
     }
     m0 = max3(m0, __uint_as_float(r[28]), __uint_as_float(r[29]));
     m1 = max3(m1, __uint_as_float(r[30]), __uint_as_float(r[31]));
-    return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+    return max_or_nan(max_or_nan(m0, m1), max_or_nan(m2, m3));
 }
 
 // exp2(c*s - m) of 8 scores -> four packed fp16 pairs; adds the fp32 values to `sum`.

@@ -739,13 +739,12 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                     if (p.col_pack == 2) { tg = wg >> 1; mine = tg < it.nt; }
                     const int k_abs = (it.kt + tg) * TILE + row;
                     if (k_abs < p.Sk && mine)
-                        atomicAdd_system(p.out + (long long)it.b * p.out_ld + k_abs,
-                                         (acc[0] + acc[1]) + (acc[2] + acc[3]));
+                        atomicAdd_system(p.out + (long long)it.b * p.out_ld + k_abs, column_sum(acc));
                     acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
                 } else {
                     if (cpend) { ok = finish_cols(); if (!ok) break; }
                     const int slot = item_cnt & (MERGE_SLOTS - 1);
-                    colbuf[(slot * CONSUMER_GROUPS + wg) * TILE + row] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+                    colbuf[(slot * CONSUMER_GROUPS + wg) * TILE + row] = column_sum(acc);
                     mbar_arrive(merge_bar(slot));
                     if ((item_cnt % CONSUMER_GROUPS) == wg) {
                         cpend = true;
@@ -758,8 +757,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                     const int k_abs = it.kt * TILE + row;
                     if (k_abs < p.Sk)
                         // system scope: `out` may live on another GPU and take adds from several
-                        atomicAdd_system(p.out + (long long)it.b * p.out_ld + k_abs,
-                                         (acc[0] + acc[1]) + (acc[2] + acc[3]));
+                        atomicAdd_system(p.out + (long long)it.b * p.out_ld + k_abs, column_sum(acc));
                     acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
                 }
             }

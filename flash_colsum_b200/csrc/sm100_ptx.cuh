@@ -307,14 +307,14 @@ __device__ __forceinline__ f32x2 add2_round_down(f32x2 a, f32x2 b) {
 }
 
 // exp2 of two values without the special-function unit, for arguments <= 0
-// (clamped at -126, where the result is 2^-126 rather than 0).
+// (clamped at -126, where the result is 2^-126 rather than 0; NaN becomes FLT_MAX).
 // t = n + f with n = floor(t): adding 1.5 * 2^23 rounding down leaves n in the low
 // mantissa bits; 2^f on [0, 1) is a cubic with p(0) = 1 whose relative error is
 // below 9.4e-5 and averages to zero over f; n goes straight into the exponent.
 __device__ __forceinline__ f32x2 ex2_poly2(f32x2 t) {
     float t0, t1;
     unpack2(t, t0, t1);
-    const f32x2 tc = pack2(fmaxf(t0, -126.f), fmaxf(t1, -126.f));
+    const f32x2 tc = pack2(max_or_nan(t0, -126.f), max_or_nan(t1, -126.f));
     const f32x2 magic = pack2(12582912.f, 12582912.f);
     const f32x2 r = add2_round_down(tc, magic);
     const f32x2 f = sub2(tc, sub2(r, magic));

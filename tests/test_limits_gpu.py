@@ -165,3 +165,30 @@ def test_few_rows_pass_nan_on(fc, B, H, Sk, D, R, dtype):
         got = fc.flash_colsum_causal(qn.cuda(), kn.cuda(), k_past=Sk).cpu()
         assert torch.isnan(got[0]).all(), at
         torch.testing.assert_close(got[1:], want[1:])
+
+
+@pytest.mark.parametrize("Sq,Sk,causal", [
+    (65, 65, False), (150, 150, False), (256, 256, False), (577, 577, False), (700, 700, False), (1024, 1024, False),
+    (128, 200, True), (128, 700, True),                                     # one-kernel form
+    (129, 130, True), (300, 300, True), (300, 5000, True), (900, 900, True),     # streaming passes
+])
+@pytest.mark.parametrize("D,dtype", [(64, "fp16"), (128, "bf16"), (80, "fp32")])
+@pytest.mark.parametrize("what,value", [("key", "nan"), ("query", "nan"), ("key", "inf")])
+def test_nan_is_passed_on(fc, Sq, Sk, causal, D, dtype, what, value):
+    """A NaN in a key that every row sees, or in a query row, makes the batch entry's means NaN (the keys the row
+    sees, under a causal mask) and no other's, whichever exp unit its column falls to; so does a score of +inf."""
+    q, k = make_inputs(Workload("nan", 2, 2, Sq, Sk, D, dtype, is_causal=causal, seed=Sk + D))
+    if value == "inf":
+        q = q.abs()
+    # (fp32 operands with an infinite value are rounded to bf16, all of them: outside fp16's range)
+    qw, kw = (q.bfloat16(), k.bfloat16()) if dtype == "fp32" and value == "inf" else (q, k)
+    want = fc.flash_colsum_causal(qw.cuda(), kw.cuda()) if causal else fc.flash_colsum(qw.cuda(), kw.cuda())
+    rows = Sq if what == "query" else Sk - Sq + 1 if causal else Sk
+    for at in sorted({0, 1, 2, 3, 6, 14, 31, rows // 2, rows - 2, rows - 1} & set(range(rows))):
+        qn, kn = with_nan(q, k, what, at)
+        if value == "inf":
+            kn[0, 0, at, 3] = float("inf")
+        got = fc.flash_colsum_causal(qn.cuda(), kn.cuda()) if causal else fc.flash_colsum(qn.cuda(), kn.cuda())
+        seen = Sk if not causal or what == "key" else Sk - Sq + at + 1
+        assert torch.isnan(got[0, :seen]).all(), (at, int(torch.isnan(got[0]).sum()))
+        torch.testing.assert_close(got[1:], want[1:])
