@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import operator
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -19,6 +20,8 @@ import torch
 from . import _cabi
 
 _DTYPE_CODE = {torch.float16: _cabi.FCS_DTYPE_FP16, torch.bfloat16: _cabi.FCS_DTYPE_BF16}
+
+_INT_MAX = 2 ** 31 - 1
 
 # one sticky device-status word per device, zeroed once
 _status: Dict[int, torch.Tensor] = {}
@@ -334,7 +337,7 @@ def flash_colsum_causal(
         (B, K_len), fp32 unless ``out_dtype`` says otherwise.
     """
     if _native is not None and (k_past is None or k_past >= 0):
-        out = _native.launch(query, key, scale, True, -1 if k_past is None else k_past, -1, 0)
+        out = _native.launch(query, key, scale, True, -1 if k_past is None else min(int(k_past), _INT_MAX), -1, 0)
         if out is not None:
             return out if out_dtype is None or out_dtype == torch.float32 else out.to(out_dtype)
     if query.ndim != 4 or key.ndim != 4:
@@ -352,7 +355,7 @@ def flash_colsum_causal(
     out = _without_work(query, key)
     if out is not None:
         return out if out_dtype is None else out.to(out_dtype)
-    out = _launch(query, key, scale, True, -1 if k_past is None else int(k_past), -1, 0)
+    out = _launch(query, key, scale, True, -1 if k_past is None else min(int(k_past), _INT_MAX), -1, 0)
     if out_dtype is not None and out_dtype != out.dtype:
         out = out.to(out_dtype)
     return out
@@ -430,7 +433,7 @@ def topk_columns(colsum: torch.Tensor, k: int) -> Tuple[torch.Tensor, torch.Tens
     B, S = colsum.shape
     if not 1 <= k <= S:
         raise ValueError(f"k must be in 1..{S}, got {k}")
-    return _load_native(colsum.device).topk(colsum, int(k))
+    return _load_native(colsum.device).topk(colsum, operator.index(k))
 
 
 def threshold_columns(colsum: torch.Tensor, threshold: float, relative: bool = False

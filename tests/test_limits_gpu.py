@@ -3,6 +3,7 @@
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 import torch
 
@@ -192,3 +193,19 @@ def test_nan_is_passed_on(fc, Sq, Sk, causal, D, dtype, what, value):
         seen = Sk if not causal or what == "key" else Sk - Sq + at + 1
         assert torch.isnan(got[0, :seen]).all(), (at, int(torch.isnan(got[0]).sum()))
         torch.testing.assert_close(got[1:], want[1:])
+
+
+def test_number_arguments_of_other_types(fc):
+    """What int() takes is a k_past, whether or not the native path has been loaded; only a whole number of
+    any integer type is a k."""
+    q, k = (t.cuda() for t in make_inputs(Workload("args", 1, 2, 40, 300, 64, "fp16", is_causal=True, seed=3)))
+    want = fc.flash_colsum_causal(q, k, k_past=100)
+    for k_past in (100.0, 100.9, np.int64(100), np.float32(100), torch.tensor(100)):
+        assert torch.equal(fc.flash_colsum_causal(q, k, k_past=k_past) > 0, want > 0)
+    everything = fc.flash_colsum_causal(q, k, k_past=300)
+    torch.testing.assert_close(fc.flash_colsum_causal(q, k, k_past=2 ** 70), everything)
+    for k_top in (5, np.int32(5), torch.tensor(5)):
+        assert fc.topk_columns(want, k_top)[1].shape == (1, 5)
+    for k_top in (5.0, 5.5, "5"):
+        with pytest.raises(TypeError):
+            fc.topk_columns(want, k_top)
