@@ -192,7 +192,7 @@ def _flash_colsum_causal(Q: torch.Tensor, K: torch.Tensor, scale: float, K_past:
     """
     k_past = -1 if K_past is None else int(K_past)
     if accumulate_into is None:
-        return _launch(Q, K, scale, True, k_past, -1, int(h_norm))
+        return _launch(Q[:1], K[:1], scale, True, k_past, -1, int(h_norm))
     lib = _cabi.load()
     Q, K, code = _prepare(Q, K)
     _, H, Q_len, D = Q.shape

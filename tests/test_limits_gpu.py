@@ -209,3 +209,11 @@ def test_number_arguments_of_other_types(fc):
     for k_top in (5.0, 5.5, "5"):
         with pytest.raises(TypeError):
             fc.topk_columns(want, k_top)
+
+
+def test_the_single_sample_launcher_takes_the_first_entry(fc):
+    from flash_colsum_b200.ops import _flash_colsum_causal
+    q, k = (t.cuda() for t in make_inputs(Workload("first", 3, 2, 40, 300, 64, "fp16", is_causal=True, seed=4)))
+    got = _flash_colsum_causal(q, k, 0.125)
+    assert got.shape == (1, 300)
+    torch.testing.assert_close(got, fc.flash_colsum(q[:1], k[:1], scale=0.125, is_causal=True))
