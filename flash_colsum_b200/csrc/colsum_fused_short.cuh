@@ -95,7 +95,6 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     float2* xch = reinterpret_cast<float2*>(smem + L::XCH_OFF);
     float* lse_buf = reinterpret_cast<float*>(smem + L::LSE_OFF);
 
-    if (clusters_pack(fp.CL)) grid_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t cr = smallq_cluster_rank();
@@ -131,6 +130,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (clusters_pack(fp.CL)) grid_launch_dependents();   // (not before this CTA has its tensor memory)
     // every CTA of the cluster has set up its barriers once this completes; it is waited for
     // before the first store into another CTA's shared memory
     smallq_cluster_arrive();

@@ -293,7 +293,6 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     float2* lstats = reinterpret_cast<float2*>(smem + LST_OFF);
     const float2* xchg = reinterpret_cast<const float2*>(smem + XCHG_OFF);
 
-    if (clusters_pack(p.CL)) grid_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
@@ -342,6 +341,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     cluster_sync_all();   // every CTA's barriers exist before a peer signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (clusters_pack(p.CL)) grid_launch_dependents();   // (not before this CTA has its tensor memory)
     grid_dependency_wait();   // the set-up is done; what follows reads the inputs and adds into the cleared output
 
     auto wait_all = [&](uint32_t bar, uint32_t parity, int code) -> bool {

@@ -43,7 +43,9 @@ __device__ __forceinline__ bool elect_one_sync() {
 // A kernel launched with the programmatic-serialization attribute may start while the
 // kernel before it in the stream is still running; `grid_dependency_wait` holds it until
 // that kernel has completed and its memory is visible (a no-op for an ordinary launch), and
-// `grid_launch_dependents` tells the scheduler that the next kernel may start filling SMs.
+// `grid_launch_dependents` tells the scheduler that the next kernel may start filling SMs.  A kernel
+// that uses tensor memory says so only once it has it: a dependent (of another library, say) that took
+// the columns first and then waited for this kernel would never be given up by either.
 __device__ __forceinline__ void grid_dependency_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
