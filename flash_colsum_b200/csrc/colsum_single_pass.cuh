@@ -41,7 +41,7 @@ struct SinglePassParams {
     int units;              // B * H
     int clusters;           // gridDim.x / CL
     int flush_units;        // most (batch, head) pairs accumulated in tensor memory before a flush
-    float c;                // |scale| * log2(e), never zero
+    float c;                // |scale| * log2(e); not zero where the key axis ends inside a group of 64
     float out_scale;        // 1 / (h_norm * R * 2^10): the weights are stored times 2^10
     float* out;
     long long out_ld;

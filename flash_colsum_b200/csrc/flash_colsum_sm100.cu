@@ -1401,9 +1401,9 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
     }
     // at most ~1024 accumulations (16 query rows each) per flush
     sp_.flush_units = 128 / sp_.NQ > 1 ? 128 / sp_.NQ : 1;
-    // (a scale of zero as the smallest number there is: every fp32 score times it is below 5e-7 in size, and the
-    // -inf of a column of padding stays -inf)
-    sp_.c = fmaxf(fabsf(scale) * 1.4426950408889634f, 1.4e-45f);
+    // (a scale of zero under a ragged end as the smallest number there is: every fp32 score times it is below 5e-7
+    // in size, and the -inf of a column of padding stays -inf)
+    sp_.c = fmaxf(fabsf(scale) * 1.4426950408889634f, Sk % 64 ? 1.4e-45f : 0.f);
     sp_.out_scale = 1.0f / ((float)h_norm * (float)Sq * 1024.0f);
     sp_.out = out;
     sp_.out_ld = out_ld;

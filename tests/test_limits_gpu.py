@@ -142,6 +142,8 @@ def test_scales_at_the_end_of_the_range(fc, S, scale):
     assert fc.device_status() == 0
     rel, mx = parity_errors(got, naive_colsum_f64(q, k, scale=scale))
     assert rel <= REL_L2_TOL, (rel, mx)
+    if scale == 0.0 and S % 64 == 0:
+        assert (got == 1.0 / S).all()        # (every exp is one, every sum exact)
 
 
 def with_nan(q, k, what, at):
