@@ -393,3 +393,39 @@ extern "C" long long check_stats_digits(int B, int H, int Sq, int Sk, int causal
     }
     return walked == p.stats_items ? walked : -4;
 }
+
+// Walks the statistics pass's items of all CTAs of a causal call: how many (b, h) pairs share a round of the
+// longest-first order (0: the plain order), or negative where an item is missing, comes twice, is empty, or is not
+// among the round's longest left.
+extern "C" int check_stats_order(int B, int H, int Sq, int Sk, int k_past, int sms) {
+    if (k_past < 0) k_past = Sk > Sq ? Sk - Sq : 0;
+    Problem p;
+    memset(&p, 0, sizeof(p));
+    plan(p, B, H, Sq, Sk, 1, k_past, sms);
+    const int grid = (int)(p.stats_items < sms ? p.stats_items : sms);
+    stats_set_grid(p, grid);
+    std::vector<char> seen((size_t)p.stats_items, 0);
+    std::vector<int> tile((size_t)p.stats_items, -1), pair((size_t)p.stats_items, -1);
+    for (int cta = 0; cta < grid; ++cta) {
+        StatsItems it;
+        it.init(p, cta, grid);
+        for (; !it.done; it.next(p)) {
+            if (it.b < 0 || it.b >= B || it.h < 0 || it.h >= H || it.qt < 0 || it.qt >= p.NQ || it.sp < 0 || it.sp >= p.nsplit)
+                return -1;
+            const size_t id = (((size_t)it.b * H + it.h) * p.NQ + it.qt) * p.nsplit + it.sp;
+            if (seen[id]) return -2;
+            seen[id] = 1;
+            if (it.s1 <= it.s0) return -3;
+            tile[(size_t)it.item] = it.qt;
+            pair[(size_t)it.item] = it.b * H + it.h;
+        }
+    }
+    for (char c : seen)
+        if (!c) return -4;
+    if (p.stats_heads > 0)
+        for (long long i = 1; i < p.stats_items; ++i) {
+            const int round = pair[i] / p.stats_heads, before = pair[i - 1] / p.stats_heads;
+            if (round < before || (round == before && tile[i] > tile[i - 1])) return -5;
+        }
+    return p.stats_heads;
+}

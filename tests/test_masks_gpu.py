@@ -49,3 +49,23 @@ def test_few_rows_over_many_pairs(B, H, S, D, cls):
         assert fc.device_status() == 0
         rel, mx = parity_errors(got, want)
         assert rel <= REL_L2_TOL and mx <= REL_L2_TOL, (strided, rel, mx)
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,D", [(1, 16, 4000, 4000, 64), (2, 16, 4000, 4100, 128), (1, 15, 6100, 20000, 64)])
+def test_causal_statistics_longest_tiles_first(B, H, Sq, Sk, D):
+    """Calls whose statistics items go by rounds of heads (24 query tiles and more, few items; the last shape in
+    rounds of 13 and 2), against a materialising evaluation in double precision."""
+    if not torch.cuda.is_available():
+        pytest.fail("the gpu-marked tests need a CUDA device")
+    import flash_colsum_b200 as fc
+    q, k = (t.cuda() for t in make_inputs(Workload("rounds", B, H, Sq, Sk, D, "bf16", is_causal=True, seed=Sq)))
+    got = fc.flash_colsum_causal(q, k).cpu().numpy()
+    assert fc.device_status() == 0
+    hidden = torch.arange(Sk, device="cuda")[None, :] > (Sk - Sq + torch.arange(Sq, device="cuda"))[:, None]
+    want = torch.zeros(B, Sk, dtype=torch.float64, device="cuda")
+    for b in range(B):
+        for h in range(H):
+            s = (q[b, h].double() @ k[b, h].double().T) / D ** 0.5
+            want[b] += torch.softmax(s.masked_fill_(hidden, float("-inf")), dim=-1).sum(dim=0) / (H * Sq)
+    rel, mx = parity_errors(got, want.cpu().numpy())
+    assert rel <= REL_L2_TOL and mx <= REL_L2_TOL, (rel, mx)

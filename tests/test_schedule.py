@@ -34,6 +34,8 @@ def emu():
     lib.check_fused_short.argtypes = [ctypes.c_int] * 7 + [ctypes.c_void_p, ctypes.c_int]
     lib.check_stats_digits.restype = ctypes.c_longlong
     lib.check_stats_digits.argtypes = [ctypes.c_int] * 7
+    lib.check_stats_order.restype = ctypes.c_int
+    lib.check_stats_order.argtypes = [ctypes.c_int] * 6
     lib.scratch_need.restype = ctypes.c_longlong
     lib.scratch_need.argtypes = [ctypes.c_int] * 7 + [ctypes.c_void_p]
     return lib
@@ -300,3 +302,19 @@ def test_statistics_items_advance_by_digits(emu, B, H, Sq, Sk, causal, k_past, s
     """Going from one item of a CTA to its next by adding the grid's digits gives the same items as
     decoding every index afresh, for every CTA, and covers every item once."""
     assert emu.check_stats_digits(B, H, Sq, Sk, causal, k_past, sms) > 0
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,k_past,sms,heads", [
+    (1, 16, 4000, 4000, -1, 148, 16),       # all pairs in one round
+    (2, 16, 4000, 4100, -1, 148, 32),       # ... of two batch entries
+    (1, 15, 20000, 20000, -1, 148, 13),     # rounds of 13 and of 2
+    (3, 5, 6272, 60000, -1, 148, 4),        # rounds across batch entries, 15 = 3 x 4 + 3
+    (1, 3, 6272, 300000, 1000, 148, 1),     # a head a round
+    (1, 16, 2944, 2944, -1, 148, 0),        # 23 query tiles: the plain order
+    (1, 16, 2945, 2945, -1, 148, 16),       # 24
+    (4, 32, 4000, 4000, -1, 148, 0),        # 4096 items of 2368
+])
+def test_causal_statistics_items_longest_first(emu, B, H, Sq, Sk, k_past, sms, heads):
+    """Every item of the rounds of heads comes once, the longest query tiles of a round first."""
+    got = emu.check_stats_order(B, H, Sq, Sk, k_past, sms)
+    assert got == heads

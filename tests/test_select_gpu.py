@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("S", [1, 33, 1024, 1025, 4096, 4097, 8193, 16385, 32769, 65537, 131072, 131073, 300001])
-@pytest.mark.parametrize("B,ties", [(1, False), (2, True), (10, True)])    # (ten rows take smaller clusters)
+@pytest.mark.parametrize("B,ties", [(1, False), (2, True), (10, True)])    # (one row, and several at once)
 def test_selection_at_the_edges_of_the_launch_shapes(S, B, ties):
     if not torch.cuda.is_available():
         pytest.fail("the gpu-marked tests need a CUDA device")
