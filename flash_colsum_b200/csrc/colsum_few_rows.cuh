@@ -261,7 +261,7 @@ __device__ __forceinline__ float ld_peer_f32(uint32_t local_addr, uint32_t rank)
     return v;
 }
 
-// DK: 64 or 128, a bound on the head dimension; R: a bound on the query rows (fp32 operands: 1, 2, 4;
+// DK: 64 or 128, a bound on the head dimension; R: a bound on the query rows (fp32 operands: 1 or 4;
 // 16-bit operands: 4, the matrix instruction has eight columns anyway).
 template <int DK, int T, int R>
 __global__ void __launch_bounds__(THREADS, 1)

@@ -540,8 +540,10 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         // second copy of it for the ragged group does not fit the instruction cache next to the first
         // (385-447 keys: 89 us a call against 62)
         const int padding = keys_valid < 64 ? 64 - keys_valid : 0;
-        // (5 of 16 pairs on the FMA pipe, where it is short of time; a cluster that waits for its ragged CTA is not:
-        // 577 keys 117.3 us with 5, 113.0 with 3, 115.2 with 2; 1024 keys 232.7 / 234.6 / 232.6)
+        // Pairs of 16 on the FMA pipe.  In the padded instance 3 is the fastest throughout, one slice or several, the
+        // last one full or not; us per call with 2 / 3 / 4 / 5: 32 x 16 x 200 keys 25.2 / 24.6 / 24.9 / 25.3, 400 62.0 /
+        // 60.1 / 61.5 / 62.9, 577 114.3 / 112.0 / 114.4 / 117.5, 1000 237.5 / 231.7 / 234.6 / 242.0, 8 x 16 x 1500 139.0 /
+        // 136.2 / 137.3 / 140.2 (only 300: 62.0 / 62.0 / 61.8 / 61.5).  In the other 5: 1024 keys 234.6 with 3, 232.7 with 5.
         constexpr int POLY = PADDED ? 3 : FCS_POLY_PAIRS;
         auto consume = [&](auto keys) {
         constexpr bool KEYS = decltype(keys)::value;     // false: nothing but padding

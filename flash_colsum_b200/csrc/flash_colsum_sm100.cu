@@ -1062,8 +1062,7 @@ static int check_operand(const char* name, const void* ptr, int64_t sb, int64_t 
 // Few query rows: the matrix-vector kernel (a kernel that clears the output, then the
 // clustered kernel as its programmatic dependent).
 template <int D, bool BF16, int RMAX, int W>
-static cudaError_t launch_small_q_w(const SmallQParams& sp, int grid, size_t smem, cudaStream_t stream,
-                                    bool after_clear) {
+static cudaError_t launch_small_q_w(const SmallQParams& sp, int grid, size_t smem, cudaStream_t stream) {
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1095,18 +1094,16 @@ static cudaError_t launch_small_q_w(const SmallQParams& sp, int grid, size_t sme
 }
 
 template <int D, bool BF16, int RMAX>
-static cudaError_t launch_small_q_r(const SmallQParams& sp, int grid, size_t smem, cudaStream_t stream,
-                                    bool after_clear) {
-    if (sp.wide) return launch_small_q_w<D, BF16, RMAX, SMALLQ_WIDE_WARPS>(sp, grid, smem, stream, after_clear);
-    return launch_small_q_w<D, BF16, RMAX, SMALLQ_CONSUMER_WARPS>(sp, grid, smem, stream, after_clear);
+static cudaError_t launch_small_q_r(const SmallQParams& sp, int grid, size_t smem, cudaStream_t stream) {
+    if (sp.wide) return launch_small_q_w<D, BF16, RMAX, SMALLQ_WIDE_WARPS>(sp, grid, smem, stream);
+    return launch_small_q_w<D, BF16, RMAX, SMALLQ_CONSUMER_WARPS>(sp, grid, smem, stream);
 }
 
 template <int D, bool BF16>
-static cudaError_t launch_small_q_t(const SmallQParams& sp, int grid, size_t smem, cudaStream_t stream,
-                                    bool after_clear) {
-    if (sp.R == 1) return launch_small_q_r<D, BF16, 1>(sp, grid, smem, stream, after_clear);
-    if (sp.R == 2) return launch_small_q_r<D, BF16, 2>(sp, grid, smem, stream, after_clear);
-    return launch_small_q_r<D, BF16, 4>(sp, grid, smem, stream, after_clear);
+static cudaError_t launch_small_q_t(const SmallQParams& sp, int grid, size_t smem, cudaStream_t stream) {
+    if (sp.R == 1) return launch_small_q_r<D, BF16, 1>(sp, grid, smem, stream);
+    if (sp.R == 2) return launch_small_q_r<D, BF16, 2>(sp, grid, smem, stream);
+    return launch_small_q_r<D, BF16, 4>(sp, grid, smem, stream);
 }
 
 static int launch_small_q(const void* q, const void* k, float* out, int64_t out_ld, int B, int H, int R, int Sk,
@@ -1138,10 +1135,10 @@ static int launch_small_q(const void* q, const void* k, float* out, int64_t out_
     const int grid = sp.clusters * sp.CL;
     const bool bf16 = dtype == FCS_DTYPE_BF16;
     const cudaError_t e =
-        (D == 64) ? (bf16 ? launch_small_q_t<64, true>(sp, grid, smem, stream, clear_out)
-                          : launch_small_q_t<64, false>(sp, grid, smem, stream, clear_out))
-                  : (bf16 ? launch_small_q_t<128, true>(sp, grid, smem, stream, clear_out)
-                          : launch_small_q_t<128, false>(sp, grid, smem, stream, clear_out));
+        (D == 64) ? (bf16 ? launch_small_q_t<64, true>(sp, grid, smem, stream)
+                          : launch_small_q_t<64, false>(sp, grid, smem, stream))
+                  : (bf16 ? launch_small_q_t<128, true>(sp, grid, smem, stream)
+                          : launch_small_q_t<128, false>(sp, grid, smem, stream));
     if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "few-row kernel launch failed: %s", cudaGetErrorString(e));
     return FCS_OK;
 }
@@ -1276,11 +1273,9 @@ static int launch_few_rows(const void* q, const void* k, float* out, int64_t out
                          : D <= 64 ? few::ClusterStage<64, few::T_FP16>::ROWS
                                    : few::ClusterStage<128, few::T_FP16>::ROWS;
         if ((rc = make_plain_tensor_map(&tk, k, dtype, B, H, Sk, D, ksb, ksh, kss, rows)) != FCS_OK) return rc;
-        if (fp32)
-            e = D <= 64 ? (R == 1 ? launch_few_rows_cluster_t<64, few::T_FP32, 1>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
-                                  : launch_few_rows_cluster_t<64, few::T_FP32, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream))
-                        : (R == 1 ? launch_few_rows_cluster_t<128, few::T_FP32, 1>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
-                                  : launch_few_rows_cluster_t<128, few::T_FP32, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream));
+        if (fp32)   // (more than 64 columns never come here: the stages alone are over both limits)
+            e = R == 1 ? launch_few_rows_cluster_t<64, few::T_FP32, 1>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
+                       : launch_few_rows_cluster_t<64, few::T_FP32, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream);
         else
             e = D <= 64 ? (bf16 ? launch_few_rows_cluster_t<64, few::T_BF16, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream)
                             : launch_few_rows_cluster_t<64, few::T_FP16, 4>(tk, fp, form == FEW_CLUSTER_NARROW, stream))
