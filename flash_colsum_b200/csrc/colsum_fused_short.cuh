@@ -269,7 +269,7 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         int n = 0;
 
         // phase 1: running (maximum, sum) of this thread's query row over the group's columns
-        float m_run = -INFINITY, l_run = 0.f;
+        float m_run = ROW_MAX_START, l_run = 0.f;
         int f_lo, f_hi;
         stats_full_range(p, 0, f_lo, f_hi);
         for (int i = 0; i < nblk; ++i, ++n) {

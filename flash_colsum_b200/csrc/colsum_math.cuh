@@ -30,6 +30,9 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return r;
 }
 
+// Where a row's running maximum starts.
+constexpr float ROW_MAX_START = -FLT_MAX;
+
 // Online (max, sum) update of one query row with 32 more scores.
 // `last_valid`: columns 0..last_valid are visible (>= 31: all).
 template <bool MASKED>
@@ -53,18 +56,11 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
     m0 = max3(m0, s[28], s[29]);
     m1 = max3(m1, s[30], s[31]);
     const float cm = max_or_nan(max_or_nan(m0, m1), max_or_nan(m2, m3));
-    float m_safe;
-    if (MASKED) {   // a row may see nothing of this block (or nothing yet): keep -inf out of the arithmetic
-        const float scaled = (cm == -INFINITY) ? -INFINITY : cm * c;
-        const float m_new = fmaxf(m, scaled);
-        m_safe = (m_new == -INFINITY) ? 0.f : m_new;
-        l *= ex2_approx(m - m_safe);
-        m = m_new;
-    } else {        // (the floor: where all of them are -inf -- masked keys -- their exps are zero)
-        m_safe = max3(m, cm * c, -FLT_MAX);
-        l *= ex2_approx(m - m_safe);
-        m = m_safe;
-    }
+    // (m is at its start or above, so that a run of -inf -- hidden columns, masked keys -- has exps of zero; a row
+    // may see nothing of this block, and c may be 0)
+    const float m_safe = max_or_nan(m, MASKED && cm == -INFINITY ? -INFINITY : cm * c);
+    l *= ex2_approx(m - m_safe);
+    m = m_safe;
     if constexpr (!MASKED) {
         const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_safe, -m_safe);
         f32x2 s0 = pack2(0.f, 0.f), s1 = s0;
@@ -103,7 +99,7 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
 }
 
 // -(log2-sum-exp + log2_norm) of a row from its (maximum, sum); NaN, as the softmax has it, for a row with a
-// score of +inf, and for one whose scores are all -inf (a maximum at the floor above, or none).
+// score of +inf, and for one whose scores are all -inf (the maximum is where it started, or is none).
 __device__ __forceinline__ float negative_lse(float m, float l, float log2_norm) {
     return fabsf(m) < FLT_MAX ? -(m + log2f(l) + log2_norm) : nanf("");
 }

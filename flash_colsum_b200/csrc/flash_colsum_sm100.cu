@@ -544,7 +544,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 
         Items it;
         it.init(ps, blockIdx.x, gridDim.x);
-        float m_run = -INFINITY, l_run = 0.f;      // statistics pass state
+        float m_run = ROW_MAX_START, l_run = 0.f;      // statistics pass state
         float acc[4] = {0.f, 0.f, 0.f, 0.f};       // column pass state
         int item_cnt = 0, n = 0;
         // statistics pass: the item whose partials this group still has to combine
@@ -730,7 +730,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                     pending = true;
                     pend_cnt = item_cnt; pend_b = it.b; pend_h = it.h; pend_qt = it.qt; pend_sp = it.sp;
                 }
-                m_run = -INFINITY; l_run = 0.f;
+                m_run = ROW_MAX_START; l_run = 0.f;
             } else if constexpr (L::SHORT) {
                 if constexpr (!L::COMBINE) {
                     // four adds per key, straight from the groups: cheapest when `out` is local
