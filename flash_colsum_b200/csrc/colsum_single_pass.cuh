@@ -429,7 +429,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 float L = 0.f;
 #pragma unroll
                 for (int r = 0; r < MAX_CL; ++r) L = fmaf(o[r].y, ex2_approx(o[r].x - M), L);
-                const float base = M > -FLT_MAX ? W_SCALE_LOG2 - M - __log2f(L) : nanf("");   // (a row without a key left)
+                const float base = !PADDED || M > -FLT_MAX ? W_SCALE_LOG2 - M - __log2f(L) : nanf("");
                 const bool live = t * 128 + row < p.Sq;   // rows past the end of the query axis weigh nothing
                 // columns 2a (hi), 2a + 1 (lo) of half hf's operand belong to group 2*hf + a
                 const uint32_t w_row = w_smem + (row >> 4) * 512 + (row & 15) * 2;
@@ -572,8 +572,15 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 uint32_t h[32];
                 float m_g = -INFINITY, l_g = 0.f;
                 if constexpr (KEYS) {
-                    m_g = max3(max_of_32(sa) * c, max_of_32(sb) * c, -FLT_MAX);   // (nothing but -inf -- masked keys -- has exps of zero)
-                    const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_g, -m_g);
+                    // A group of nothing but -inf (masked keys) has exps of zero and no part in its row; a row of such
+                    // groups is NaN.  The maximum that is passed on is -inf then, and the exchange comes to NaN by
+                    // -inf - -inf; in the padded instance it is the floor itself, and the exchange asks for it.  (us per
+                    // call, 32 x 16 pairs: 1024 keys 229.6 in this form, 237.5 in the padded instance's; 577 keys 113.1
+                    // in the other's, 112.0 in this one; 400 60.9 / 60.1.)
+                    m_g = PADDED ? max3(max_of_32(sa) * c, max_of_32(sb) * c, -FLT_MAX)
+                                 : max_or_nan(max_of_32(sa), max_of_32(sb)) * c;
+                    const float m_safe = PADDED ? m_g : max_or_nan(m_g, -FLT_MAX);
+                    const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_safe, -m_safe);
                     f32x2 sum0 = pack2(0.f, 0.f), sum1 = sum0;
 #pragma unroll
                     for (int j8 = 0; j8 < 4; ++j8) exp8_packed<POLY>(j8 * 4, &sa[8 * j8], c2, nm2, sum0, sum1, &h[4 * j8]);
@@ -594,7 +601,8 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 mbar_arrive(stats_bar(slot));
                 const uint32_t line = p_smem + slot * P_BYTES + p_line;
                 if constexpr (KEYS) {
-                    if (t * 128 + row >= p.Sq) {   // past the query axis: weighs zero, but zero times a masked key is NaN
+                    if (m_g != m_g) {   // (a NaN row: one past the query axis -- zero times a masked key -- weighs zero,
+                                        // and adds nothing then; any other is NaN by its weights)
 #pragma unroll
                         for (int j = 0; j < 32; ++j) h[j] = 0u;
                     }

@@ -164,7 +164,10 @@ FCS_HD inline void colsum_full_range(const Problem& p, int kt, int& lo, int& hi)
 // 2000 and 128 heads, 1.5 at 4000 x 4000 and 16.  Longest first over all heads brings that to 1.06 / 1.29 --
 // over as many heads at a time as have their keys in L2 together (every head is read by all SMs at once).
 // us per call, plain / longest first: 4000 x 4000, 16 heads 99 / 93; 6000, 8 heads 122 / 110; 8000, 32 heads
-// 682 / 664 -- but 700 x 700, 256 heads 83 / 89, 1500, 32 heads 42.7 / 43.5, 20000, 32 heads 3745 / 3768.
+// 682 / 664 -- but 700 x 700, 256 heads 83 / 89, 1500, 32 heads 42.7 / 43.5, 20000, 32 heads 3745 / 3768.  The line
+// at 24 query tiles lies inside a range where it gains on both sides (16 tiles: 128 heads 208 / 206, 16 heads
+// 44.3 / 44.2; 20: 16 heads 57 / 53; 23: 32 heads 109 / 107; 25: 16 heads 80 / 68; 32: 16 heads 119 / 114, but 64 heads
+// 328 / 339): it is on the safe side, not where the orders cross.
 struct StatsItems {
     bool done;
     int b, h, qt, sp, s0, s1, grid;   // steps = key blocks s0..s1-1
