@@ -1341,6 +1341,16 @@ static bool single_pass_applies(int B, int H, int Sq, int Sk, int D, int causal)
     return tiles <= 512;
 }
 
+// The instance for clusters of `cl` CTAs.
+typedef void (*SinglePassKernel)(const CUtensorMap, const CUtensorMap, const SinglePassParams);
+template <bool PADDED>
+static SinglePassKernel single_pass_kernel(int cl) {
+    if (cl <= 1) return colsum_single_pass_kernel<PADDED, 1>;
+    if (cl == 2) return colsum_single_pass_kernel<PADDED, 2>;
+    if (cl <= 4) return colsum_single_pass_kernel<PADDED, 4>;
+    return colsum_single_pass_kernel<PADDED, 8>;
+}
+
 // Clusters of `cl` CTAs that can be resident at once (0 if the query fails).
 static int single_pass_max_clusters(int cl) {
     static int cached[64][sp::MAX_CL + 1] = {{0}};
@@ -1348,10 +1358,10 @@ static int single_pass_max_clusters(int cl) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || cl < 1 || cl > sp::MAX_CL) return 0;
     const int idx = cl;
     if (cached[dev][idx] == 0) {
-        // (both instances: the same block, shared memory and registers)
-        if (cudaFuncSetAttribute(colsum_single_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        // (both instances for this size: the same block, shared memory and registers)
+        if (cudaFuncSetAttribute(single_pass_kernel<true>(cl), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  sp::DYN_BYTES) != cudaSuccess ||
-            cudaFuncSetAttribute(colsum_single_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(single_pass_kernel<false>(cl), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  sp::DYN_BYTES) != cudaSuccess)
             return 0;
         cudaLaunchConfig_t cfg;
@@ -1367,7 +1377,7 @@ static int single_pass_max_clusters(int cl) {
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, colsum_single_pass_kernel<false>, &cfg) != cudaSuccess || n <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, single_pass_kernel<false>(cl), &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
             return 0;
         }
@@ -1405,11 +1415,11 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
     sp_.status = status;
     sp_.fmt = fmt_word;
     const uint32_t fmt = dtype == FCS_DTYPE_BF16 ? 1u : 0u;
-    // one score MMA covers the 256 keys of the slice: M = 128, N = 256
+    // a score MMA covers half the 256 keys of the slice: M = 128, N = 128
     sp_.idesc_scores = (1u << 4) | (fmt << 7) | (fmt << 10) | ((scale < 0.f ? 1u : 0u) << 13) |
-                       ((uint32_t)(BLOCK >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
-    // fp16 x fp16 -> fp32, A stored with the M index contiguous, B K-major, M = 128, N = 16
-    sp_.idesc_colsum = (1u << 4) | (1u << 15) | ((uint32_t)(sp::W_N >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+                       ((uint32_t)((BLOCK / 2) >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+    // fp16 x fp16 -> fp32, A and B stored with the M and N index contiguous, M = 128, N = 16
+    sp_.idesc_colsum = (1u << 4) | (1u << 15) | (1u << 16) | ((uint32_t)(sp::W_N >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)(sp_.clusters * sp_.CL));
@@ -1425,7 +1435,7 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = overlap_previous() ? 2 : 1;
-    auto kern = Sk % 64 ? colsum_single_pass_kernel<true> : colsum_single_pass_kernel<false>;
+    const SinglePassKernel kern = Sk % 64 ? single_pass_kernel<true>(sp_.CL) : single_pass_kernel<false>(sp_.CL);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tq, tk, sp_);
     if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "single-pass kernel launch failed: %s", cudaGetErrorString(e));
     return FCS_OK;
