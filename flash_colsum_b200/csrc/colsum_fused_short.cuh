@@ -280,12 +280,15 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             const uint32_t taddr = lane_addr + buf * BLOCK;
             if (ok) {
                 if (kb >= f_lo && kb < f_hi) {
-                    stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
+                    stats_tile_full(taddr, c, m_run, l_run);
                 } else {
-                    const int lim = stats_last_visible(p, 0, kb, row) - col0;
+                    // the columns that some row sees, in four runs of whole 32
+                    int seen = stats_last_visible(p, 0, kb, TILE - 1) + 1;
+                    seen = seen < BLOCK ? seen : BLOCK;
+                    const int cols = ((seen + 127) >> 7) << 5, first = wg * cols;
+                    const int lim = stats_last_visible(p, 0, kb, row) - first;
                     const int lim_first = __shfl_sync(0xffffffffu, lim, 0), lim_last = __shfl_sync(0xffffffffu, lim, 31);
-                    if (lim_first >= GROUP_COLS - 1) stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
-                    else if (lim_last >= 0) stats_tile<true>(taddr, lim, c, m_run, l_run);
+                    stats_tile(taddr - col0 + first, cols, lim, lim_first, lim_last, c, m_run, l_run);
                 }
             }
             tc_fence_before();
@@ -357,8 +360,8 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             if (ok && end > 0 && thr_first_row < GROUP_COLS) {
                 const bool whole = end >= GROUP_COLS && thr_last_row <= 0;
                 if (fp.use_ext) {
-                    if (whole) colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
-                    else colsum_tile_ext<true>(taddr, thr, end, c, acc);
+                    if (whole) colsum_tile_ext_full(taddr, c, acc);
+                    else colsum_tile_ext(taddr, GROUP_COLS, thr, thr_first_row, thr_last_row, end, c, acc);
                 } else {
                     if (whole) colsum_tile<false>(taddr, nl, 0, GROUP_COLS, c, acc);
                     else colsum_tile<true>(taddr, nl, thr, end, c, acc);

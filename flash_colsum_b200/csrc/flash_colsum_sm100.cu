@@ -102,7 +102,8 @@ struct Layout {
     //           l_full[NUM_LSE] l_empty[NUM_LSE]
     static constexpr int NUM_BARS = 2 * NA + 2 * NS + 2 * NUM_TBUF + MERGE_SLOTS + 2 * NUM_LSE;
     static constexpr int MISC_OFF = BAR_OFF + NUM_BARS * 8;        // tmem address, abort flag
-    static constexpr int MERGE_OFF = (MISC_OFF + 16 + 15) / 16 * 16;  // float2[MERGE_SLOTS][groups][128]
+    static constexpr int META_OFF = (MISC_OFF + 16 + 15) / 16 * 16;   // int4[MERGE_SLOTS]: (b, h, query tile, key range) of an item
+    static constexpr int MERGE_OFF = META_OFF + (MODE == MODE_STATS ? MERGE_SLOTS * 16 : 0);  // float2[MERGE_SLOTS][groups][128]
     // (short column modes: float[MERGE_SLOTS][groups][128], the groups' sums of an item before the one add)
     static constexpr int PROB_OFF = MERGE_OFF + (MODE == MODE_STATS ? MERGE_SLOTS * CONSUMER_GROUPS * TILE * 8
                                                                     : COMBINE ? MERGE_SLOTS * CONSUMER_GROUPS * TILE * 4 : 0);
@@ -113,44 +114,63 @@ struct Layout {
     static_assert(DYN_BYTES <= 227 * 1024, "shared memory budget");
 };
 
-// A group's 64 columns of one accumulator.  `taddr`, `lim`, `thr`, `end` and
-// `nl` are relative to the group's first column.
-template <bool MASKED>
-__device__ __forceinline__ void stats_tile(uint32_t taddr, int lim, float c, float& m, float& l) {
+// A group's 64 columns of one accumulator, all of them visible: `taddr` and `nl` are relative to its first column.
+__device__ __forceinline__ void stats_tile_full(uint32_t taddr, float c, float& m, float& l) {
     uint32_t r[32];
     tmem_ld_x32(taddr, r);
     tmem_ld_wait(r);
-    stats_block32<MASKED>(r, lim, c, m, l);
+    stats_block32<false>(r, 32, c, m, l);
     tmem_ld_x32(taddr + 32, r);
     tmem_ld_wait(r);
-    stats_block32<MASKED>(r, lim - 32, c, m, l);
+    stats_block32<false>(r, 32, c, m, l);
 }
-template <bool MASKED>
-__device__ __forceinline__ void colsum_tile_ext(uint32_t taddr, int thr, int end, float c, float (&acc)[4]) {
-    if constexpr (!MASKED) {
-        // 16 columns at a time, the next 16 in flight from tensor memory while these are in the exp pipes
-        uint32_t ra[16], rb[16];
-        tmem_ld_16cols(taddr, ra);
-        tmem_wait_16cols(ra);
-        tmem_ld_16cols(taddr + 16, rb);
-        colsum_chunk16_ext<0>(ra, c, acc);
-        tmem_wait_16cols(rb);
-        tmem_ld_16cols(taddr + 32, ra);
-        colsum_chunk16_ext<8>(rb, c, acc);
-        tmem_wait_16cols(ra);
-        tmem_ld_16cols(taddr + 48, rb);
-        colsum_chunk16_ext<0>(ra, c, acc);
-        tmem_wait_16cols(rb);
-        colsum_chunk16_ext<8>(rb, c, acc);
-        return;
+__device__ __forceinline__ void colsum_tile_ext_full(uint32_t taddr, float c, float (&acc)[4]) {
+    // 16 columns at a time, the next 16 in flight from tensor memory while these are in the exp pipes
+    uint32_t ra[16], rb[16];
+    tmem_ld_16cols(taddr, ra);
+    tmem_wait_16cols(ra);
+    tmem_ld_16cols(taddr + 16, rb);
+    colsum_chunk16_ext<0>(ra, c, acc);
+    tmem_wait_16cols(rb);
+    tmem_ld_16cols(taddr + 32, ra);
+    colsum_chunk16_ext<8>(rb, c, acc);
+    tmem_wait_16cols(ra);
+    tmem_ld_16cols(taddr + 48, rb);
+    colsum_chunk16_ext<0>(ra, c, acc);
+    tmem_wait_16cols(rb);
+    colsum_chunk16_ext<8>(rb, c, acc);
+}
+// The same where some elements are hidden, in runs of 32 columns: what no row of the warp sees is not read, what all
+// rows see takes the arithmetic above, and only the runs that the diagonal or the ragged end goes through are masked;
+// the four groups share what is visible (2000 x 2000 causal, 128 heads of 128 columns, passes apart: statistics 117 ->
+// 114 us, columns 119 -> 105; back to back 240.9 -> 229.2 us a call.  Before, a group masked its fixed quarter as a whole).
+//
+// Statistics: columns 0 .. lim of this row are visible; lim_first / lim_last: the same of the warp's first and
+// last row (the least and the most any of its rows sees).
+__device__ __forceinline__ void stats_tile(uint32_t taddr, int cols, int lim, int lim_first, int lim_last, float c, float& m,
+                                           float& l) {
+    if (lim_last < cols - 1) cols = lim_last + 1;
+#pragma unroll 1
+    for (int j = 0; j < cols; j += 32) {
+        uint32_t r[32];
+        tmem_ld_x32(taddr + j, r);
+        tmem_ld_wait(r);
+        if (lim_first >= j + 31) stats_block32<false>(r, 32, c, m, l);
+        else stats_block32<true>(r, lim - j, c, m, l);
     }
-    uint32_t r[32];
-    tmem_ld_x32(taddr, r);
-    tmem_ld_wait(r);
-    colsum_chunk_ext<MASKED>(r, thr, end, c, acc);
-    tmem_ld_x32(taddr + 32, r);
-    tmem_ld_wait(r);
-    colsum_chunk_ext<MASKED>(r, thr - 32, end - 32, c, acc);
+}
+// Columns thr <= j < end of this row are visible; thr_first / thr_last: thr of the warp's first and last row.
+__device__ __forceinline__ void colsum_tile_ext(uint32_t taddr, int cols, int thr, int thr_first, int thr_last, int end, float c,
+                                                float (&acc)[4]) {
+    if (end < cols) cols = end;
+#pragma unroll 1
+    for (int j = thr_first > 0 ? thr_first & ~31 : 0; j < cols; j += 32) {
+        uint32_t r[32];
+        tmem_ld_x32(taddr + j, r);
+        tmem_ld_wait(r);
+        if (thr_last <= j && j + 32 <= end) colsum_chunk_ext<false>(r, 0, 32, c, acc);
+        else colsum_chunk_ext<true>(r, thr - j, end - j, c, acc);
+    }
 }
 template <bool MASKED>
 __device__ __forceinline__ void colsum_tile(uint32_t taddr, const float4* nl, int thr, int end, float c,
@@ -548,15 +568,17 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         float acc[4] = {0.f, 0.f, 0.f, 0.f};       // column pass state
         int item_cnt = 0, n = 0;
         // statistics pass: the item whose partials this group still has to combine
-        bool pending = false;
-        int pend_cnt = 0, pend_b = 0, pend_h = 0, pend_qt = 0, pend_sp = 0;
+        // (its count; which item that is waits in shared memory, not in four registers)
+        int pend_cnt = -1;
+        int4* meta = reinterpret_cast<int4*>(smem + L::META_OFF);
         auto finish_item = [&]() -> bool {
             const int slot = pend_cnt & (MERGE_SLOTS - 1);
             bool good = mbar_wait(merge_bar(slot), (pend_cnt / MERGE_SLOTS) & 1, abort_flag, p.status,
                                   FCS_STATUS_WAIT_CONSUMER);
             good = __all_sync(0xffffffffu, good);
-            pending = false;
+            pend_cnt = -1;
             if (!good) return false;
+            const int4 item = meta[slot];
             const float2* mb = merge_buf + slot * CONSUMER_GROUPS * TILE;
             float mm = -INFINITY;
 #pragma unroll
@@ -568,8 +590,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 const float2 o = mb[g * TILE + row];
                 ll += o.y * exp2f(o.x - ms);
             }
-            const long long bh = (long long)pend_b * p.H + pend_h;
-            const int q_abs = pend_qt * TILE + row;
+            const long long bh = (long long)item.x * p.H + item.y;
+            const int q_abs = item.z * TILE + row;
             if (p.nsplit == 1) {
                 const float nlv = (q_abs < p.Sq) ? negative_lse(mm, ll, p.log2_norm) : -INFINITY;
                 p.neg_lse[bh * p.lse_rows + q_abs] = nlv;
@@ -580,7 +602,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 er[1] = e1;
             } else {
                 const long long rows = (long long)p.NQ * TILE;
-                reinterpret_cast<float2*>(p.part)[((long long)pend_sp * p.B * p.H + bh) * rows + q_abs] =
+                reinterpret_cast<float2*>(p.part)[((long long)item.w * p.B * p.H + bh) * rows + q_abs] =
                     make_float2(mm, ll);
             }
             return true;
@@ -627,68 +649,46 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 const bool full = (st >= f_lo) && (st < f_hi);
                 if constexpr (MODE == MODE_STATS) {
                     if (full) {
-                        stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
+                        stats_tile_full(taddr, c, m_run, l_run);
                     } else {
-                        // what the rows of this warp see of the group's columns: everything, nothing, or some
-                        const int lim = stats_last_visible(p, it.qt, st, row) - col0;
+                        // the columns that some row of the tile sees, in four runs of whole 32
+                        int seen = stats_last_visible(p, it.qt, st, TILE - 1) + 1;
+                        seen = seen < BLOCK ? seen : BLOCK;
+                        const int cols = ((seen + 127) >> 7) << 5, first = wg * cols;
+                        const int lim = stats_last_visible(p, it.qt, st, row) - first;
                         const int lim_first = __shfl_sync(0xffffffffu, lim, 0), lim_last = __shfl_sync(0xffffffffu, lim, 31);
-                        if (lim_first >= GROUP_COLS - 1) stats_tile<false>(taddr, GROUP_COLS, c, m_run, l_run);
-                        else if (lim_last >= 0) stats_tile<true>(taddr, lim, c, m_run, l_run);
+                        stats_tile(taddr - col0 + first, cols, lim, lim_first, lim_last, c, m_run, l_run);
                     }
                 } else if constexpr (EXT) {
                     // the accumulator already holds s - lse/c
                     if (full) {
-                        colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
+                        colsum_tile_ext_full(taddr, c, acc);
                     } else {
-                        bool done_short = false;
-                        if constexpr (L::SHORT) {
-                            if (p.col_pack == 2) {
-                                // two key tiles in this accumulator buffer, 128 query columns each: groups
-                                // 0, 1 take the halves of the first tile's columns, groups 2, 3 the second's
-                                done_short = true;
-                                const int tg = wg >> 1;
-                                if (tg < it.nt) {
-                                    const int ktg = it.kt + tg;
-                                    const int q0 = (wg & 1) * GROUP_COLS;
-                                    const int end = colsum_end_visible(p, st) - q0;
-                                    const int thr = colsum_first_visible(p, ktg, st, row) - q0;
-                                    const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
-                                    const int thr_last_row = __shfl_sync(0xffffffffu, thr, 31);
-                                    if (end > 0 && thr_first_row < GROUP_COLS) {
-                                        if (end >= GROUP_COLS && thr_last_row <= 0)
-                                            colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
-                                        else
-                                            colsum_tile_ext<true>(taddr, thr, end, c, acc);
-                                    }
-                                }
-                            } else if (colsum_end_visible(p, st) <= BLOCK / 2) {
-                                // at most 128 query columns, one key tile per item: the four groups take
-                                // 32 columns each, not two of them 64
-                                done_short = true;
-                                const int c0 = wg * (GROUP_COLS / 2);
-                                const int end = colsum_end_visible(p, st) - c0;
-                                const int thr = colsum_first_visible(p, it.kt, st, row) - c0;
-                                const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
-                                const int thr_last_row = __shfl_sync(0xffffffffu, thr, 31);
-                                if (end > 0 && thr_first_row < GROUP_COLS / 2) {
-                                    uint32_t r[32];
-                                    tmem_ld_x32(taddr - col0 + c0, r);
-                                    tmem_ld_wait(r);
-                                    if (end >= GROUP_COLS / 2 && thr_last_row <= 0) colsum_chunk_ext<false>(r, 0, 32, c, acc);
-                                    else colsum_chunk_ext<true>(r, thr, end, c, acc);
-                                }
-                            }
+                        // the columns that some row of the tile sees, in four runs of whole 32 -- or two key tiles
+                        // in this accumulator buffer, 128 query columns each: groups 0, 1 take the halves of the
+                        // first tile's columns, groups 2, 3 the second's
+                        const bool packed = L::SHORT && p.col_pack == 2;
+                        int kt = it.kt, q0, cols = GROUP_COLS, base = 0;
+                        bool any = true;
+                        if (packed) {
+                            const int tg = wg >> 1;
+                            if constexpr (L::SHORT) any = tg < it.nt;
+                            kt += tg;
+                            q0 = (wg & 1) * GROUP_COLS;
+                            base = tg * (BLOCK / 2);
+                        } else {
+                            const int from = colsum_first_visible(p, kt, st, 0) & ~31;
+                            cols = ((colsum_end_visible(p, st) - from + 127) >> 7) << 5;
+                            q0 = from + wg * cols;
                         }
-                        if (!done_short) {
-                            const int thr = colsum_first_visible(p, it.kt, st, row) - col0;
-                            const int end = colsum_end_visible(p, st) - col0;
+                        if (any) {
+                            const int end = colsum_end_visible(p, st) - q0;
+                            const int thr = colsum_first_visible(p, kt, st, row) - q0;
                             // what the block's queries see of this warp's keys: nothing, everything, or some
-                            const int thr_first_row = __shfl_sync(0xffffffffu, thr, 0);
-                            const int thr_last_row = __shfl_sync(0xffffffffu, thr, 31);
-                            if (end > 0 && thr_first_row < GROUP_COLS) {
-                                if (end >= GROUP_COLS && thr_last_row <= 0) colsum_tile_ext<false>(taddr, 0, GROUP_COLS, c, acc);
-                                else colsum_tile_ext<true>(taddr, thr, end, c, acc);
-                            }
+                            const int thr_first = __shfl_sync(0xffffffffu, thr, 0), thr_last = __shfl_sync(0xffffffffu, thr, 31);
+                            const uint32_t at = taddr - col0 + base + q0;
+                            if (cols == GROUP_COLS && end >= GROUP_COLS && thr_last <= 0) colsum_tile_ext_full(at, c, acc);
+                            else colsum_tile_ext(at, cols, thr, thr_first, thr_last, end, c, acc);
                         }
                     }
                 } else {
@@ -711,7 +711,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 tc_fence_before();
                 mbar_arrive(t_empty(buf));
                 if constexpr (MODE == MODE_STATS) {
-                    if (pending) { ok = finish_item(); if (!ok) break; }
+                    if (pend_cnt >= 0) { ok = finish_item(); if (!ok) break; }
                 }
                 if constexpr (L::COMBINE) {
                     if (cpend) { ok = finish_cols(); if (!ok) break; }
@@ -722,14 +722,14 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 // post this group's partial (max, sum); one group, a different one every
                 // item, combines the four partials after its next step, when the others
                 // have long since posted -- nobody stands waiting at the end of an item
-                if (pending) { ok = finish_item(); if (!ok) break; }
+                if (pend_cnt >= 0) { ok = finish_item(); if (!ok) break; }
                 const int slot = item_cnt & (MERGE_SLOTS - 1);
                 merge_buf[(slot * CONSUMER_GROUPS + wg) * TILE + row] = make_float2(m_run, l_run);
-                mbar_arrive(merge_bar(slot));
                 if ((item_cnt % CONSUMER_GROUPS) == wg) {
-                    pending = true;
-                    pend_cnt = item_cnt; pend_b = it.b; pend_h = it.h; pend_qt = it.qt; pend_sp = it.sp;
+                    pend_cnt = item_cnt;
+                    if (row == 0) meta[slot] = make_int4(it.b, it.h, it.qt, it.sp);
                 }
+                mbar_arrive(merge_bar(slot));
                 m_run = ROW_MAX_START; l_run = 0.f;
             } else if constexpr (L::SHORT) {
                 if constexpr (!L::COMBINE) {
@@ -763,7 +763,7 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             }
         }
         if constexpr (MODE == MODE_STATS) {
-            if (ok && pending) finish_item();
+            if (ok && pend_cnt >= 0) finish_item();
         }
         if constexpr (L::COMBINE) {
             if (ok && cpend) finish_cols();
