@@ -1564,8 +1564,10 @@ static int launch_fused_short(const CUtensorMap& tq, const CUtensorMap& tk, cons
     return FCS_OK;
 }
 
-// fp32 operands rounded into `q16` / `k16` (dense [B][H][rows][D]); `fmt` receives the type.
-static int launch_round_fp32(const float* q, const float* k, void* q16, void* k16, int* notes, int n_notes, int* fmt, int B,
+// fp32 operands rounded into `q16` / `k16` (dense [B][H][rows][D]); `fmt` receives the type.  `out` (or NULL): B rows
+// of Sk values, out_ld apart, that are zeroed alongside.
+static int launch_round_fp32(const float* q, const float* k, void* q16, void* k16, int* notes, int n_notes, int* fmt, float* out,
+                             int64_t out_ld, int B,
                              int H, int Sq, int Sk, int D, int64_t qsb, int64_t qsh, int64_t qss, int64_t ksb, int64_t ksh,
                              int64_t kss, cudaStream_t stream) {
     rnd::Params rp;
@@ -1586,18 +1588,43 @@ static int launch_round_fp32(const float* q, const float* k, void* q16, void* k1
     rp.notes = notes;
     rp.n_notes = n_notes;
     rp.fmt = fmt;
+    rp.out = out;
+    rp.out_ld = out_ld;
+    rp.out_rows = (unsigned)B;
+    rp.out_cols = (unsigned)Sk;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)n_notes);
-    cfg.blockDim = dim3(rnd::THREADS);
     cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = overlap_previous() ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, rnd::round_kernel, rp);
-    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, rnd::settle_kernel, rp);
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = rnd::SMALL_CTAS;
+    attrs[1].val.clusterDim.y = 1;
+    attrs[1].val.clusterDim.z = 1;
+    cudaError_t e;
+    if ((long long)rp.op[0].pieces + rp.op[1].pieces <= rnd::SMALL_PIECES) {
+        static bool configured[64] = {false};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 0 && dev < 64 && !configured[dev]) {
+            e = cudaFuncSetAttribute(rnd::round_small_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "rounding fp32 operands failed: %s", cudaGetErrorString(e));
+            configured[dev] = true;
+        }
+        cfg.gridDim = dim3(rnd::SMALL_CTAS);
+        cfg.blockDim = dim3(rnd::SMALL_THREADS);
+        cfg.attrs = overlap_previous() ? attrs : attrs + 1;
+        cfg.numAttrs = overlap_previous() ? 2 : 1;
+        e = cudaLaunchKernelEx(&cfg, rnd::round_small_kernel, rp);
+    } else {
+        cfg.gridDim = dim3((unsigned)n_notes);
+        cfg.blockDim = dim3(rnd::THREADS);
+        cfg.attrs = attrs;
+        cfg.numAttrs = overlap_previous() ? 1 : 0;
+        e = cudaLaunchKernelEx(&cfg, rnd::round_kernel, rp);
+        if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, rnd::settle_kernel, rp);
+    }
     if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "rounding fp32 operands failed: %s", cudaGetErrorString(e));
     return FCS_OK;
 }
@@ -1676,6 +1703,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
         return rc;
     }
     const int* fmt_word = nullptr;
+    bool to_clear = clear_out;     // the output still has to be zeroed
     if (dtype == FCS_DTYPE_FP32) {
         // one allocation: the type, the notes, both operands
         const long long pieces = (long long)B * H * ((long long)Sq + Sk) * (D / 8);
@@ -1687,8 +1715,10 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
         if (!ws) return fail(FCS_ERR_WORKSPACE, "no scratch memory for the rounded fp32 operands");
         int* words = reinterpret_cast<int*>(ws);
         rc = launch_round_fp32(static_cast<const float*>(q), static_cast<const float*>(k), ws + head, ws + head + q_bytes,
-                               words + 1, (int)notes, words, B, H, Sq, Sk, D, qsb, qsh, qss, ksb, ksh, kss, stream);
+                               words + 1, (int)notes, words, passes == PASSES_BOTH && clear_out ? out : nullptr, out_ld, B, H, Sq,
+                               Sk, D, qsb, qsh, qss, ksb, ksh, kss, stream);
         if (rc != FCS_OK) return rc;
+        to_clear = false;
         q = ws + head;
         k = ws + head + q_bytes;
         qss = kss = D;
@@ -1726,7 +1756,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
     p.fmt = fmt_word;
     p.out = out;
     p.out_ld = out_ld;
-    p.clear_out = (clear_out && passes == PASSES_BOTH) ? 1 : 0;   // (the statistics pass does the clearing)
+    p.clear_out = (to_clear && passes == PASSES_BOTH) ? 1 : 0;   // (the statistics pass does the clearing)
     p.col_combine = clear_out ? 0 : 1;   // accumulating into a caller's buffer: it may be peer-mapped
     p.clear_extra = clear_extra_n > 0 ? clear_extra : nullptr;
     p.clear_extra_n = clear_extra_n;
@@ -1759,7 +1789,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
                 tms->recorded = false;
                 for (int i = 0; i < 3; ++i) cudaEventRecord(tms->ev[i], stream);
             }
-            rc = launch_single_pass(tq_a, tk_b, out, out_ld, B, H, Sq, Sk, scale, h_norm, dtype, clear_out,
+            rc = launch_single_pass(tq_a, tk_b, out, out_ld, B, H, Sq, Sk, scale, h_norm, dtype, to_clear,
                                     max_clusters, status, fmt_word, stream);
             if (rc == FCS_OK && tms) { cudaEventRecord(tms->ev[3], stream); tms->recorded = true; }
             return rc;
@@ -1773,7 +1803,7 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
                 tms->recorded = false;
                 for (int i = 0; i < 3; ++i) cudaEventRecord(tms->ev[i], stream);
             }
-            rc = launch_fused_short(tq_a, tk_b, p, DK, scale, use_ext, fcl, fnkb, fbpc, clear_out, clear_extra,
+            rc = launch_fused_short(tq_a, tk_b, p, DK, scale, use_ext, fcl, fnkb, fbpc, to_clear, clear_extra,
                                     clear_extra_n, stream);
             if (rc == FCS_OK && tms) { cudaEventRecord(tms->ev[3], stream); tms->recorded = true; }
             return rc;

@@ -9,17 +9,25 @@
 // and the kernels behind them take the element type from `fmt` (Problem::fmt).  Bound by memory: 6
 // bytes per element.  (An abs / max / read-back per operand and two conversions by torch
 // operators took 85 us for a call of a megabyte.)
+//
+// Operands of up to SMALL_PIECES pieces are over before a launch is: there both steps are one kernel on one
+// cluster of sixteen CTAs, which ask each other through shared memory instead of notes.  Either way the output of
+// the call is zeroed on the side, which is a launch less for the kernels that add into it (2 x 4 x 256 x 64, a
+// megabyte, back to back: four launches 11.45 us, two 10.24).
 #pragma once
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "colsum_small_q.cuh"
 #include "sm100_ptx.cuh"
 
 namespace fcs {
 namespace rnd {
 
 constexpr int THREADS = 256;
+constexpr int SMALL_CTAS = 16, SMALL_THREADS = 512;
+constexpr long long SMALL_PIECES = 65536;
 constexpr float FP16_LIMIT = 60000.f;
 
 struct Operand {
@@ -35,7 +43,19 @@ struct Params {
     int* notes;                    // one per CTA of round_kernel
     int n_notes;
     int* fmt;
+    float* out;                    // zeroed: `out_rows` rows of `out_cols`, out_ld apart (NULL: nothing)
+    long long out_ld;
+    unsigned out_rows, out_cols;
 };
+
+__device__ __forceinline__ void clear_output(const Params& p, unsigned thread, unsigned threads) {
+    if (!p.out) return;
+    const unsigned long long n = (unsigned long long)p.out_rows * p.out_cols;
+    for (unsigned long long i = thread; i < n; i += threads) {
+        const unsigned long long r = n <= 0xffffffffull ? (unsigned)i / p.out_cols : i / p.out_cols;
+        p.out[(long long)r * p.out_ld + (long long)(i - r * p.out_cols)] = 0.f;
+    }
+}
 
 __device__ __forceinline__ const float* piece_source(const Operand& o, unsigned i) {
     if (o.dense) return o.src + (size_t)i * 8;
@@ -43,6 +63,23 @@ __device__ __forceinline__ const float* piece_source(const Operand& o, unsigned 
     const unsigned unit = row / o.rows, r = row - unit * o.rows;
     const unsigned b = unit / o.H, h = unit - b * o.H;
     return o.src + (long long)b * o.sb + (long long)h * o.sh + (long long)r * o.ss + e * 8;
+}
+
+// Piece `i` (a, b) as fp16; whether a value of it does not fit.
+__device__ __forceinline__ bool to_fp16(const Operand& o, unsigned i, const float4& a, const float4& b) {
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
+                          fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
+    __half2 h[4] = {__floats2half2_rn(a.x, a.y), __floats2half2_rn(a.z, a.w), __floats2half2_rn(b.x, b.y),
+                    __floats2half2_rn(b.z, b.w)};
+    *reinterpret_cast<uint4*>(o.dst + (size_t)i * 8) = *reinterpret_cast<const uint4*>(h);
+    return m >= FP16_LIMIT;
+}
+__device__ __forceinline__ void to_bf16(const Operand& o, unsigned i) {
+    const float4* s = reinterpret_cast<const float4*>(piece_source(o, i));
+    const float4 a = s[0], b = s[1];
+    __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w),
+                           __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
+    *reinterpret_cast<uint4*>(o.dst + (size_t)i * 8) = *reinterpret_cast<const uint4*>(h);
 }
 
 __global__ void __launch_bounds__(THREADS)
@@ -56,14 +93,10 @@ round_kernel(const Params p) {
         for (unsigned i = blockIdx.x * THREADS + threadIdx.x; i < o.pieces; i += gridDim.x * THREADS) {
             const float4* s = reinterpret_cast<const float4*>(piece_source(o, i));
             const float4 a = s[0], b = s[1];
-            const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
-                                  fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
-            outside = outside || m >= FP16_LIMIT;
-            __half2 h[4] = {__floats2half2_rn(a.x, a.y), __floats2half2_rn(a.z, a.w), __floats2half2_rn(b.x, b.y),
-                            __floats2half2_rn(b.z, b.w)};
-            *reinterpret_cast<uint4*>(o.dst + (size_t)i * 8) = *reinterpret_cast<const uint4*>(h);
+            outside = to_fp16(o, i, a, b) || outside;
         }
     }
+    clear_output(p, blockIdx.x * THREADS + threadIdx.x, gridDim.x * THREADS);
     const int any = __syncthreads_or(outside ? 1 : 0);
     if (threadIdx.x == 0) p.notes[blockIdx.x] = any;
 }
@@ -80,13 +113,57 @@ settle_kernel(const Params p) {
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         const Operand& o = p.op[t];
-        for (unsigned i = blockIdx.x * THREADS + threadIdx.x; i < o.pieces; i += gridDim.x * THREADS) {
-            const float4* s = reinterpret_cast<const float4*>(piece_source(o, i));
-            const float4 a = s[0], b = s[1];
-            __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w),
-                                   __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
-            *reinterpret_cast<uint4*>(o.dst + (size_t)i * 8) = *reinterpret_cast<const uint4*>(h);
+        for (unsigned i = blockIdx.x * THREADS + threadIdx.x; i < o.pieces; i += gridDim.x * THREADS) to_bf16(o, i);
+    }
+}
+
+// Both steps on one cluster of SMALL_CTAS CTAs.
+__global__ void __launch_bounds__(SMALL_THREADS)
+round_small_kernel(const Params p) {
+    __shared__ uint32_t notes[SMALL_CTAS];
+    grid_launch_dependents();
+    smallq_cluster_arrive();
+    grid_dependency_wait();
+    const unsigned thread = blockIdx.x * SMALL_THREADS + threadIdx.x, threads = SMALL_CTAS * SMALL_THREADS;
+    const unsigned first = p.op[0].pieces, all_pieces = first + p.op[1].pieces;
+    bool outside = false;
+    for (unsigned i0 = thread; i0 < all_pieces; i0 += 4 * threads) {     // four pieces of either operand in flight
+        float4 a[4], b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const unsigned i = i0 + j * threads;
+            if (i >= all_pieces) break;
+            const float4* s = reinterpret_cast<const float4*>(i < first ? piece_source(p.op[0], i) : piece_source(p.op[1], i - first));
+            a[j] = s[0];
+            b[j] = s[1];
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const unsigned i = i0 + j * threads;
+            if (i >= all_pieces) break;
+            outside = (i < first ? to_fp16(p.op[0], i, a[j], b[j]) : to_fp16(p.op[1], i - first, a[j], b[j])) || outside;
+        }
+    }
+    clear_output(p, thread, threads);
+    const int any = __syncthreads_or(outside ? 1 : 0);
+    smallq_cluster_wait();       // (the other CTAs run)
+    if (threadIdx.x < SMALL_CTAS) {
+        uint32_t addr;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&notes[blockIdx.x])), "r"(threadIdx.x));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(any) : "memory");
+    }
+    __syncwarp();
+    smallq_cluster_arrive();
+    smallq_cluster_wait();
+    uint32_t all = 0;
+#pragma unroll
+    for (int r = 0; r < SMALL_CTAS; ++r) all |= notes[r];
+    if (thread == 0) *p.fmt = all ? 1 : 0;
+    if (!all) return;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const Operand& o = p.op[t];
+        for (unsigned i = thread; i < o.pieces; i += threads) to_bf16(o, i);
     }
 }
 
