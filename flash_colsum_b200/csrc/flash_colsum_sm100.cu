@@ -1950,7 +1950,7 @@ template <int NT, int E, int BITS, int CL>
 static cudaError_t launch_topk_t(const float* colsum, long long ld, int B, int S, int k, int* indices, float* values,
                                  cudaStream_t stream) {
     static bool configured[64] = {false};
-    return launch_row_clusters(sel::topk_kernel<NT, E, BITS, CL>, sel::topk_smem<NT, E, BITS>(), configured, B, CL, NT,
+    return launch_row_clusters(sel::topk_kernel<NT, E, BITS, CL>, sel::topk_smem<NT, E, BITS, CL>(), configured, B, CL, NT,
                                stream, colsum, ld, S, k, indices, values);
 }
 static cudaError_t launch_topk(const float* colsum, long long ld, int B, int S, int k, int* indices, float* values,

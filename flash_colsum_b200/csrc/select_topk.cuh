@@ -10,13 +10,16 @@
 //   top-k      exact radix selection, 11 bits at a time from the top (8 for rows of at most
 //              1024, where scanning 2048 bins costs more than a fourth pass): every CTA
 //              counts its elements that still match the prefix chosen so far, sums its bins in
-//              groups of 32, and one warp of every CTA reads the group sums of all CTAs
-//              through distributed shared memory, finds the group and then the bin the k-th
-//              largest falls into -- every CTA for itself, so that a pass has one
-//              cluster barrier.  A bin that is wanted whole ends the selection early.
-//   threshold  (with `relative`: against a share of the row's average) a comparison per element.
-//   both       one scan over the block of the kept elements per thread, the counts of the CTAs
-//              exchanged once, and every kept element knows its place in the output.
+//              groups of 32 and stores the group sums into every CTA of the cluster; after the pass's only
+//              cluster barrier one warp of every CTA finds the group the k-th largest falls into,
+//              reads that group's bins of all CTAs through distributed shared memory and finds the
+//              bin -- every CTA for itself.  What it adds up for the CTAs before its own, in
+//              the bins passed over and in the bin chosen, says where its elements go: there is nothing to
+//              exchange at the end.  A bin that is wanted whole ends the selection early.
+//   threshold  (with `relative`: against a share of the row's average) a comparison per element; the counts
+//              of the CTAs are exchanged once.
+//   both       one scan over the block of the kept elements per thread, and every kept element
+//              knows its place in the output.
 //
 // What bounds it: a dozen dependent steps of half a microsecond to one (launch of the cluster,
 // load, cluster barriers, scans), not bytes.  Back to back on a B200, one CTA per row going over
@@ -50,6 +53,11 @@ __device__ __forceinline__ uint32_t ld_peer_u32(uint32_t local_addr, uint32_t ra
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
     return v;
+}
+__device__ __forceinline__ void st_peer_u32(uint32_t local_addr, uint32_t rank, uint32_t v) {
+    uint32_t addr;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 // The sum over the first `n` of the cluster's CL CTAs of the word at `local_addr` in each, all loads in
 // flight at once (a loop over a runtime count waits for each: half a microsecond more per pass).
@@ -136,9 +144,9 @@ template <int BITS>
 struct Digits {
     static constexpr int BINS = 1 << BITS, GROUPS = BINS / 32, PASSES = (32 + BITS - 1) / BITS;
 };
-template <int NT, int E, int BITS>
+template <int NT, int E, int BITS, int CL>
 constexpr int topk_smem() {
-    return stage_bytes<NT, E>() + Digits<BITS>::PASSES * (Digits<BITS>::BINS + Digits<BITS>::GROUPS) * 4;
+    return stage_bytes<NT, E>() + Digits<BITS>::PASSES * (Digits<BITS>::BINS + CL * Digits<BITS>::GROUPS) * 4;
 }
 
 template <int NT, int E, int BITS, int CL>
@@ -150,15 +158,15 @@ topk_kernel(const float* __restrict__ colsum, long long ld, int S, int k, int* _
     extern __shared__ __align__(16) uint32_t sel_smem[];
     uint32_t* stage = sel_smem;
     uint32_t* hist = sel_smem + NT * (E + 1);       // [PASSES][BINS]: a fresh one per pass, cleared once
-    uint32_t* gsum = hist + PASSES * BINS;          // [PASSES][GROUPS]
+    uint32_t* gsum = hist + PASSES * BINS;          // [PASSES][CL][GROUPS]: of every CTA
     __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t totals[2];                  // this CTA's elements before the k-th's bin / in it
-    __shared__ uint32_t choice[3];                  // digit, elements before its bin, elements in it
+    __shared__ uint32_t choice[5];                  // digit, elements before its bin, in it, and both of the CTAs before this
     const uint32_t rank = smallq_cluster_rank();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const long long b = blockIdx.x / CL;
 
     for (int i = threadIdx.x; i < PASSES * BINS; i += NT) hist[i] = 0u;
+    if constexpr (CL > 1) smallq_cluster_arrive();  // (waited for before the first store into a peer)
     grid_dependency_wait();
     grid_launch_dependents();
     Slice<NT, E> sl;
@@ -172,14 +180,16 @@ topk_kernel(const float* __restrict__ colsum, long long ld, int S, int k, int* _
     const bool resident = sl.tiles == 1;
     if (resident) fetch(0);
     else __syncthreads();                           // (the bins are clear)
+    if constexpr (CL > 1) smallq_cluster_wait();
 
     // ---- the k-th smallest key, BITS bits at a time
     uint32_t prefix = 0, mask = 0, need = (uint32_t)k;   // `need`: still to take among the elements matching `prefix`
+    uint32_t lt0 = 0, eq0 = 0;                           // elements of the CTAs before this one: below the prefix, matching it
     for (int pass = 0; pass < PASSES; ++pass) {
         const int shift = 32 - BITS * (pass + 1) > 0 ? 32 - BITS * (pass + 1) : 0;
         const uint32_t digits = pass == PASSES - 1 ? (1u << (32 - BITS * pass)) - 1u : (uint32_t)(BINS - 1);
         uint32_t* h = hist + pass * BINS;
-        uint32_t* gs = gsum + pass * GROUPS;
+        uint32_t* gs = gsum + pass * CL * GROUPS;
         for (int tile = 0; tile < sl.tiles; ++tile) {
             if (!resident) fetch(tile);
             const uint32_t i0 = sl.first(tile);
@@ -191,40 +201,60 @@ topk_kernel(const float* __restrict__ colsum, long long ld, int S, int k, int* _
         for (int g = wid; g < GROUPS; g += NT / 32) {
             uint32_t v = h[g * 32 + lane];
             v = __reduce_add_sync(0xffffffffu, v);
-            if (lane == 0) gs[g] = v;
+            if constexpr (CL > 1) {
+                if (lane < CL) st_peer_u32(smem_u32(gs + rank * GROUPS + g), (uint32_t)lane, v);
+            } else {
+                if (lane == 0) gs[g] = v;
+            }
         }
         if constexpr (CL > 1) cluster_sync(); else __syncthreads();
         if (wid == 0) {
-            uint32_t gv[GPL], sum = 0;
+            uint32_t gv[GPL], gl[GPL], sum = 0, low = 0;    // of all CTAs, and of those before this one
 #pragma unroll
             for (int i = 0; i < GPL; ++i) {
                 const int g = lane * GPL + i;
-                gv[i] = g < GROUPS ? sum_over_cluster<CL>(smem_u32(gs + g)) : 0u;
+                gv[i] = gl[i] = 0u;
+#pragma unroll
+                for (int r = 0; r < CL; ++r) {
+                    const uint32_t x = g < GROUPS ? gs[r * GROUPS + g] : 0u;
+                    gv[i] += x;
+                    gl[i] += (uint32_t)r < rank ? x : 0u;
+                }
                 sum += gv[i];
+                low += gl[i];
             }
             const uint32_t inc = warp_scan(sum, lane);
             const int f = __ffs(__ballot_sync(0xffffffffu, inc >= need)) - 1;
-            uint32_t before = inc - sum;            // (of lane f, below)
+            uint32_t before = inc - sum, low_before = CL > 1 ? warp_scan(low, lane) - low : 0u;    // (of lane f, below)
             int g = lane * GPL;
 #pragma unroll
             for (int i = 0; i + 1 < GPL; ++i)
-                if (before + gv[i] < need && g == lane * GPL + i) { before += gv[i]; ++g; }
+                if (before + gv[i] < need && g == lane * GPL + i) { before += gv[i]; low_before += gl[i]; ++g; }
             g = __shfl_sync(0xffffffffu, g, f);
             before = __shfl_sync(0xffffffffu, before, f);
-            const uint32_t v = sum_over_cluster<CL>(smem_u32(h + g * 32 + lane));
+            low_before = __shfl_sync(0xffffffffu, low_before, f);
+            uint32_t bins[CL], v = 0, lv = 0;
+#pragma unroll
+            for (int r = 0; r < CL; ++r)             // (all loads in flight at once)
+                bins[r] = CL > 1 ? ld_peer_u32(smem_u32(h + g * 32 + lane), (uint32_t)r) : h[g * 32 + lane];
+#pragma unroll
+            for (int r = 0; r < CL; ++r) { v += bins[r]; lv += (uint32_t)r < rank ? bins[r] : 0u; }
             const uint32_t vi = before + warp_scan(v, lane);
+            const uint32_t li = low_before + (CL > 1 ? warp_scan(lv, lane) - lv : 0u);
             const int d = __ffs(__ballot_sync(0xffffffffu, vi >= need)) - 1;
-            if (lane == d) { choice[0] = (uint32_t)(g * 32 + d); choice[1] = vi - v; choice[2] = v; }
+            if (lane == d) { choice[0] = (uint32_t)(g * 32 + d); choice[1] = vi - v; choice[2] = v; choice[3] = li; choice[4] = lv; }
         }
         __syncthreads();
         prefix |= choice[0] << shift;
         mask |= digits << shift;
         need -= choice[1];
+        lt0 += choice[3];
+        eq0 = choice[4];
         const bool whole = choice[2] == need;       // every element of the bin is wanted
         if (whole) break;
     }
 
-    // ---- how many elements of the row precede this CTA's: below the prefix, and matching it
+    // ---- every element's place: the elements of its CTA before it, below the prefix and matching it
     auto counts = [&](int tile) {
         uint32_t c = 0;
         const uint32_t i0 = sl.first(tile);
@@ -235,28 +265,13 @@ topk_kernel(const float* __restrict__ colsum, long long ld, int S, int k, int* _
         }
         return c;
     };
-    uint32_t scan = 0, tile_total = 0, n_lt = 0, n_eq = 0;   // (counts of a tile fit 16 bits each: at most NT * E = 16384)
-    for (int tile = 0; tile < sl.tiles; ++tile) {
-        if (!resident) fetch(tile);
-        scan = block_scan<NT>(counts(tile), warp_sums, tile_total);
-        n_lt += tile_total & 0xffffu;
-        n_eq += tile_total >> 16;
-    }
-    uint32_t lt0 = 0, eq0 = 0;
-    if constexpr (CL > 1) {
-        if (threadIdx.x == 0) { totals[0] = n_lt; totals[1] = n_eq; }
-        cluster_sync();
-        lt0 = sum_over_cluster<CL>(smem_u32(&totals[0]), rank);
-        eq0 = sum_over_cluster<CL>(smem_u32(&totals[1]), rank);
-        smallq_cluster_arrive();                    // nobody leaves before its peers have read its counts
-    }
+    uint32_t scan = 0, tile_total = 0;              // (counts of a tile fit 16 bits each: at most NT * E = 16384)
+    if constexpr (CL > 1) smallq_cluster_arrive();  // nobody leaves before its peers have read its bins
     int* out_idx = indices + b * k;
     float* out_val = values ? values + b * k : nullptr;
     for (int tile = 0; tile < sl.tiles; ++tile) {
-        if (!resident) {
-            fetch(tile);
-            scan = block_scan<NT>(counts(tile), warp_sums, tile_total);
-        }
+        if (!resident) fetch(tile);
+        scan = block_scan<NT>(counts(tile), warp_sums, tile_total);
         uint32_t lt = lt0 + (scan & 0xffffu), eq = eq0 + (scan >> 16);
         const uint32_t i0 = sl.first(tile);
 #pragma unroll
