@@ -103,15 +103,9 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// Asynchronous store of two floats into another CTA's shared memory; its 8 bytes are
+// Asynchronous store of four floats (16-byte aligned) into another CTA's shared memory; its 16 bytes are
 // counted on that CTA's barrier `mbar` when they have landed, so the sender neither
 // waits nor fences.
-__device__ __forceinline__ void st_async_f32x2(uint32_t addr, float a, float b, uint32_t mbar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
-                 ::"r"(addr), "f"(a), "f"(b), "r"(mbar)
-                 : "memory");
-}
-// The same for four floats (16-byte aligned).
 __device__ __forceinline__ void st_async_f32x4(uint32_t addr, float a, float b, float c, float d, uint32_t mbar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
                  ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"(mbar)
@@ -278,7 +272,7 @@ template <bool V> struct Flag { static constexpr bool value = V; };
 // ---------------------------------------------------------------------------
 // PADDED: the key axis ends inside a group of 64 keys.  (An instance of its own: the test for it in the
 // loop costs 4 % at 512 and 1024 keys.)  CLMAX: most CTAs of a cluster (1, 2, 4 or 8): the exchange is unrolled
-// for as many.
+// for as many.  The instance for one CTA has no cluster instruction and is launched without a cluster.
 template <bool PADDED, int CLMAX>
 __global__ void __launch_bounds__(sp::THREADS, 1)
 colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -313,8 +307,8 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_ctarank();
-    const int CL = p.CL;
+    const uint32_t rank = CLMAX > 1 ? cluster_ctarank() : 0u;
+    const int CL = CLMAX > 1 ? p.CL : 1;
     const int cluster_id = blockIdx.x / CL;
     const int NQ = p.NQ;
     // this cluster's share of the (batch, head, query tile) list
@@ -353,10 +347,10 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();   // every CTA's barriers exist before a peer signals them
+    if constexpr (CLMAX > 1) cluster_sync_all();   // every CTA's barriers exist before a peer signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (clusters_pack(p.CL)) grid_launch_dependents();   // (not before this CTA has its tensor memory)
+    if (CLMAX == 1 || clusters_pack(p.CL)) grid_launch_dependents();   // (not before this CTA has its tensor memory)
     grid_dependency_wait();   // the set-up is done; what follows reads the inputs and adds into the cleared output
 
     auto wait_all = [&](uint32_t bar, uint32_t parity, int code) -> bool {
@@ -704,7 +698,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     // ---------------------------------------------------- teardown
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();   // nobody leaves while a peer may still write into its shared memory
+    if constexpr (CLMAX > 1) cluster_sync_all();   // nobody leaves while a peer may still write into its shared memory
     if (warp == COLSUM_WARP) {
         if (*abort_flag) __nanosleep(1000000);   // let copies and MMAs in flight land
         tc_fence_after();

@@ -1364,6 +1364,7 @@ static int single_pass_max_clusters(int cl) {
             cudaFuncSetAttribute(single_pass_kernel<false>(cl), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  sp::DYN_BYTES) != cudaSuccess)
             return 0;
+        if (cl == 1) return cached[dev][idx] = num_sms();    // (no clusters: a CTA fills an SM)
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3((unsigned)(cl * 64));
@@ -1427,14 +1428,14 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
     cfg.dynamicSmemBytes = sp::DYN_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
-    attrs[0].id = cudaLaunchAttributeClusterDimension;
-    attrs[0].val.clusterDim.x = (unsigned)sp_.CL;
-    attrs[0].val.clusterDim.y = 1;
-    attrs[0].val.clusterDim.z = 1;
-    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = overlap_previous() ? 1 : 0;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = (unsigned)sp_.CL;
+    attrs[1].val.clusterDim.y = 1;
+    attrs[1].val.clusterDim.z = 1;
     cfg.attrs = attrs;
-    cfg.numAttrs = overlap_previous() ? 2 : 1;
+    cfg.numAttrs = sp_.CL > 1 ? 2 : 1;      // (the instance for one CTA has no cluster instruction)
     const SinglePassKernel kern = Sk % 64 ? single_pass_kernel<true>(sp_.CL) : single_pass_kernel<false>(sp_.CL);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tq, tk, sp_);
     if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "single-pass kernel launch failed: %s", cudaGetErrorString(e));
