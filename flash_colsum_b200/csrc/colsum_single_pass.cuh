@@ -266,7 +266,7 @@ template <bool V> struct Flag { static constexpr bool value = V; };
 // for the weights of the tile before last, the consumers for the scores -- all groups at once, so that their
 // loads, exps and stores never overlapped -- and the exchange warps were busy for 2 700 of a tile's 3 200 cycles.
 // Apart, with the exchange unrolled for the cluster's size, two rows to a load and a store, and the weights in
-// one 16-byte store per row: us per call, 32 x 16 pairs, back to back, 577 keys 112.4 -> 101.8, 1024 keys 230.4 -> 221.7.
+// one 16-byte store per row: us per call, 32 x 16 pairs, back to back, 577 keys 112.4 -> 100.8, 1024 keys 230.4 -> 211.2.
 // What is left of a tile's 2 900 cycles: 1 400 in the exps, the rest the latencies around them (tensor-memory loads
 // 270, stores 330, barriers and loop 600), and a half that runs ahead waits for the other one's statistics.
 // ---------------------------------------------------------------------------
@@ -421,10 +421,11 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     }
                     __syncwarp();
                     if (++sb == S_BUFS) { sb = 0; sph ^= 1; }
+                    // The next query tile: its buffer is free since scores(i-1), and fetched only behind both halves of
+                    // scores(i) it came 1 100 cycles after them, with an accumulator free (1024 keys 222.6 -> 211.2 us)
+                    if (hf == 0) ok = fetch_query_tile();
                 }
                 if (!ok) break;
-                // (its buffer is the one scores(i-1) were formed from: free by now)
-                if (!fetch_query_tile()) { ok = false; break; }
             }
         }
     } else if (warp >= XCHG_WARP) {
