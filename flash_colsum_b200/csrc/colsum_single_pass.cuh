@@ -266,7 +266,7 @@ template <bool V> struct Flag { static constexpr bool value = V; };
 // for the weights of the tile before last, the consumers for the scores -- all groups at once, so that their
 // loads, exps and stores never overlapped -- and the exchange warps were busy for 2 700 of a tile's 3 200 cycles.
 // Apart, with the exchange unrolled for the cluster's size, two rows to a load and a store, and the weights in
-// one 16-byte store per row: us per call, 32 x 16 pairs, back to back, 577 keys 112.4 -> 100.8, 1024 keys 230.4 -> 211.2.
+// one 16-byte store per row: us per call, 32 x 16 pairs, back to back, 577 keys 112.4 -> 100.9, 1024 keys 230.4 -> 198.5.
 // What is left of a tile's 2 900 cycles: 1 400 in the exps, the rest the latencies around them (tensor-memory loads
 // 270, stores 330, barriers and loop 600), and a half that runs ahead waits for the other one's statistics.
 // ---------------------------------------------------------------------------
@@ -570,10 +570,9 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         // second copy of it for the ragged group does not fit the instruction cache next to the first
         // (385-447 keys: 89 us a call against 62)
         const int padding = keys_valid < 64 ? 64 - keys_valid : 0;
-        // Pairs of 16 on the FMA pipe.  In the padded instance 3 is the fastest throughout, one slice or several, the
-        // last one full or not; us per call with 2 / 3 / 4 / 5: 32 x 16 x 200 keys 25.2 / 24.6 / 24.9 / 25.3, 400 62.0 /
-        // 60.1 / 61.5 / 62.9, 577 114.3 / 112.0 / 114.4 / 117.5, 1000 237.5 / 231.7 / 234.6 / 242.0, 8 x 16 x 1500 139.0 /
-        // 136.2 / 137.3 / 140.2 (only 300: 62.0 / 62.0 / 61.8 / 61.5).  In the other 5: 1024 keys 234.6 with 3, 232.7 with 5.
+        // Pairs of 16 on the FMA pipe, us per call with 2 / 3 / 4 / 5: padded, 32 x 16 x 577 keys 104.0 / 100.9 / 102.4 / 98.4,
+        // 8 x 12 x 900 47.6 / 46.1 / 47.9 / 46.9, 16 x 16 x 1000 110.0 / 106.2 / 109.4 / 106.9, 8 x 16 x 1500 122.0 / 119.5 /
+        // 122.3 / 120.2; in the other instance 32 x 16 x 512 keys 55.5 / 56.1 / 53.2 / 52.1, 1024 214.9 / 215.6 / 205.9 / 198.5.
         constexpr int POLY = PADDED ? 3 : FCS_POLY_PAIRS;
         auto consume = [&](auto keys) {
         constexpr bool KEYS = decltype(keys)::value;     // false: nothing but padding
@@ -627,8 +626,11 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             mbar_arrive(s_empty(sb));
             sb += 2;                                   // (accumulators 2 i + hf, mod 3)
             if (sb >= S_BUFS) { sb -= S_BUFS; sph ^= 1; }
-            // whether tile i-2 is through, asked early: the answer is there when it is needed
-            const bool freed = mbar_test_wait(pw_free(slot, hf), ((i >> 1) & 1) ^ 1);
+            // Whether tile i-2 is through, asked early in the padded instance, so that the answer is there when it is
+            // needed.  (us per call, 32 x 16 pairs, asked early / not: 577 keys 100.9 / 107.8; 512 keys 56.2 / 52.1, 1024
+            // keys 211.4 / 198.5 -- the two instances have their registers differently full, and each has the form
+            // that leaves it the better schedule.)
+            const bool freed = PADDED && mbar_test_wait(pw_free(slot, hf), ((i >> 1) & 1) ^ 1);
 
             // ---- P~ = exp2(c*s - m_g) as packed fp16
             uint32_t h[32];
@@ -655,7 +657,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             }
             // ---- tile i-2 is through: its column-sum MMA has read P~(i-2), and (before that)
             // the exchange warps have read its statistics -- both slots are free
-            if (!__all_sync(0xffffffffu, freed)) {
+            if (!PADDED || !__all_sync(0xffffffffu, freed)) {
                 ok = mbar_wait(pw_free(slot, hf), ((i >> 1) & 1) ^ 1, abort_flag, p.status, FCS_STATUS_WAIT_CONSUMER);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
