@@ -12,9 +12,9 @@
 //                                        byte counts: nobody waits for a store to land)
 //   w_g    = exp2(m_g - M) / L           the factor that turns P~ into softmax probabilities
 //   D2    += P~^T W                      second MMA: contraction over the 128 query rows; W holds
-//                                        w_g as two fp16 parts (hi + lo) in columns of a 16-wide
-//                                        operand, so D2[key][2a], D2[key][2a+1] are the column
-//                                        sums of the keys of 64-key group a of a key tile
+//                                        w_g of the four groups as two fp16 parts (hi in columns
+//                                        0..3, lo in 4..7 of a 16-wide operand), so D2[key][g] and
+//                                        D2[key][4 + g] are the column sums of a key of group g
 //
 // D2 lives in tensor memory across all query tiles and heads of a batch entry and
 // is added to the output once per (cluster, batch entry).  P~ is double-buffered:

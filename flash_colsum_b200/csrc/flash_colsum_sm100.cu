@@ -1333,7 +1333,8 @@ static bool single_pass_applies(int B, int H, int Sq, int Sk, int D, int causal)
     // time goes by whole slices of 256 keys, and up to six of them it wins at any fill from 60 %
     // (one slice: at any length); clusters of 7 and 8 fit only 15 at a time (105 / 120 of 148 SMs) and lose
     // on large calls (2048 keys: 1046/998) but win on small ones (41/50), where the fixed costs of two
-    // launches and partial waves weigh more
+    // launches and partial waves weigh more.  (Both forms as they were when the line was drawn.  This one takes 10 to
+    // 16 % less now -- 1024 keys 230 -> 199 us, 577 112 -> 101 -- and the line stays: past it, exps keep 32 bits.)
     if (cl == 1) return true;
     if (cl <= 6) return (long long)Sk * 100 >= (long long)cl * 256 * 60;
     if ((long long)Sk * 100 < (long long)cl * 256 * 85) return false;
@@ -1957,6 +1958,8 @@ static cudaError_t launch_topk_t(const float* colsum, long long ld, int B, int S
 static cudaError_t launch_topk(const float* colsum, long long ld, int B, int S, int k, int* indices, float* values,
                                cudaStream_t stream) {
     const int cl = sel::cluster_size(S);
+    // (half the elements per CTA while all rows' clusters of sixteen run at once)
+    const bool wide = cl == 8 && S > 8 * 8192 && B <= sel::TOPK_WIDE_ROWS;
 #define FCS_TOPK(NT, E, BITS, CL) return launch_topk_t<NT, E, BITS, CL>(colsum, ld, B, S, k, indices, values, stream)
     if (S <= 1024) FCS_TOPK(256, 4, 8, 1);
     if (cl == 1) FCS_TOPK(1024, 4, 11, 1);
@@ -1964,6 +1967,7 @@ static cudaError_t launch_topk(const float* colsum, long long ld, int B, int S, 
     if (cl == 4) FCS_TOPK(1024, 4, 11, 4);
     if (cl == 8 && S <= 8 * 4096) FCS_TOPK(1024, 4, 11, 8);
     if (cl == 8 && S <= 8 * 8192) FCS_TOPK(1024, 8, 11, 8);
+    if (wide) FCS_TOPK(1024, 8, 11, 16);
     if (cl == 8) FCS_TOPK(1024, 16, 11, 8);
     FCS_TOPK(1024, 16, 11, 16);
 #undef FCS_TOPK

@@ -24,7 +24,8 @@
 // What bounds it: a dozen dependent steps of half a microsecond to one (launch of the cluster,
 // load, cluster barriers, scans), not bytes.  Back to back on a B200, one CTA per row going over
 // it from L2 with an element per thread and step (the form before) against this one: the 16384
-// largest of 131072 216 -> 14.6 us, 2048 of 16384 32 -> 7.5, 32 rows of 65536 118 -> 31; values
+// largest of 131072 216 -> 14.6 us (13.2 since the group sums are stored into the peers and nothing is exchanged at
+// the end, 11.0 on sixteen CTAs), 2048 of 16384 32 -> 7.5, 32 rows of 65536 118 -> 31; values
 // above the mean, 131072 122 -> 11.6 us, 32 rows of 65536 64 -> 13.6.  Rows of a few thousand are
 // bound by the host (4.4 us a call).  Four copies of the first pass's bins, against lanes meeting
 // on one bin, were no faster (14.9 us): the hardware adds equal addresses of a warp in one go.
@@ -400,6 +401,12 @@ inline int cluster_size(int S) {
     while (cl < most && (long long)cl * 4096 < S) cl *= 2;
     return cl;
 }
+
+// Top-k rows of 65537 to 131072 elements go to sixteen CTAs instead of eight up to this many rows.  us per call, eight /
+// sixteen: one row of 70000 11.8 / 10.6, of 100000 12.4 / 10.8, of 131072 12.6 / 11.0; two of 131072 15.0 / 14.1, four 15.0 / 14.4,
+// six 15.0 / 14.6 -- but eight of 80000 14.8 / 21.4: not all clusters of sixteen run at once any more.  Four is inside
+// the range where sixteen win.
+constexpr int TOPK_WIDE_ROWS = 4;
 
 }  // namespace sel
 }  // namespace fcs
