@@ -664,29 +664,41 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                     if (full) {
                         colsum_tile_ext_full(taddr, c, acc);
                     } else {
-                        // the columns that some row of the tile sees, in four runs of whole 32 -- or two key tiles
-                        // in this accumulator buffer, 128 query columns each: groups 0, 1 take the halves of the
-                        // first tile's columns, groups 2, 3 the second's
-                        const bool packed = L::SHORT && p.col_pack == 2;
-                        int kt = it.kt, q0, cols = GROUP_COLS, base = 0;
-                        bool any = true;
-                        if (packed) {
-                            const int tg = wg >> 1;
-                            if constexpr (L::SHORT) any = tg < it.nt;
-                            kt += tg;
-                            q0 = (wg & 1) * GROUP_COLS;
-                            base = tg * (BLOCK / 2);
+                        if constexpr (L::SHORT) {
+                            // Partly visible here are the blocks at the end of the query axis -- every item has one -- and
+                            // a few key tiles on the diagonal: fixed shares, decided with the fewest instructions.
+                            // Two key tiles in this accumulator buffer, 128 query columns each: groups 0, 1 take the
+                            // halves of the first tile's columns, groups 2, 3 the second's.  At most 128 query
+                            // columns otherwise: 32 for each group, not 64 for two of them.
+                            const bool packed = p.col_pack == 2, narrow = !packed && colsum_end_visible(p, st) <= BLOCK / 2;
+                            const int tg = packed ? wg >> 1 : 0;
+                            const int q0 = packed ? (wg & 1) * GROUP_COLS : narrow ? wg * (GROUP_COLS / 2) : col0;
+                            if (tg < it.nt) {
+                                const int end = colsum_end_visible(p, st) - q0;
+                                const int thr = colsum_first_visible(p, it.kt + tg, st, row) - q0;
+                                const int thr_first = __shfl_sync(0xffffffffu, thr, 0), thr_last = __shfl_sync(0xffffffffu, thr, 31);
+                                if (narrow) {
+                                    if (end > 0 && thr_first < GROUP_COLS / 2) {
+                                        uint32_t r[32];
+                                        tmem_ld_x32(taddr - col0 + q0, r);
+                                        tmem_ld_wait(r);
+                                        if (end >= GROUP_COLS / 2 && thr_last <= 0) colsum_chunk_ext<false>(r, 0, 32, c, acc);
+                                        else colsum_chunk_ext<true>(r, thr, end, c, acc);
+                                    }
+                                } else if (end > 0 && thr_first < GROUP_COLS) {
+                                    if (end >= GROUP_COLS && thr_last <= 0) colsum_tile_ext_full(taddr, c, acc);
+                                    else colsum_tile_ext(taddr, GROUP_COLS, thr, thr_first, thr_last, end, c, acc);
+                                }
+                            }
                         } else {
-                            const int from = colsum_first_visible(p, kt, st, 0) & ~31;
-                            cols = ((colsum_end_visible(p, st) - from + 127) >> 7) << 5;
-                            q0 = from + wg * cols;
-                        }
-                        if (any) {
+                            // the columns that some row of the tile sees, in four runs of whole 32
+                            const int from = colsum_first_visible(p, it.kt, st, 0) & ~31;
+                            const int cols = ((colsum_end_visible(p, st) - from + 127) >> 7) << 5, q0 = from + wg * cols;
                             const int end = colsum_end_visible(p, st) - q0;
-                            const int thr = colsum_first_visible(p, kt, st, row) - q0;
+                            const int thr = colsum_first_visible(p, it.kt, st, row) - q0;
                             // what the block's queries see of this warp's keys: nothing, everything, or some
                             const int thr_first = __shfl_sync(0xffffffffu, thr, 0), thr_last = __shfl_sync(0xffffffffu, thr, 31);
-                            const uint32_t at = taddr - col0 + base + q0;
+                            const uint32_t at = taddr - col0 + q0;
                             if (cols == GROUP_COLS && end >= GROUP_COLS && thr_last <= 0) colsum_tile_ext_full(at, c, acc);
                             else colsum_tile_ext(at, cols, thr, thr_first, thr_last, end, c, acc);
                         }
