@@ -288,7 +288,8 @@ colsum_fused_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     const int cols = ((seen + 127) >> 7) << 5, first = wg * cols;
                     const int lim = stats_last_visible(p, 0, kb, row) - first;
                     const int lim_first = __shfl_sync(0xffffffffu, lim, 0), lim_last = __shfl_sync(0xffffffffu, lim, 31);
-                    stats_tile(taddr - col0 + first, cols, lim, lim_first, lim_last, c, m_run, l_run);
+                    if (cols == GROUP_COLS && lim_first >= GROUP_COLS - 1) stats_tile_full(taddr, c, m_run, l_run);
+                    else stats_tile(taddr - col0 + first, cols, lim, lim_first, lim_last, c, m_run, l_run);
                 }
             }
             tc_fence_before();

@@ -23,6 +23,11 @@ constexpr uint32_t IDESC_BF16 = (1u << 7) | (1u << 10);
 __host__ __device__ constexpr bool pair_uses_polynomial(int pair, int of_16 = FCS_POLY_PAIRS) {
     return ((pair * of_16) % 16) < of_16;
 }
+// What a block of 32 columns goes through: all visible, with that share of polynomials; all visible, but in a tile that
+// a diagonal or a ragged end cuts, where no exp is a polynomial; or masked element by element, without polynomials.
+// (Polynomials in the visible blocks of cut tiles, too, left columns of small causal calls off by 1.4e-5, 2e-6 without,
+// for 0.5 % of the time of 8 x 16 x 2048 and of causal 2000 x 2000.)
+constexpr int BLOCK_FULL = 0, BLOCK_EXACT = 1, BLOCK_MASKED = 2;
 // The largest of three values, NaN if one of them is.
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
@@ -35,9 +40,10 @@ constexpr float ROW_MAX_START = -FLT_MAX;
 
 // Online (max, sum) update of one query row with 32 more scores.
 // `last_valid`: columns 0..last_valid are visible (>= 31: all).
-template <bool MASKED>
+template <int KIND>
 __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_valid, float c, float& m,
                                               float& l) {
+    constexpr bool MASKED = KIND == BLOCK_MASKED;
     float s[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
@@ -61,7 +67,7 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
     const float m_safe = max_or_nan(m, MASKED && cm == -INFINITY ? -INFINITY : cm * c);
     l *= ex2_approx(m - m_safe);
     m = m_safe;
-    if constexpr (!MASKED) {
+    if constexpr (KIND == BLOCK_FULL) {
         const f32x2 c2 = pack2(c, c), nm2 = pack2(-m_safe, -m_safe);
         f32x2 s0 = pack2(0.f, 0.f), s1 = s0;
 #pragma unroll
@@ -86,11 +92,12 @@ __device__ __forceinline__ void stats_block32(const uint32_t (&r)[32], int last_
         for (int j = 0; j < 32; j += 4) {
             float t0 = fmaf(s[j], c, -m_safe), t1 = fmaf(s[j + 1], c, -m_safe);
             float t2 = fmaf(s[j + 2], c, -m_safe), t3 = fmaf(s[j + 3], c, -m_safe);
-            // c may be 0 and s -inf: select after the multiply
-            t0 = (j <= last_valid) ? t0 : -INFINITY;
-            t1 = (j + 1 <= last_valid) ? t1 : -INFINITY;
-            t2 = (j + 2 <= last_valid) ? t2 : -INFINITY;
-            t3 = (j + 3 <= last_valid) ? t3 : -INFINITY;
+            if (MASKED) {   // c may be 0 and s -inf: select after the multiply
+                t0 = (j <= last_valid) ? t0 : -INFINITY;
+                t1 = (j + 1 <= last_valid) ? t1 : -INFINITY;
+                t2 = (j + 2 <= last_valid) ? t2 : -INFINITY;
+                t3 = (j + 3 <= last_valid) ? t3 : -INFINITY;
+            }
             a0 += ex2_approx(t0); a1 += ex2_approx(t1);
             a2 += ex2_approx(t2); a3 += ex2_approx(t3);
         }
@@ -196,11 +203,12 @@ __device__ __forceinline__ void make_ext_row(float nl, float inv_c, bool bf16, u
 }
 
 // Column-pass chunk when the accumulator already holds s + nl/c: add exp2(c * acc).
-template <bool MASKED>
+template <int KIND>
 __device__ __forceinline__ void colsum_chunk_ext(const uint32_t (&r)[32], int first_valid, int end_valid, float c,
                                                  float (&acc)[4]) {
+    constexpr int POLY = KIND == BLOCK_FULL ? FCS_POLY_PAIRS : 0;
     const f32x2 c2 = pack2(c, c);
-    if constexpr (!MASKED) {
+    if constexpr (KIND != BLOCK_MASKED) {
         f32x2 a01 = pack2(acc[0], acc[1]), a23 = pack2(acc[2], acc[3]);
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
@@ -208,9 +216,9 @@ __device__ __forceinline__ void colsum_chunk_ext(const uint32_t (&r)[32], int fi
             const f32x2 tb = mul2(pack2(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])), c2);
             f32x2 ea, eb;
             float u0, u1;
-            if (pair_uses_polynomial((j >> 1) & 15)) { ea = ex2_poly2(ta); }
+            if (pair_uses_polynomial((j >> 1) & 15, POLY)) { ea = ex2_poly2(ta); }
             else { unpack2(ta, u0, u1); ea = pack2(ex2_approx(u0), ex2_approx(u1)); }
-            if (pair_uses_polynomial(((j >> 1) + 1) & 15)) { eb = ex2_poly2(tb); }
+            if (pair_uses_polynomial(((j >> 1) + 1) & 15, POLY)) { eb = ex2_poly2(tb); }
             else { unpack2(tb, u0, u1); eb = pack2(ex2_approx(u0), ex2_approx(u1)); }
             a01 = add2(a01, ea);
             a23 = add2(a23, eb);

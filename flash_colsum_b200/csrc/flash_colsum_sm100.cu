@@ -119,10 +119,10 @@ __device__ __forceinline__ void stats_tile_full(uint32_t taddr, float c, float& 
     uint32_t r[32];
     tmem_ld_x32(taddr, r);
     tmem_ld_wait(r);
-    stats_block32<false>(r, 32, c, m, l);
+    stats_block32<BLOCK_FULL>(r, 32, c, m, l);
     tmem_ld_x32(taddr + 32, r);
     tmem_ld_wait(r);
-    stats_block32<false>(r, 32, c, m, l);
+    stats_block32<BLOCK_FULL>(r, 32, c, m, l);
 }
 __device__ __forceinline__ void colsum_tile_ext_full(uint32_t taddr, float c, float (&acc)[4]) {
     // 16 columns at a time, the next 16 in flight from tensor memory while these are in the exp pipes
@@ -140,10 +140,10 @@ __device__ __forceinline__ void colsum_tile_ext_full(uint32_t taddr, float c, fl
     tmem_wait_16cols(rb);
     colsum_chunk16_ext<8>(rb, c, acc);
 }
-// The same where some elements are hidden, in runs of 32 columns: what no row of the warp sees is not read, what all
-// rows see takes the arithmetic above, and only the runs that the diagonal or the ragged end goes through are masked;
-// the four groups share what is visible (2000 x 2000 causal, 128 heads of 128 columns, passes apart: statistics 117 ->
-// 114 us, columns 119 -> 105; back to back 240.9 -> 229.2 us a call.  Before, a group masked its fixed quarter as a whole).
+// The same where some elements are hidden, in runs of 32 columns: what no row of the warp sees is not read, only the runs
+// that the diagonal or the ragged end goes through are masked, and the four groups share what is visible.  (Before, a
+// group masked its fixed quarter as a whole.)  Its exps are all the special-function unit's, in a run that all rows see
+// too: the polynomial is for whole tiles and whole quarters of one.
 //
 // Statistics: columns 0 .. lim of this row are visible; lim_first / lim_last: the same of the warp's first and
 // last row (the least and the most any of its rows sees).
@@ -155,8 +155,8 @@ __device__ __forceinline__ void stats_tile(uint32_t taddr, int cols, int lim, in
         uint32_t r[32];
         tmem_ld_x32(taddr + j, r);
         tmem_ld_wait(r);
-        if (lim_first >= j + 31) stats_block32<false>(r, 32, c, m, l);
-        else stats_block32<true>(r, lim - j, c, m, l);
+        if (lim_first >= j + 31) stats_block32<BLOCK_EXACT>(r, 32, c, m, l);
+        else stats_block32<BLOCK_MASKED>(r, lim - j, c, m, l);
     }
 }
 // Columns thr <= j < end of this row are visible; thr_first / thr_last: thr of the warp's first and last row.
@@ -168,8 +168,8 @@ __device__ __forceinline__ void colsum_tile_ext(uint32_t taddr, int cols, int th
         uint32_t r[32];
         tmem_ld_x32(taddr + j, r);
         tmem_ld_wait(r);
-        if (thr_last <= j && j + 32 <= end) colsum_chunk_ext<false>(r, 0, 32, c, acc);
-        else colsum_chunk_ext<true>(r, thr - j, end - j, c, acc);
+        if (thr_last <= j && j + 32 <= end) colsum_chunk_ext<BLOCK_EXACT>(r, 0, 32, c, acc);
+        else colsum_chunk_ext<BLOCK_MASKED>(r, thr - j, end - j, c, acc);
     }
 }
 template <bool MASKED>
@@ -648,17 +648,21 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 const uint32_t taddr = lane_addr + buf * BLOCK;
                 const bool full = (st >= f_lo) && (st < f_hi);
                 if constexpr (MODE == MODE_STATS) {
-                    if (full) {
-                        stats_tile_full(taddr, c, m_run, l_run);
-                    } else {
+                    bool whole = full;
+                    int cols = GROUP_COLS, first = col0, lim = 0, lim_first = 0, lim_last = 0;
+                    if (!full) {
                         // the columns that some row of the tile sees, in four runs of whole 32
                         int seen = stats_last_visible(p, it.qt, st, TILE - 1) + 1;
                         seen = seen < BLOCK ? seen : BLOCK;
-                        const int cols = ((seen + 127) >> 7) << 5, first = wg * cols;
-                        const int lim = stats_last_visible(p, it.qt, st, row) - first;
-                        const int lim_first = __shfl_sync(0xffffffffu, lim, 0), lim_last = __shfl_sync(0xffffffffu, lim, 31);
-                        stats_tile(taddr - col0 + first, cols, lim, lim_first, lim_last, c, m_run, l_run);
+                        cols = ((seen + 127) >> 7) << 5;
+                        first = wg * cols;
+                        lim = stats_last_visible(p, it.qt, st, row) - first;
+                        lim_first = __shfl_sync(0xffffffffu, lim, 0);
+                        lim_last = __shfl_sync(0xffffffffu, lim, 31);
+                        whole = cols == GROUP_COLS && lim_first >= GROUP_COLS - 1;
                     }
+                    if (whole) stats_tile_full(taddr, c, m_run, l_run);
+                    else stats_tile(taddr - col0 + first, cols, lim, lim_first, lim_last, c, m_run, l_run);
                 } else if constexpr (EXT) {
                     // the accumulator already holds s - lse/c
                     if (full) {
@@ -682,8 +686,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                                         uint32_t r[32];
                                         tmem_ld_x32(taddr - col0 + q0, r);
                                         tmem_ld_wait(r);
-                                        if (end >= GROUP_COLS / 2 && thr_last <= 0) colsum_chunk_ext<false>(r, 0, 32, c, acc);
-                                        else colsum_chunk_ext<true>(r, thr, end, c, acc);
+                                        if (end >= GROUP_COLS / 2 && thr_last <= 0) colsum_chunk_ext<BLOCK_FULL>(r, 0, 32, c, acc);
+                                        else colsum_chunk_ext<BLOCK_MASKED>(r, thr, end, c, acc);
                                     }
                                 } else if (end > 0 && thr_first < GROUP_COLS) {
                                     if (end >= GROUP_COLS && thr_last <= 0) colsum_tile_ext_full(taddr, c, acc);
@@ -699,7 +703,8 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                             // what the block's queries see of this warp's keys: nothing, everything, or some
                             const int thr_first = __shfl_sync(0xffffffffu, thr, 0), thr_last = __shfl_sync(0xffffffffu, thr, 31);
                             const uint32_t at = taddr - col0 + q0;
-                            if (cols == GROUP_COLS && end >= GROUP_COLS && thr_last <= 0) colsum_tile_ext_full(at, c, acc);
+                            if (cols == GROUP_COLS && from % GROUP_COLS == 0 && end >= GROUP_COLS && thr_last <= 0)
+                                colsum_tile_ext_full(at, c, acc);
                             else colsum_tile_ext(at, cols, thr, thr_first, thr_last, end, c, acc);
                         }
                     }
