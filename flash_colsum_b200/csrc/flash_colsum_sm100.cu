@@ -1359,6 +1359,34 @@ static bool single_pass_applies(int B, int H, int Sq, int Sk, int D, int causal)
     return tiles <= 512;
 }
 
+// Clusters of `cl` CTAs of `kern` that the current device runs at once; 0 where it holds none, or does not say.  Asked
+// once per device; `answers` holds one more than the answer.
+static int resident_clusters(const void* kern, int cl, int threads, int smem, int (&answers)[64]) {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (answers[dev]) return answers[dev] - 1;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(cl * 64));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)cl;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 0) {
+        cudaGetLastError();
+        n = 0;
+    }
+    answers[dev] = n + 1;
+    return n;
+}
+
 // The instance for clusters of `cl` CTAs.
 typedef void (*SinglePassKernel)(const CUtensorMap, const CUtensorMap, const SinglePassParams);
 template <bool PADDED>
@@ -1622,15 +1650,10 @@ static int launch_round_fp32(const float* q, const float* k, void* q16, void* k1
     attrs[1].val.clusterDim.y = 1;
     attrs[1].val.clusterDim.z = 1;
     cudaError_t e;
-    if ((long long)rp.op[0].pieces + rp.op[1].pieces <= rnd::SMALL_PIECES) {
-        static bool configured[64] = {false};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev >= 0 && dev < 64 && !configured[dev]) {
-            e = cudaFuncSetAttribute(rnd::round_small_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (e != cudaSuccess) return fail(FCS_ERR_CUDA, "rounding fp32 operands failed: %s", cudaGetErrorString(e));
-            configured[dev] = true;
-        }
+    static int resident[64] = {0};
+    if (round_in_one_kernel((long long)rp.op[0].pieces + rp.op[1].pieces,
+                            resident_clusters(reinterpret_cast<const void*>(rnd::round_small_kernel), rnd::SMALL_CTAS,
+                                              rnd::SMALL_THREADS, 0, resident))) {
         cfg.gridDim = dim3(rnd::SMALL_CTAS);
         cfg.blockDim = dim3(rnd::SMALL_THREADS);
         cfg.attrs = overlap_previous() ? attrs : attrs + 1;
@@ -1975,8 +1998,10 @@ static cudaError_t launch_topk_t(const float* colsum, long long ld, int B, int S
 static cudaError_t launch_topk(const float* colsum, long long ld, int B, int S, int k, int* indices, float* values,
                                cudaStream_t stream) {
     const int cl = sel::cluster_size(S);
-    // (half the elements per CTA while all rows' clusters of sixteen run at once)
-    const bool wide = cl == 8 && S > 8 * 8192 && B <= sel::TOPK_WIDE_ROWS;
+    static int resident[64] = {0};
+    const bool wide = topk_on_sixteen(S, B, 16) &&
+                      topk_on_sixteen(S, B, resident_clusters(reinterpret_cast<const void*>(sel::topk_kernel<1024, 8, 11, 16>),
+                                                              16, 1024, sel::topk_smem<1024, 8, 11, 16>(), resident));
 #define FCS_TOPK(NT, E, BITS, CL) return launch_topk_t<NT, E, BITS, CL>(colsum, ld, B, S, k, indices, values, stream)
     if (S <= 1024) FCS_TOPK(256, 4, 8, 1);
     if (cl == 1) FCS_TOPK(1024, 4, 11, 1);

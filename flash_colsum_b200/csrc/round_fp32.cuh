@@ -10,7 +10,7 @@
 // bytes per element.  (An abs / max / read-back per operand and two conversions by torch
 // operators took 85 us for a call of a megabyte.)
 //
-// Operands of up to SMALL_PIECES pieces are over before a launch is: there both steps are one kernel on one
+// Small operands (round_in_one_kernel) are over before a launch is: there both steps are one kernel on one
 // cluster of sixteen CTAs, which ask each other through shared memory instead of notes.  Either way the output of
 // the call is zeroed on the side, which is a launch less for the kernels that add into it (2 x 4 x 256 x 64, a
 // megabyte, back to back: four launches 11.45 us, two 10.24).
@@ -27,7 +27,6 @@ namespace rnd {
 
 constexpr int THREADS = 256;
 constexpr int SMALL_CTAS = 16, SMALL_THREADS = 512;
-constexpr long long SMALL_PIECES = 65536;
 constexpr float FP16_LIMIT = 60000.f;
 
 struct Operand {

@@ -640,6 +640,25 @@ FCS_HD inline bool fused_short_plan(int B, int H, int Sq, int Sk, int causal, in
     return true;
 }
 
+// ---------------------------------------------------------------------------
+// Two kernels run on clusters of sixteen CTAs, which a device need not be able to hold (a partition of one has too few
+// neighbouring SMs).  `resident`: how many such clusters the device runs at once.  Without one, the forms that were there
+// before them take the call.
+// ---------------------------------------------------------------------------
+// fp32 operands of up to this many pieces of eight elements (both together) are rounded by one kernel on one cluster,
+// larger ones by two kernels.
+constexpr long long ROUND_SMALL_PIECES = 65536;
+FCS_HD inline bool round_in_one_kernel(long long pieces, int resident) {
+    return pieces <= ROUND_SMALL_PIECES && resident >= 1;
+}
+// Top-k rows of 65537 to 131072 elements go to sixteen CTAs instead of eight while all rows' clusters run at once, up to
+// four rows.  us per call, eight / sixteen: one row of 70000 11.8 / 10.6, of 100000 12.4 / 10.8, of 131072 12.6 / 11.0; two of
+// 131072 15.0 / 14.1, four 15.0 / 14.4, six 15.0 / 14.6 -- but eight of 80000 14.8 / 21.4: more rows than clusters.
+constexpr int TOPK_WIDE_ROWS = 4;
+FCS_HD inline bool topk_on_sixteen(int S, int B, int resident) {
+    return S > 8 * 8192 && S <= 8 * 16384 && B <= TOPK_WIDE_ROWS && B <= resident;
+}
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Scratch layout: [neg_lse | ext | part]; returns the total and the offsets.

@@ -394,19 +394,13 @@ threshold_kernel(const float* __restrict__ colsum, long long ld, int S, float th
 // CTAs per row: as many as it takes for 4096 elements each, at most eight -- or sixteen where that
 // keeps the slices in registers (more than 131072 elements; one row of 262144: 17.7 us against 38).
 // (Below that sixteen lose to eight, 12.3 against 10.7 us at 65536 elements: the cluster barriers
-// and the launch grow with the cluster.)
+// and the launch grow with the cluster.  Top-k calls of few rows have a line of their own, topk_on_sixteen.)
 inline int cluster_size(int S) {
     const int most = S > 8 * 16384 ? MAX_CL : 8;
     int cl = 1;
     while (cl < most && (long long)cl * 4096 < S) cl *= 2;
     return cl;
 }
-
-// Top-k rows of 65537 to 131072 elements go to sixteen CTAs instead of eight up to this many rows.  us per call, eight /
-// sixteen: one row of 70000 11.8 / 10.6, of 100000 12.4 / 10.8, of 131072 12.6 / 11.0; two of 131072 15.0 / 14.1, four 15.0 / 14.4,
-// six 15.0 / 14.6 -- but eight of 80000 14.8 / 21.4: not all clusters of sixteen run at once any more.  Four is inside
-// the range where sixteen win.
-constexpr int TOPK_WIDE_ROWS = 4;
 
 }  // namespace sel
 }  // namespace fcs

@@ -429,3 +429,6 @@ extern "C" int check_stats_order(int B, int H, int Sq, int Sk, int k_past, int s
         }
     return p.stats_heads;
 }
+
+extern "C" int rounds_in_one_kernel(long long pieces, int resident) { return round_in_one_kernel(pieces, resident); }
+extern "C" int topk_takes_sixteen(int S, int B, int resident) { return topk_on_sixteen(S, B, resident); }

@@ -318,3 +318,16 @@ def test_causal_statistics_items_longest_first(emu, B, H, Sq, Sk, k_past, sms, h
     """Every item of the rounds of heads comes once, the longest query tiles of a round first."""
     got = emu.check_stats_order(B, H, Sq, Sk, k_past, sms)
     assert got == heads
+
+
+def test_clusters_of_sixteen_only_where_the_device_holds_them(emu):
+    """A device (or a partition of one) that cannot hold a cluster of sixteen CTAs keeps the other forms."""
+    emu.rounds_in_one_kernel.argtypes = [ctypes.c_longlong, ctypes.c_int]
+    for pieces in (1, 1000, 32768, 65536, 65537, 10 ** 9):
+        assert not emu.rounds_in_one_kernel(pieces, 0)
+    assert emu.rounds_in_one_kernel(1000, 1) and not emu.rounds_in_one_kernel(65537, 9)
+    for S in (1, 65536, 65537, 100000, 131072, 131073):
+        for B in (1, 2, 4, 5):
+            for resident in (0, 1, 3, 9):
+                want = 65536 < S <= 131072 and B <= 4 and B <= resident
+                assert bool(emu.topk_takes_sixteen(S, B, resident)) == want, (S, B, resident)
