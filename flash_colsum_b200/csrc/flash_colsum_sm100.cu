@@ -1612,9 +1612,9 @@ static int launch_fused_short(const CUtensorMap& tq, const CUtensorMap& tk, cons
 }
 
 // fp32 operands rounded into `q16` / `k16` (dense [B][H][rows][D]); `fmt` receives the type.  `out` (or NULL): B rows
-// of Sk values, out_ld apart, that are zeroed alongside.
+// of Sk values, out_ld apart, that are zeroed alongside.  `one_kernel_follows`: the call's kernels behind it are one.
 static int launch_round_fp32(const float* q, const float* k, void* q16, void* k16, int* notes, int n_notes, int* fmt, float* out,
-                             int64_t out_ld, int B,
+                             int64_t out_ld, bool one_kernel_follows, int B,
                              int H, int Sq, int Sk, int D, int64_t qsb, int64_t qsh, int64_t qss, int64_t ksb, int64_t ksh,
                              int64_t kss, cudaStream_t stream) {
     rnd::Params rp;
@@ -1651,7 +1651,7 @@ static int launch_round_fp32(const float* q, const float* k, void* q16, void* k1
     attrs[1].val.clusterDim.z = 1;
     cudaError_t e;
     static int resident[64] = {0};
-    if (round_in_one_kernel((long long)rp.op[0].pieces + rp.op[1].pieces,
+    if (round_in_one_kernel((long long)rp.op[0].pieces + rp.op[1].pieces, one_kernel_follows,
                             resident_clusters(reinterpret_cast<const void*>(rnd::round_small_kernel), rnd::SMALL_CTAS,
                                               rnd::SMALL_THREADS, 0, resident))) {
         cfg.gridDim = dim3(rnd::SMALL_CTAS);
@@ -1756,9 +1756,12 @@ static int colsum_impl(const void* q, const void* k, float* out, int64_t out_ld,
         uint8_t* ws = static_cast<uint8_t*>(alloc(alloc_ctx, head + q_bytes + k_bytes));
         if (!ws) return fail(FCS_ERR_WORKSPACE, "no scratch memory for the rounded fp32 operands");
         int* words = reinterpret_cast<int*>(ws);
+        const bool one_kernel = passes == PASSES_BOTH &&
+                                (single_pass_applies(B, H, Sq, Sk, D, causal) ||
+                                 (!sig && short_fused_applies(B, H, Sq, Sk, D, causal, k_past, nullptr, nullptr, nullptr)));
         rc = launch_round_fp32(static_cast<const float*>(q), static_cast<const float*>(k), ws + head, ws + head + q_bytes,
-                               words + 1, (int)notes, words, passes == PASSES_BOTH && clear_out ? out : nullptr, out_ld, B, H, Sq,
-                               Sk, D, qsb, qsh, qss, ksb, ksh, kss, stream);
+                               words + 1, (int)notes, words, passes == PASSES_BOTH && clear_out ? out : nullptr, out_ld,
+                               one_kernel, B, H, Sq, Sk, D, qsb, qsh, qss, ksb, ksh, kss, stream);
         if (rc != FCS_OK) return rc;
         to_clear = false;
         q = ws + head;

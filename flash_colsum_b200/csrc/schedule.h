@@ -645,11 +645,16 @@ FCS_HD inline bool fused_short_plan(int B, int H, int Sq, int Sk, int causal, in
 // neighbouring SMs).  `resident`: how many such clusters the device runs at once.  Without one, the forms that were there
 // before them take the call.
 // ---------------------------------------------------------------------------
-// fp32 operands of up to this many pieces of eight elements (both together) are rounded by one kernel on one cluster,
-// larger ones by two kernels.
-constexpr long long ROUND_SMALL_PIECES = 65536;
-FCS_HD inline bool round_in_one_kernel(long long pieces, int resident) {
-    return pieces <= ROUND_SMALL_PIECES && resident >= 1;
+// fp32 operands of few pieces of eight elements (both together) are rounded by one kernel on one cluster, the others by two
+// kernels on all SMs.  One kernel takes the device longer (16 of 148 SMs) and the host less: it wins where the call
+// behind it is one kernel, too, and waits for the host, as long as a thread's pieces are one round of loads (16 x 512
+// threads of four); in front of the streaming passes, half of that.  us per call, one / two, fp16 values (bf16 ones, which
+// are read twice): one kernel follows, D = 64, 24576 pieces 9.2 / 9.8 (10.4 / 10.5), 32768 9.3 / 9.7 (10.6 / 10.4),
+// 40960 11.8 / 11.4 (13.6 / 12.4), 65536 11.5 / 11.0 (13.6 / 12.0); streaming, D = 128, 16384 16.1 / 16.6
+// (16.9 / 17.3), 22400 20.7 / 20.1, 24576 20.0 / 19.5 (21.2 / 20.2), 65536 22.0 / 20.0 (24.2 / 21.0).
+constexpr long long ROUND_SMALL_PIECES = 32768, ROUND_SMALL_PIECES_STREAMING = 16384;
+FCS_HD inline bool round_in_one_kernel(long long pieces, bool one_kernel_follows, int resident) {
+    return pieces <= (one_kernel_follows ? ROUND_SMALL_PIECES : ROUND_SMALL_PIECES_STREAMING) && resident >= 1;
 }
 // Top-k rows of 65537 to 131072 elements go to sixteen CTAs instead of eight while all rows' clusters run at once, up to
 // four rows.  us per call, eight / sixteen: one row of 70000 11.8 / 10.6, of 100000 12.4 / 10.8, of 131072 12.6 / 11.0; two of

@@ -430,5 +430,7 @@ extern "C" int check_stats_order(int B, int H, int Sq, int Sk, int k_past, int s
     return p.stats_heads;
 }
 
-extern "C" int rounds_in_one_kernel(long long pieces, int resident) { return round_in_one_kernel(pieces, resident); }
+extern "C" int rounds_in_one_kernel(long long pieces, int one_kernel_follows, int resident) {
+    return round_in_one_kernel(pieces, one_kernel_follows != 0, resident);
+}
 extern "C" int topk_takes_sixteen(int S, int B, int resident) { return topk_on_sixteen(S, B, resident); }

@@ -1,4 +1,4 @@
-"""fp32 operands on both sides of the line between one rounding kernel and two: the same call on operands that were rounded
+"""fp32 operands on both sides of the lines between one rounding kernel and two: the same call on operands that were rounded
 beforehand, and an output that holds something else before the call."""
 
 import pytest
@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("B,H,S,D", [(1, 2, 2048, 64), (1, 2, 2049, 64), (1, 1, 5, 64), (2, 4, 256, 64), (3, 3, 301, 80),
-                                     (1, 8, 512, 64), (1, 8, 513, 64)])
+                                     (1, 8, 512, 64), (1, 8, 513, 64),
+                                     (1, 2, 1024, 64), (1, 2, 1025, 64), (1, 1, 512, 128), (1, 1, 513, 128)])
 @pytest.mark.parametrize("factor", [1.0, 1e5])
 def test_one_rounding_kernel_or_two(B, H, S, D, factor):
     if not torch.cuda.is_available():

@@ -322,10 +322,11 @@ def test_causal_statistics_items_longest_first(emu, B, H, Sq, Sk, k_past, sms, h
 
 def test_clusters_of_sixteen_only_where_the_device_holds_them(emu):
     """A device (or a partition of one) that cannot hold a cluster of sixteen CTAs keeps the other forms."""
-    emu.rounds_in_one_kernel.argtypes = [ctypes.c_longlong, ctypes.c_int]
-    for pieces in (1, 1000, 32768, 65536, 65537, 10 ** 9):
-        assert not emu.rounds_in_one_kernel(pieces, 0)
-    assert emu.rounds_in_one_kernel(1000, 1) and not emu.rounds_in_one_kernel(65537, 9)
+    emu.rounds_in_one_kernel.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+    for pieces in (1, 1000, 16384, 16385, 32768, 32769, 65536, 10 ** 9):
+        for follows, line in ((0, 16384), (1, 32768)):      # (past these two kernels were measured to be faster)
+            assert not emu.rounds_in_one_kernel(pieces, follows, 0)
+            assert bool(emu.rounds_in_one_kernel(pieces, follows, 1)) == (pieces <= line)
     for S in (1, 65536, 65537, 100000, 131072, 131073):
         for B in (1, 2, 4, 5):
             for resident in (0, 1, 3, 9):
