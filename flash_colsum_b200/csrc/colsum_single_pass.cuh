@@ -22,8 +22,8 @@
 // which is the time the statistics of tile i have to go around the cluster.
 //
 // A tile takes a CTA the same time whatever the number of real keys in its slice; keys past S_k are
-// overwritten in tensor memory.  us per call (B = 32, H = 16) with the padding masked in registers and here:
-// 400 keys 71 -> 63, 577 137 -> 117; the rule for which calls come here is with the launcher.
+// overwritten in tensor memory (masked in registers, 400 keys took 71 us instead of 63, 577 137 instead of 117,
+// B = 32, H = 16, when that was measured; 56 and 101 now).  The rule for which calls come here is with the launcher.
 #pragma once
 
 #include <float.h>
@@ -360,7 +360,8 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     // The column sums leave tensor memory at the end of a batch entry, of this cluster's range,
     // and every `flush_units` pairs: the tensor core truncates when it adds into its fp32
     // accumulator (about half a unit in the last place lost per accumulation), and the bound
-    // keeps that bias below ~1e-4 of a column sum however many heads there are.
+    // keeps that bias below ~1e-4 of a column sum however many heads there are.  (A pair has at most 16 query
+    // tiles: these calls have no more queries than keys.)
     auto last_of_batch = [&](int u) { return range.flush_after(u, p.H, p.flush_units); };
 
     if (warp == SCORES_WARP) {
@@ -574,6 +575,11 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         // 8 x 12 x 900 47.6 / 46.1 / 47.9 / 46.9, 16 x 16 x 1000 110.0 / 106.2 / 109.4 / 106.9, 8 x 16 x 1500 122.0 / 119.5 /
         // 122.3 / 120.2; in the other instance 32 x 16 x 512 keys 55.5 / 56.1 / 53.2 / 52.1, 1024 214.9 / 215.6 / 205.9 / 198.5.
         constexpr int POLY = PADDED ? 3 : FCS_POLY_PAIRS;
+        // Whether the wait for tile i-2's buffers is asked early, so that the answer is there when it is needed.  Measured, not
+        // derived: the two instances have their registers differently full, and each has the form that leaves it the
+        // better schedule.  (us per call, 32 x 16 pairs, asked early / not: 577 keys 100.9 / 107.8; 512 keys 56.2 /
+        // 52.1, 1024 keys 211.4 / 198.5.)  Another compiler may turn it over.
+        constexpr bool ASK_EARLY = PADDED;
         auto consume = [&](auto keys) {
         constexpr bool KEYS = decltype(keys)::value;     // false: nothing but padding
         int i = 0, fc = 0, sb = hf, sph = 0;             // sb, sph: this half's score accumulator and its phase
@@ -626,11 +632,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             mbar_arrive(s_empty(sb));
             sb += 2;                                   // (accumulators 2 i + hf, mod 3)
             if (sb >= S_BUFS) { sb -= S_BUFS; sph ^= 1; }
-            // Whether tile i-2 is through, asked early in the padded instance, so that the answer is there when it is
-            // needed.  (us per call, 32 x 16 pairs, asked early / not: 577 keys 100.9 / 107.8; 512 keys 56.2 / 52.1, 1024
-            // keys 211.4 / 198.5 -- the two instances have their registers differently full, and each has the form
-            // that leaves it the better schedule.)
-            const bool freed = PADDED && mbar_test_wait(pw_free(slot, hf), ((i >> 1) & 1) ^ 1);
+            const bool freed = ASK_EARLY && mbar_test_wait(pw_free(slot, hf), ((i >> 1) & 1) ^ 1);
 
             // ---- P~ = exp2(c*s - m_g) as packed fp16
             uint32_t h[32];
@@ -657,7 +659,7 @@ colsum_single_pass_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             }
             // ---- tile i-2 is through: its column-sum MMA has read P~(i-2), and (before that)
             // the exchange warps have read its statistics -- both slots are free
-            if (!PADDED || !__all_sync(0xffffffffu, freed)) {
+            if (!ASK_EARLY || !__all_sync(0xffffffffu, freed)) {
                 ok = mbar_wait(pw_free(slot, hf), ((i >> 1) & 1) ^ 1, abort_flag, p.status, FCS_STATUS_WAIT_CONSUMER);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;

@@ -23,9 +23,9 @@
 //     into every CTA of the cluster with st.async, counted on the receiver's mbarrier -- no
 //     cluster-wide barrier per unit.  A unit is finished (weights, one add per key into the
 //     output) one unit late, behind the scores of the next, when every range's values are in.
-//   * The output is cleared by a small kernel launched just before; this kernel is a
-//     programmatic dependent of it and waits for it only before its first add, so the
-//     clear costs no time on the device.
+//   * The output is cleared by a small kernel launched just before.  This kernel is a programmatic
+//     dependent of it, and only its set-up overlaps: the clear lets its dependents go before its own wait,
+//     so that its end is what says that the operands are written, too, and nothing is read before.
 #pragma once
 
 #include <cuda_bf16.h>

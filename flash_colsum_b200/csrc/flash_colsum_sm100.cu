@@ -1333,8 +1333,8 @@ static int launch_few_rows(const void* q, const void* k, float* out, int64_t out
 }
 
 // Short key axes (non-causal, head dimension 64, S_k <= 2048): the single-pass
-// cluster kernel.  g_single_pass: 0 = where it is the faster of the two (see
-// single_pass_applies), 1 = never, 2 = whenever the shape allows.
+// cluster kernel.  g_single_pass: 0 = as single_pass_applies says, 1 = never, 2 = whenever
+// the shape allows.
 static int g_single_pass = 0;
 
 static int single_pass_cluster_size(int Sk) {
@@ -1345,13 +1345,13 @@ static bool single_pass_applies(int B, int H, int Sq, int Sk, int D, int causal)
     if (g_single_pass == 1 || causal || D > 64 || Sk > 256 * sp::MAX_CL) return false;   // (D < 64: zero-filled columns)
     if (g_single_pass == 2) return true;
     const int cl = single_pass_cluster_size(Sk);
-    // us per call, this form / the two passes, at 32 x 16 pairs and at 2 x 8: 96 keys 19/23 9/9, 150 27/34
-    // 8/13, 320 50/54 9/14, 520 118/133 13/20, 640 114/139 12/20, 1030 342/381 21/23, 1400 489/544 24/38 -- the
-    // time goes by whole slices of 256 keys, and up to six of them it wins at any fill from 60 %
-    // (one slice: at any length); clusters of 7 and 8 fit only 15 at a time (105 / 120 of 148 SMs) and lose
-    // on large calls (2048 keys: 1046/998) but win on small ones (41/50), where the fixed costs of two
-    // launches and partial waves weigh more.  (Both forms as they were when the line was drawn.  This one takes 10 to
-    // 16 % less now -- 1024 keys 230 -> 199 us, 577 112 -> 101 -- and the line stays: past it, exps keep 32 bits.)
+    // us per call, this form / the two passes, at 32 x 16 pairs and at 2 x 8: 96 keys 16/20 7/8, 150 21/30 7/12,
+    // 300 48/56 9/15, 320 44/54 10/15, 520 101/119 12/20, 640 95/141 12/21, 1030 293/358 19/22, 1400 416/556 22/37,
+    // 1700 760/805 34/46, 2048 847/1077 37/49.  The line lies where this form won when it was drawn, before it took the
+    // last 10 to 20 %: at any fill of one slice, from a fill of 60 % up to six (the time goes by whole slices of 256
+    // keys), and with clusters of 7 and 8, which fit only 15 at a time (105 / 120 of 148 SMs), on small calls only.  It is
+    // the faster one beyond the line, too, by now; the line stays because calls past it have their exps summed in
+    // 32 bits, and here they are rounded to fp16.
     if (cl == 1) return true;
     if (cl <= 6) return (long long)Sk * 100 >= (long long)cl * 256 * 60;
     if ((long long)Sk * 100 < (long long)cl * 256 * 85) return false;
@@ -1451,7 +1451,8 @@ static int launch_single_pass(const CUtensorMap& tq, const CUtensorMap& tk, floa
         const long long tiles = (long long)sp_.units * sp_.NQ;
         sp_.clusters = tiles < max_clusters ? (int)tiles : max_clusters;
     }
-    // at most ~1024 accumulations (16 query rows each) per flush
+    // at most 1024 accumulations (16 query rows each) per flush: NQ is 16 at most, since every entry point that comes
+    // here has as many keys as queries (or fewer rows that enter the mean)
     sp_.flush_units = 128 / sp_.NQ > 1 ? 128 / sp_.NQ : 1;
     // (a scale of zero under a ragged end as the smallest number there is: every fp32 score times it is below 5e-7
     // in size, and the -inf of a column of padding stays -inf)
@@ -1546,8 +1547,9 @@ static bool short_fused_applies(int B, int H, int Sq, int Sk, int D, int causal,
 
 // Whether all (batch, head) pairs of a call the one-kernel form takes run at once: such a call
 // goes there even where the single-pass kernel would take it (B=4 H=16, 100 CLS rows over 577
-// keys: 19 against 23.5 us); with several waves of CTAs the single-pass kernel keeps it (B=32:
-// 50 against 58 us).
+// keys: 11.9 against 12.6 us, 20 rows 10.5 / 11.9, 8 x 16 x 577 a tie at 14); with several waves of CTAs the
+// single-pass kernel keeps it (B=32: 31 against 51 us).  (8 x 16 x 256, 64 rows: 8.4 here, 7.3 there; as with
+// the line above, this form's exps keep 32 bits.)
 static bool short_fused_one_wave(int B, int H, int D, int cl) {
     const int* table = D <= 64 ? fused_short_max_clusters<64>() : fused_short_max_clusters<128>();
     return (long long)B * H <= (cl > 1 ? table[cl] : num_sms());

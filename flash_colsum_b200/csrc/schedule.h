@@ -657,8 +657,10 @@ FCS_HD inline bool round_in_one_kernel(long long pieces, bool one_kernel_follows
     return pieces <= (one_kernel_follows ? ROUND_SMALL_PIECES : ROUND_SMALL_PIECES_STREAMING) && resident >= 1;
 }
 // Top-k rows of 65537 to 131072 elements go to sixteen CTAs instead of eight while all rows' clusters run at once, up to
-// four rows.  us per call, eight / sixteen: one row of 70000 11.8 / 10.6, of 100000 12.4 / 10.8, of 131072 12.6 / 11.0; two of
-// 131072 15.0 / 14.1, four 15.0 / 14.4, six 15.0 / 14.6 -- but eight of 80000 14.8 / 21.4: more rows than clusters.
+// four rows.  us per call, eight / sixteen, in the faster of the two times a call takes: one row of 40000 8.4 / 9.2, of 57000
+// 8.8 / 9.4, of 65536 9.0 / 9.5 -- eight, 8192 elements a CTA at most; of 65537, where eight take twice the registers,
+// 11.5 / 10.5, of 100000 12.1 / 10.8, of 131072 12.5 / 11.0.  In the slower one: two of 131072 15.0 / 14.0, four 14.9 /
+// 14.4, six 15.0 / 14.6, but eight of 80000 14.8 / 21.4: more rows than clusters.
 constexpr int TOPK_WIDE_ROWS = 4;
 FCS_HD inline bool topk_on_sixteen(int S, int B, int resident) {
     return S > 8 * 8192 && S <= 8 * 16384 && B <= TOPK_WIDE_ROWS && B <= resident;

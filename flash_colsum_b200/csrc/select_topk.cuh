@@ -24,10 +24,11 @@
 // What bounds it: a dozen dependent steps of half a microsecond to one (launch of the cluster,
 // load, cluster barriers, scans), not bytes.  Back to back on a B200, one CTA per row going over
 // it from L2 with an element per thread and step (the form before) against this one: the 16384
-// largest of 131072 216 -> 14.6 us (13.2 since the group sums are stored into the peers and nothing is exchanged at
-// the end, 11.0 on sixteen CTAs), 2048 of 16384 32 -> 7.5, 32 rows of 65536 118 -> 31; values
+// largest of 131072 216 -> 14.6 us, 2048 of 16384 32 -> 7.5, 32 rows of 65536 118 -> 31; values
 // above the mean, 131072 122 -> 11.6 us, 32 rows of 65536 64 -> 13.6.  Rows of a few thousand are
-// bound by the host (4.4 us a call).  Four copies of the first pass's bins, against lanes meeting
+// bound by the host (4.4 us a call).  Since then the group sums are stored into the peers and nothing is exchanged at
+// the end, and rows of 131072 go to sixteen CTAs where they can: 11.1 or 14.0 us a call, 12.5 or 15.0 on eight -- a call of
+// this kernel takes one of two times, 2 to 3 us apart, and keeps to it for a while; why is not known.  Four copies of the first pass's bins, against lanes meeting
 // on one bin, were no faster (14.9 us): the hardware adds equal addresses of a warp in one go.
 #pragma once
 
@@ -393,8 +394,8 @@ threshold_kernel(const float* __restrict__ colsum, long long ld, int S, float th
 
 // CTAs per row: as many as it takes for 4096 elements each, at most eight -- or sixteen where that
 // keeps the slices in registers (more than 131072 elements; one row of 262144: 17.7 us against 38).
-// (Below that sixteen lose to eight, 12.3 against 10.7 us at 65536 elements: the cluster barriers
-// and the launch grow with the cluster.  Top-k calls of few rows have a line of their own, topk_on_sixteen.)
+// (Below that sixteen lose to eight in general: the cluster barriers and the launch grow with the cluster, and fewer
+// of them run at once.  Top-k calls of few rows have a line of their own, topk_on_sixteen.)
 inline int cluster_size(int S) {
     const int most = S > 8 * 16384 ? MAX_CL : 8;
     int cl = 1;

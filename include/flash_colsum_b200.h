@@ -340,8 +340,9 @@ int fcs_last_pass_ms(float *stats_ms, float *merge_ms, float *colsum_ms);
  * Kernel choice for non-causal calls with head dimension 64 and at most 2048
  * keys, which can run as one pass on thread-block clusters instead of the two
  * streaming passes.  No counterpart in the reference.  mode 0 (default): the
- * single pass where it is the faster one (up to 1536 keys that fill their
- * 256-key slices to 60 % or more, or up to 2048 when the call is small);
+ * single pass up to 1536 keys that fill their 256-key slices to 60 % or more
+ * (256 keys: at any fill), or up to 2048 that fill them to 85 % when the call is
+ * small -- where it is clearly the faster one; past that the exps keep 32 bits;
  * 1: never; 2: whenever the shape allows.  Process-wide; not
  * thread-safe.  A single-pass call reports its whole duration as the column
  * pass in fcs_last_pass_ms().  Its results agree with the two-pass kernels to
