@@ -568,7 +568,10 @@ colsum_stream_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         float acc[4] = {0.f, 0.f, 0.f, 0.f};       // column pass state
         int item_cnt = 0, n = 0;
         // statistics pass: the item whose partials this group still has to combine
-        // (its count; which item that is waits in shared memory, not in four registers)
+        // (its count; which item that is waits in shared memory, not in four registers.  Item n + 4 is this group's next, in
+        // the same place: every item has a step, and the step of item n + 4 comes into an accumulator that all threads have
+        // released in item n + 2 or later, after they have finished item n.)
+        static_assert(MERGE_SLOTS == CONSUMER_GROUPS && NUM_TBUF == 2, "a slot is one group's, and free when it comes round");
         int pend_cnt = -1;
         int4* meta = reinterpret_cast<int4*>(smem + L::META_OFF);
         auto finish_item = [&]() -> bool {

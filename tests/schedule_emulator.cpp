@@ -387,6 +387,7 @@ extern "C" long long check_stats_digits(int B, int H, int Sq, int Sk, int causal
             if (ref.done) return -1;
             if (ref.b != it.b || ref.h != it.h || ref.qt != it.qt || ref.sp != it.sp || ref.s0 != it.s0 || ref.s1 != it.s1)
                 return -2;
+            if (it.s1 <= it.s0) return -5;      // (the consumers' item slots rely on a step per item)
             ++walked;
         }
         if (it.item < p.stats_items) return -3;
